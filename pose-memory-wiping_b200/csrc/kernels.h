@@ -55,8 +55,6 @@ typedef struct {
     uint32_t team_warps;         /* T warps per team */
     uint32_t nbatches;           /* ceil(nunits / G) */
     unsigned int *queue;         /* zeroed work counter */
-    uint32_t fma_adds;           /* 1: additions on the FMA pipe (throughput-bound launches) */
-    uint32_t one;                /* must be 1 */
 } pb_label_params_t;
 
 /* Multi-topology launch (batched sessions): batch b runs units
@@ -86,8 +84,6 @@ typedef struct {
     uint32_t nbatches;
     uint32_t team_warps;
     unsigned int *queue;
-    uint32_t fma_adds;
-    uint32_t one;
     /* optional completion signal: when a batch finishes, each of its units
      * adds 1 to req_done[unit_req[unit]] (system-scope, after a system
      * fence), so the host sees every request end as it happens */
@@ -198,7 +194,7 @@ int pb_dev_label_balance_smem(uint32_t cta_threads, uint32_t per_sm, uint32_t *s
 int pb_dev_label_single(uint32_t *d_out, int is_source, uint64_t node_index, const uint32_t *d_in,
                         int have_p0, int have_p1, cudaStream_t stream);
 int pb_dev_compress_bench(uint32_t grid, uint32_t iters, uint32_t salt, uint32_t *d_sink,
-                          int fma_adds, cudaStream_t stream);
+                          cudaStream_t stream);
 int pb_dev_compress_latency(uint32_t iters, unsigned long long *d_cycles, uint32_t *d_sink,
                             cudaStream_t stream);
 

@@ -138,7 +138,7 @@ static double model_latency(int cv0)
 }
 
 typedef struct {
-    uint32_t T, G, teams, grid, cta, kernel, smem, fma;
+    uint32_t T, G, teams, grid, cta, kernel, smem;
     uint32_t per_sm; /* lockstep kernel: teams per SM to cap residency at (0 = no cap) */
     uint32_t cluster; /* depth kernel: CTAs per chunk copy (1 = k_label_ws, >1 = k_label_wsc) */
     uint64_t team_scratch, scratch_bytes;
@@ -296,7 +296,6 @@ static int make_plan(const pose_hbm_topo_t *ct, uint64_t nunits, const pose_b200
                          * of teams go on every SM */
                         best->smem = 0;
                         best->per_sm = R % t->sms == 0 && R / t->sms < (uint64_t)occ ? (uint32_t)(R / t->sms) : 0;
-                        best->fma = kernel == 1 && alu >= lat; /* ALU-bound: move adds to the FMA pipe */
                     }
                 }
             }
@@ -329,7 +328,7 @@ static int make_plan(const pose_hbm_topo_t *ct, uint64_t nunits, const pose_b200
             best->T = nc; best->G = 1; best->teams = (uint32_t)nunits;
             best->grid = (uint32_t)(nunits * C); best->cta = 32 * (nc + 1);
             best->team_scratch = team_scratch; best->scratch_bytes = sbytes;
-            best->cost = cost; best->kernel = 3; best->smem = ws_smem_bytes(t, nc); best->fma = 0;
+            best->cost = cost; best->kernel = 3; best->smem = ws_smem_bytes(t, nc);
             best->per_sm = 0;
             best->cluster = C;
         }
@@ -361,7 +360,7 @@ static int make_plan(const pose_hbm_topo_t *ct, uint64_t nunits, const pose_b200
             best->T = nc; best->G = 1; best->teams = (uint32_t)R;
             best->grid = (uint32_t)R; best->cta = 32 * (nc + 1);
             best->team_scratch = team_scratch; best->scratch_bytes = sbytes;
-            best->cost = cost; best->kernel = 3; best->smem = ws_smem_bytes(t, nc); best->fma = 0;
+            best->cost = cost; best->kernel = 3; best->smem = ws_smem_bytes(t, nc);
             best->per_sm = 0;
             best->cluster = 1;
         }
@@ -917,9 +916,6 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
             p.team_warps = plan.T;
             p.nbatches = (uint32_t)((p.nunits + plan.G - 1) / plan.G);
             p.queue = t->d_queue;
-            p.fma_adds = plan.fma;
-            p.one = 1;
-            { const char *e = getenv("POSE_B200_FMA_ADDS"); if (e && e[0]) p.fma_adds = (uint32_t)atoi(e); }
             CK(cudaEventRecord(t->ev[1], t->stream), "event");
             int lrc;
             if (plan.kernel == 3) {
@@ -1126,17 +1122,14 @@ double pose_b200_compress_rate(uint32_t iters, double *latency_cycles)
     CK(cudaEventCreate(&b), "event");
     {
         uint32_t grid = (uint32_t)sms * 8; /* 8 CTAs x 256 threads per SM */
-        for (int fma = 0; fma <= 1; fma++) {
-            if (pb_dev_compress_bench(grid, iters / 8 + 1, 1, d_sink, fma, 0) != 0) goto fail; /* warm-up */
-            CK(cudaEventRecord(a, 0), "event");
-            if (pb_dev_compress_bench(grid, iters, 2, d_sink, fma, 0) != 0) goto fail;
-            CK(cudaEventRecord(b, 0), "event");
-            CK(cudaEventSynchronize(b), "bench");
-            float ms = 0;
-            cudaEventElapsedTime(&ms, a, b);
-            double r = (double)grid * 256.0 * iters / (ms * 1e-3);
-            if (r > rate) rate = r;
-        }
+        if (pb_dev_compress_bench(grid, iters / 8 + 1, 1, d_sink, 0) != 0) goto fail; /* warm-up */
+        CK(cudaEventRecord(a, 0), "event");
+        if (pb_dev_compress_bench(grid, iters, 2, d_sink, 0) != 0) goto fail;
+        CK(cudaEventRecord(b, 0), "event");
+        CK(cudaEventSynchronize(b), "bench");
+        float ms = 0;
+        cudaEventElapsedTime(&ms, a, b);
+        rate = (double)grid * 256.0 * iters / (ms * 1e-3);
         if (latency_cycles) {
             if (pb_dev_compress_latency(iters, d_cyc, d_sink, 0) != 0) goto fail;
             CK(cudaMemcpy(&cyc, d_cyc, 8, cudaMemcpyDeviceToHost), "cycles");

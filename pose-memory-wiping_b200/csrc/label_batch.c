@@ -39,7 +39,7 @@
 typedef struct {
     void *d_topos, *d_batches, *d_units, *d_jobs, *d_seeds, *d_scratch, *d_queue;
     uint64_t scratch_bytes, nodes, super_chunks, units, nbatches, njobs;
-    uint32_t teams, T, Gmax, fma, cv0, grid, cta_threads;
+    uint32_t teams, T, Gmax, cv0, grid, cta_threads;
     uint64_t team_scratch;
     int kind;
     pb_topo_view2_t v2;
@@ -57,7 +57,7 @@ struct pose_b200_batch {
     int nparts;
     batch_part_t part[3]; /* part[1]: the deep requests, when split; part[2]: the next-deepest topology's */
     uint64_t scratch_bytes, nodes, super_chunks, units;
-    uint32_t nbatches, teams, T, Gmax, fma, cv0;
+    uint32_t nbatches, teams, T, Gmax, cv0;
 };
 
 typedef struct {
@@ -408,7 +408,6 @@ static int part_setup(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_table
     q->grid = (uint32_t)R;
     q->cta_threads = 32 * T;
     q->teams = (uint32_t)R;
-    q->fma = (double)R * T / pl->sms >= 8.0;
     q->scratch_bytes = R * pl->team_scratch;
     if (pb_dev_malloc(&q->d_topos, pl->ntopo * sizeof(pb_topo_view_t)) != cudaSuccess ||
         pb_dev_malloc(&q->d_batches, pl->nbatches * sizeof(pb_mbatch_t)) != cudaSuccess ||
@@ -452,7 +451,6 @@ static int part_setup_wsg(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_t
     q->nodes = pl->nodes;
     q->Gmax = G;
     q->cv0 = 1;
-    q->fma = 0;
     q->nbatches = (pl->nunits + G - 1) / G;
     q->grid = (uint32_t)(q->nbatches < sms ? q->nbatches : sms);
     q->teams = q->grid;
@@ -503,8 +501,6 @@ static int part_capture(const pose_b200_batch_t *b, const batch_part_t *q, cudaS
     p.nbatches = (uint32_t)q->nbatches;
     p.team_warps = q->T;
     p.queue = (unsigned int *)q->d_queue;
-    p.fma_adds = q->fma;
-    p.one = 1;
     int crc = pb_dev_seed_jobs(q->d_jobs, (uint32_t)q->njobs, (const uint8_t *)b->d_blob, (uint32_t *)q->d_seeds, s);
     if (crc == 0) crc = cudaMemsetAsync(q->d_queue, 0, 64, s) == cudaSuccess ? 0 : -1;
     if (crc == 0 && e0) crc = cudaEventRecord(e0, s) == cudaSuccess ? 0 : -1;

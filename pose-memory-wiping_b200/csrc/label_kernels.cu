@@ -177,9 +177,9 @@ __device__ __forceinline__ uint4 staged(uint32_t b, uint32_t k)
  * two levels ahead, so that a level's dependent chain is only the
  * predecessor loads, the two compressions and the barrier.  Each thread
  * reads back only its own staging slots, after waiting for its own copies. */
-template <bool FMA, bool CTA_TEAM>
+template <bool CTA_TEAM>
 __device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const UnitCtx &c, uint32_t T,
-                                             uint32_t bar_id, uint32_t TT, uint32_t one)
+                                             uint32_t bar_id, uint32_t TT)
 {
     const uint32_t L = tp.L;
     uint32_t s0 = __ldg(tp.lstart);
@@ -229,19 +229,13 @@ __device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const Uni
                     uint32_t m0[16];
                     key_words(cv, np == 0);
                     block0_words(m0, (rec.x & PB_REC_ID_MASK) + c.id_off);
-                    if (FMA) compress_fma(cv, m0, 64, kFlagsBlock0, one);
-                    else compress(cv, m0, 64, kFlagsBlock0);
+                    compress(cv, m0, 64, kFlagsBlock0);
                 }
                 uint32_t m2[16];
 #pragma unroll
                 for (int i = 0; i < 8; i++) { m2[i] = c.seed[i]; m2[8 + i] = tp.desc[i]; }
-                if (FMA) {
-                    compress_fma(cv, m, 64, kFlagsBlock1, one);
-                    compress_fma(cv, m2, 64, kFlagsBlock2, one);
-                } else {
-                    compress(cv, m, 64, kFlagsBlock1);
-                    compress(cv, m2, 64, kFlagsBlock2);
-                }
+                compress(cv, m, 64, kFlagsBlock1);
+                compress(cv, m2, 64, kFlagsBlock2);
                 const uint4 o0 = make_uint4(cv[0], cv[1], cv[2], cv[3]);
                 const uint4 o1 = make_uint4(cv[4], cv[5], cv[6], cv[7]);
                 uint4 *d = c.tscr + (((size_t)rec.w << c.glog) + c.u) * 2;
@@ -283,7 +277,6 @@ __device__ __forceinline__ uint32_t grab_batch(unsigned int *queue, uint32_t T, 
 
 /* The lockstep kernel for one topology: one team of T warps per CTA
  * (blockDim.x == 32 T), so any number of teams can be resident per SM. */
-template <bool FMA>
 __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant__ pb_label_params_t p)
 {
     const uint32_t T = p.team_warps;
@@ -315,7 +308,7 @@ __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant_
         c.cv0 = tp.cv0 ? tp.cv0 + (uint64_t)copy * tp.S * 2 : nullptr;
 #pragma unroll
         for (int i = 0; i < 8; i++) c.seed[i] = c.valid ? p.seeds[8 * (size_t)chunk + i] : 0u;
-        label_levels<FMA, true>(tp, c, T, bar_id, TT, p.one);
+        label_levels<true>(tp, c, T, bar_id, TT);
     }
 }
 
@@ -323,7 +316,6 @@ __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant_
  * G = 2^glog units) from a queue sorted longest first, and copy the batch's
  * topology view into shared memory.  One team of T warps per CTA
  * (blockDim.x == 32 T), ending its levels with the CTA barrier. */
-template <bool FMA>
 __global__ void __launch_bounds__(PB_MULTI_CTA_THREADS, 3) k_label_multi(const __grid_constant__ pb_multi_params_t p)
 {
     const uint32_t T = p.team_warps;
@@ -360,7 +352,7 @@ __global__ void __launch_bounds__(PB_MULTI_CTA_THREADS, 3) k_label_multi(const _
         c.cv0 = tp.cv0 ? tp.cv0 + (uint64_t)copy * tp.S * 2 : nullptr;
 #pragma unroll
         for (int i = 0; i < 8; i++) c.seed[i] = c.valid ? p.seeds[8 * (size_t)un.seed + i] : 0u;
-        label_levels<FMA, true>(tp, c, T, bar_id, TT, p.one);
+        label_levels<true>(tp, c, T, bar_id, TT);
         /* label_levels ended with a team barrier, so every persisted label of
          * the batch is ordered before this fence */
         if (p.req_done != nullptr && tt < bd.count) {
@@ -446,9 +438,8 @@ __global__ void k_label_single(uint32_t *out, int is_source, uint64_t node_index
  * work cannot be elided.  Counting compressions / time with every SM full
  * gives the sustained compression rate of this GPU for the exact instruction
  * mix the labeler issues. */
-template <bool FMA>
 __global__ void __launch_bounds__(256) k_compress_bench(uint32_t iters, uint32_t salt,
-                                                        uint32_t *sink, uint32_t one)
+                                                        uint32_t *sink)
 {
     uint32_t cv[8], m[16];
 #pragma unroll
@@ -456,8 +447,7 @@ __global__ void __launch_bounds__(256) k_compress_bench(uint32_t iters, uint32_t
 #pragma unroll
     for (int i = 0; i < 16; i++) m[i] = blockIdx.x * 0x85EBCA6Bu + i * 0x27D4EB2Fu;
     for (uint32_t k = 0; k < iters; k++) {
-        if (FMA) compress_fma(cv, m, 64, kFlagsBlock1, one);
-        else compress(cv, m, 64, kFlagsBlock1);
+        compress(cv, m, 64, kFlagsBlock1);
 #pragma unroll
         for (int i = 0; i < 8; i++) m[i] ^= cv[i];
     }
@@ -532,8 +522,7 @@ extern "C" int pb_dev_chunk_seeds(const uint8_t *d_session_seed, uint32_t seed_l
 static void allow_stage_smem()
 {
     const int bytes = (int)(PB_PREF_BYTES_PER_THREAD * PB_CTA_THREADS);
-    cudaFuncSetAttribute(pb::k_label<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(pb::k_label<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(pb::k_label, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 extern "C" int pb_dev_label(const pb_label_params_t *params, uint32_t grid, uint32_t cta_threads,
@@ -543,18 +532,15 @@ extern "C" int pb_dev_label(const pb_label_params_t *params, uint32_t grid, uint
     cudaGetLastError(); /* report only this launch */
     uint32_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
     if (smem_bytes > smem) {
-        if (cudaFuncSetAttribute(pb::k_label<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(pb::k_label<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) !=
-                cudaSuccess)
+        if (cudaFuncSetAttribute(pb::k_label, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) !=
+            cudaSuccess)
             return -1;
         smem = smem_bytes;
     } else if (smem > 48 * 1024 - 1024) {
         allow_stage_smem();
     }
     cudaGetLastError();
-    if (params->fma_adds) pb::k_label<true><<<grid, cta_threads, smem, stream>>>(*params);
-    else pb::k_label<false><<<grid, cta_threads, smem, stream>>>(*params);
+    pb::k_label<<<grid, cta_threads, smem, stream>>>(*params);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -564,20 +550,17 @@ extern "C" int pb_dev_label_multi(const pb_multi_params_t *params, uint32_t grid
     if (cta_threads != 32u * params->team_warps || cta_threads > PB_MULTI_CTA_THREADS) return -1; /* one team per CTA */
     cudaGetLastError(); /* report only this launch */
     const uint32_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
-    if (params->fma_adds) pb::k_label_multi<true><<<grid, cta_threads, smem, stream>>>(*params);
-    else pb::k_label_multi<false><<<grid, cta_threads, smem, stream>>>(*params);
+    pb::k_label_multi<<<grid, cta_threads, smem, stream>>>(*params);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 extern "C" int pb_dev_label_multi_occupancy(uint32_t cta_threads, int *blocks_per_sm)
 {
-    int a = 0, b = 0;
     const size_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, pb::k_label_multi<false>, (int)cta_threads, smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, pb::k_label_multi<true>, (int)cta_threads, smem) != cudaSuccess)
-        return -1;
-    *blocks_per_sm = a < b ? a : b;
-    return 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pb::k_label_multi, (int)cta_threads, smem) ==
+                   cudaSuccess
+               ? 0
+               : -1;
 }
 
 extern "C" int pb_dev_seed_jobs(const void *jobs, uint32_t njobs, const uint8_t *blob, uint32_t *seeds,
@@ -608,24 +591,18 @@ extern "C" int pb_dev_label_balance_smem(uint32_t cta_threads, uint32_t per_sm, 
     if (pb_dev_label_occupancy(cta_threads, &occ) != 0) return -1;
     if ((uint32_t)occ <= per_sm) return 0;
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, pb::k_label<true>) != cudaSuccess) return -1;
+    if (cudaFuncGetAttributes(&fa, pb::k_label) != cudaSuccess) return -1;
     /* largest multiple of 1 KiB with per_sm CTAs fitting the SM's shared memory */
     int64_t each = (int64_t)cap / per_sm - resv - (int64_t)fa.sharedSizeBytes;
     each -= each % 1024;
     if (each > optin - (int64_t)fa.sharedSizeBytes) each = optin - (int64_t)fa.sharedSizeBytes;
     if (each < (int64_t)base) return 0;
     for (; each >= (int64_t)base; each -= 1024) {
-        int a = 0, b = 0;
-        if (cudaFuncSetAttribute(pb::k_label<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)each) !=
+        int m = 0;
+        if (cudaFuncSetAttribute(pb::k_label, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)each) !=
                 cudaSuccess ||
-            cudaFuncSetAttribute(pb::k_label<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)each) !=
-                cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, pb::k_label<false>, (int)cta_threads, each) !=
-                cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, pb::k_label<true>, (int)cta_threads, each) !=
-                cudaSuccess)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, pb::k_label, (int)cta_threads, each) != cudaSuccess)
             return -1;
-        const int m = a > b ? a : b;
         if ((uint32_t)m == per_sm) {
             *smem_bytes = (uint32_t)each;
             return 0;
@@ -637,14 +614,12 @@ extern "C" int pb_dev_label_balance_smem(uint32_t cta_threads, uint32_t per_sm, 
 
 extern "C" int pb_dev_label_occupancy(uint32_t cta_threads, int *blocks_per_sm)
 {
-    int a = 0, b = 0;
     const size_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
     allow_stage_smem();
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, pb::k_label<false>, (int)cta_threads, smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, pb::k_label<true>, (int)cta_threads, smem) != cudaSuccess)
-        return -1;
-    *blocks_per_sm = a < b ? a : b;
-    return 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pb::k_label, (int)cta_threads, smem) ==
+                   cudaSuccess
+               ? 0
+               : -1;
 }
 
 extern "C" int pb_dev_label_single(uint32_t *d_out, int is_source, uint64_t node_index,
@@ -657,11 +632,10 @@ extern "C" int pb_dev_label_single(uint32_t *d_out, int is_source, uint64_t node
 }
 
 extern "C" int pb_dev_compress_bench(uint32_t grid, uint32_t iters, uint32_t salt, uint32_t *d_sink,
-                                     int fma_adds, cudaStream_t stream)
+                                     cudaStream_t stream)
 {
     cudaGetLastError(); /* report only this launch */
-    if (fma_adds) pb::k_compress_bench<true><<<grid, 256, 0, stream>>>(iters, salt, d_sink, 1u);
-    else pb::k_compress_bench<false><<<grid, 256, 0, stream>>>(iters, salt, d_sink, 1u);
+    pb::k_compress_bench<<<grid, 256, 0, stream>>>(iters, salt, d_sink);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

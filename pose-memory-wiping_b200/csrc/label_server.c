@@ -574,8 +574,6 @@ static int admit_wave(pose_b200_server_t *s)
     p.nbatches = (uint32_t)pl.nbatches;
     p.team_warps = Tw;
     p.queue = (unsigned int *)(T + o_queue);
-    p.fma_adds = (double)R * Tw / pl.sms >= 8.0;
-    p.one = 1;
     p.unit_req = (const uint32_t *)(T + o_ureq);
     p.req_done = wv->d_done;
     if (ok) ok = pb_dev_label_multi(&p, g2, 32 * Tw, wv->stream) == 0;
