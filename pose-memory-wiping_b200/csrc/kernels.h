@@ -106,66 +106,47 @@ typedef struct {
     uint32_t desc[8];
 } pb_topo_view2_t;
 
-/* One launch of the depth kernel k_label_ws (label_ws.cu); fields as in
- * pb_label_params_t, with the pipelined records' view. */
-typedef struct {
-    pb_topo_view2_t topo;
-    const uint32_t *seeds;
-    uint8_t *persist;
-    uint64_t super_bytes;
-    uint64_t first_super;
-    uint8_t *scratch;
-    uint64_t team_scratch_bytes; /* G * gpool * 32 */
-    uint32_t nunits;
-    uint32_t copies_log2;
-    uint32_t g_log2;
-    uint32_t team_warps;
-    uint32_t nbatches;
-    unsigned int *queue;
-    /* k_label_wsc only: CTAs per chunk copy (a cluster), levels wider than
-     * split_width shared by them, and the indices of those levels */
-    uint32_t cluster;
-    uint32_t split_width;
-    const uint32_t *split_levels;
-    uint32_t nsplit;
-} pb_pipe_params_t;
-
-/* Warp-specialised depth-regime kernel (label_ws.cu): team_warps hashing
- * warps + 1 producer warp per CTA, one chunk copy per CTA, g_log2 = 0. */
-int pb_dev_label_ws(const pb_pipe_params_t *params, uint32_t grid, uint32_t cta_threads,
-                    uint32_t smem_bytes, cudaStream_t stream);
-int pb_dev_label_ws_occupancy(uint32_t cta_threads, uint32_t smem_bytes, int *blocks_per_sm);
-/* The depth kernel with a cluster of params->cluster CTAs per chunk copy
- * (label_ws.cu, k_label_wsc): params->nunits * cluster CTAs, one copy per
- * cluster, no work queue. */
-int pb_dev_label_wsc(const pb_pipe_params_t *params, uint32_t smem_bytes, cudaStream_t stream);
-int pb_dev_label_wsc_max_clusters(uint32_t C, uint32_t team_warps, uint32_t smem_bytes, int *clusters);
-
-/* Multi-unit depth kernel (label_ws.cu): k_label_ws with G = units_per_cta
- * (1 to 4) units of one topology per CTA in lockstep.  Batch b is units
- * [b * G, min(nunits, (b + 1) * G)) of `units`; unit k's global label pool
- * is scratch + (cta * G + k % G) * unit_scratch_bytes.  The
- * topology's pipelined records are built for a pool of topo.csm slots per
- * unit, and shared memory holds G such pools (pb_wsg_smem_bytes). */
+/* One launch of the depth kernels k_label_ws and k_label_wsc (label_ws.cu):
+ * batch b is units [b * G, min(nunits, (b + 1) * G)), G = units_per_cta.
+ * Unit k is entry k of `units`, or, when that is NULL, copy
+ * (k & (2^copies_log2 - 1)) of local chunk k >> copies_log2 as in
+ * pb_label_params_t.  Unit k % G of a CTA keeps its global label pool at
+ * scratch + (cta * G + k % G) * unit_scratch_bytes. */
 typedef struct {
     pb_topo_view2_t topo;
     const pb_munit_t *units;
-    const uint32_t *seeds;       /* 8 words per seed index (pb_munit_t.seed) */
+    const uint32_t *seeds;       /* 8 words per seed index (pb_munit_t.seed, or the local chunk) */
+    uint8_t *persist;            /* units == NULL only, with super_bytes, first_super, copies_log2 */
+    uint64_t super_bytes;
+    uint64_t first_super;
+    uint32_t copies_log2;
+    uint32_t nunits;
     uint8_t *scratch;
     uint64_t unit_scratch_bytes; /* topo.gpool * 32 */
-    uint32_t nunits;
     uint32_t units_per_cta;      /* G: 1 to 4 */
     uint32_t team_warps;         /* hashing warps: 7 or 15 */
     uint32_t nbatches;           /* ceil(nunits / G) */
     unsigned int *queue;         /* zeroed work counter */
-} pb_wsg_params_t;
+    /* k_label_wsc only (G = 1): CTAs per chunk copy (a cluster), levels wider
+     * than split_width shared by them, and the indices of those levels */
+    uint32_t cluster;
+    uint32_t split_width;
+    const uint32_t *split_levels;
+    uint32_t nsplit;
+} pb_depth_params_t;
 
-uint32_t pb_wsg_smem_bytes(uint32_t csm, uint32_t units_per_cta, uint32_t team_warps);
-int pb_dev_label_wsg(const pb_wsg_params_t *params, uint32_t grid, uint32_t cta_threads, uint32_t smem_bytes,
-                     cudaStream_t stream);
-/* Raise k_label_wsg's dynamic shared memory limit to the most a CTA can
- * have and report it; before any launch or stream capture of it. */
-int pb_dev_label_wsg_prepare(uint32_t *max_smem_bytes);
+/* Dynamic shared memory of a CTA: G label pools of csm slots and the staging
+ * areas of team_warps hashing warps. */
+uint32_t pb_ws_smem_bytes(uint32_t csm, uint32_t units_per_cta, uint32_t team_warps);
+/* Raise k_label_ws's dynamic shared memory limit to the most a CTA can have
+ * and report it; once per device before any launch or stream capture of it. */
+int pb_dev_label_ws_prepare(uint32_t *max_smem_bytes);
+int pb_dev_label_ws(const pb_depth_params_t *params, uint32_t grid, uint32_t smem_bytes, cudaStream_t stream);
+int pb_dev_label_ws_occupancy(uint32_t cta_threads, uint32_t smem_bytes, int *blocks_per_sm);
+/* The depth kernel with a cluster of params->cluster CTAs per chunk copy:
+ * params->nunits * cluster CTAs, one copy per cluster, no work queue. */
+int pb_dev_label_wsc(const pb_depth_params_t *params, uint32_t smem_bytes, cudaStream_t stream);
+int pb_dev_label_wsc_max_clusters(uint32_t C, uint32_t team_warps, uint32_t smem_bytes, int *clusters);
 
 /* Verifier helpers (label_verify.cu).  Compare nblocks 32-byte blocks of a
  * and b, grouped blocks_per_group to a group: first_bad[g] = min over

@@ -158,7 +158,7 @@ static double model_ws_latency(void)
 
 static uint32_t ws_smem_bytes(const pose_hbm_topo_t *t, uint32_t nc)
 {
-    return (2u * t->view2.csm + 18u * 32u * nc + 3u) * 16u;
+    return pb_ws_smem_bytes(t->view2.csm, 1, nc);
 }
 
 static int ws_occupancy(pose_hbm_topo_t *t, uint32_t nc)
@@ -919,13 +919,13 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
             CK(cudaEventRecord(t->ev[1], t->stream), "event");
             int lrc;
             if (plan.kernel == 3) {
-                pb_pipe_params_t pp;
+                pb_depth_params_t pp;
                 memset(&pp, 0, sizeof(pp));
                 pp.topo = t->view2;
                 pp.seeds = p.seeds; pp.persist = p.persist; pp.super_bytes = p.super_bytes;
                 pp.first_super = p.first_super; pp.scratch = p.scratch;
-                pp.team_scratch_bytes = plan.team_scratch; pp.nunits = p.nunits;
-                pp.copies_log2 = p.copies_log2; pp.g_log2 = p.g_log2; pp.team_warps = p.team_warps;
+                pp.unit_scratch_bytes = plan.team_scratch; pp.nunits = p.nunits;
+                pp.copies_log2 = p.copies_log2; pp.units_per_cta = 1; pp.team_warps = p.team_warps;
                 pp.nbatches = p.nbatches; pp.queue = p.queue;
                 if (plan.cluster > 1) {
                     pp.cluster = plan.cluster;
@@ -934,7 +934,7 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
                     pp.nsplit = t->nsplit;
                     lrc = pb_dev_label_wsc(&pp, plan.smem, t->stream);
                 } else {
-                    lrc = pb_dev_label_ws(&pp, plan.grid, plan.cta, plan.smem, t->stream);
+                    lrc = pb_dev_label_ws(&pp, plan.grid, plan.smem, t->stream);
                 }
             } else {
                 uint32_t smem = 0;

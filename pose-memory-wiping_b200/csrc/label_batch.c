@@ -459,7 +459,7 @@ static int part_setup_wsg(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_t
     q->team_scratch = (uint64_t)G * v2->gpool * 32;
     q->scratch_bytes = (uint64_t)q->grid * q->team_scratch;
     uint32_t max_smem = 0;
-    if (pb_dev_label_wsg_prepare(&max_smem) != 0 || pb_wsg_smem_bytes(v2->csm, G, NC) > max_smem) {
+    if (pb_dev_label_ws_prepare(&max_smem) != 0 || pb_ws_smem_bytes(v2->csm, G, NC) > max_smem) {
         fprintf(stderr, "pose_b200_batch_create: shared memory attribute: %s\n", cudaGetErrorString(cudaGetLastError()));
         return -1;
     }
@@ -505,7 +505,7 @@ static int part_capture(const pose_b200_batch_t *b, const batch_part_t *q, cudaS
     if (crc == 0) crc = cudaMemsetAsync(q->d_queue, 0, 64, s) == cudaSuccess ? 0 : -1;
     if (crc == 0 && e0) crc = cudaEventRecord(e0, s) == cudaSuccess ? 0 : -1;
     if (crc == 0 && q->kind == 1) {
-        pb_wsg_params_t w;
+        pb_depth_params_t w;
         memset(&w, 0, sizeof(w));
         w.topo = q->v2;
         w.units = (const pb_munit_t *)q->d_units;
@@ -517,7 +517,7 @@ static int part_capture(const pose_b200_batch_t *b, const batch_part_t *q, cudaS
         w.team_warps = q->T;
         w.nbatches = (uint32_t)q->nbatches;
         w.queue = (unsigned int *)q->d_queue;
-        crc = pb_dev_label_wsg(&w, q->grid, q->cta_threads, q->smem, s);
+        crc = pb_dev_label_ws(&w, q->grid, q->smem, s);
     } else if (crc == 0) {
         crc = pb_dev_label_multi(&p, q->grid, q->cta_threads, s);
     }
@@ -649,11 +649,11 @@ no_split:
                 /* a device whose CTAs cannot hold the kernel's shared memory
                  * keeps the deep part on the lockstep kernel */
                 uint32_t max_smem = 0;
-                wsg = pb_dev_label_wsg_prepare(&max_smem) == 0 && pb_wsg_smem_bytes(v2.csm, G, 15) <= max_smem;
+                wsg = pb_dev_label_ws_prepare(&max_smem) == 0 && pb_ws_smem_bytes(v2.csm, G, 15) <= max_smem;
                 cudaGetLastError();
             }
             if (wsg) {
-                const uint32_t smem = pb_wsg_smem_bytes(v2.csm, G, 15);
+                const uint32_t smem = pb_ws_smem_bytes(v2.csm, G, 15);
                 if (pb_plan_requests(pd, nd, 8, 1, 0.9999, &pl[1]) != 0 || pl[1].nunits == 0) goto fail;
                 if (part_setup_wsg(b, &b->part[1], &pl[1], &v2, G, sms, smem) != 0) goto fail;
                 /* the next-deepest topology's requests: a third launch of the
@@ -673,8 +673,8 @@ no_split:
                     const uint32_t left = sms > b->part[1].grid ? sms - b->part[1].grid : 0;
                     uint32_t max_smem2 = 0;
                     int ok2 = left > 0 && pb_topo_view2_small(pd2[0].topo, &v2b) == 0 &&
-                              pb_dev_label_wsg_prepare(&max_smem2) == 0 &&
-                              pb_wsg_smem_bytes(v2b.csm, G2, 15) <= max_smem2;
+                              pb_dev_label_ws_prepare(&max_smem2) == 0 &&
+                              pb_ws_smem_bytes(v2b.csm, G2, 15) <= max_smem2;
                     cudaGetLastError();
                     if (ok2) {
                         const uint64_t g2 = (du2 + G2 - 1) / G2 < left ? (du2 + G2 - 1) / G2 : left;
@@ -682,7 +682,7 @@ no_split:
                     }
                     if (ok2) {
                         if (pb_plan_requests(pd2, nd2, 8, 1, 0.9999, &pl[2]) != 0 || pl[2].nunits == 0) goto fail;
-                        if (part_setup_wsg(b, &b->part[2], &pl[2], &v2b, G2, left, pb_wsg_smem_bytes(v2b.csm, G2, 15)) !=
+                        if (part_setup_wsg(b, &b->part[2], &pl[2], &v2b, G2, left, pb_ws_smem_bytes(v2b.csm, G2, 15)) !=
                             0)
                             goto fail;
                     } else {

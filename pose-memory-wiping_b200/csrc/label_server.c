@@ -24,7 +24,7 @@
  *   - deep requests (topologies of at least PB_SERVER_DEEP_LEVELS levels,
  *     chunk_blocks 2^17 and up) do not join waves: the pending deep requests
  *     of one topology run together on the multi-unit depth kernel
- *     (k_label_wsg: a producer warp and 15 hashing warps per CTA, three chunk
+ *     (k_label_ws: a producer warp and 15 hashing warps per CTA, three chunk
  *     copies per CTA) in a slot of their own, on a high-priority stream.
  *     Each depth CTA holds its SM alone (its shared memory is raised to the
  *     limit), so no lockstep warp slows its chain, and at most one depth CTA
@@ -209,7 +209,7 @@ static int req_is_deep(const pose_b200_server_t *s, const pose_hbm_topo_t *topo)
         cudaGetLastError();
         return 0;
     }
-    return pb_wsg_smem_bytes(v2.csm, 4, PB_SERVER_DEEP_WARPS) <= s->wsg_smem_max &&
+    return pb_ws_smem_bytes(v2.csm, 4, PB_SERVER_DEEP_WARPS) <= s->wsg_smem_max &&
            (uint64_t)v2.gpool * 32 <= s->arena_bytes;
 }
 
@@ -399,7 +399,7 @@ static int admit_deep(pose_b200_server_t *s)
     ok = ok && pb_dev_seed_jobs(T + o_jobs, (uint32_t)nsuper, s->d_sessions, (uint32_t *)(T + o_seeds), wv->stream) == 0;
     ok = ok && cudaMemsetAsync(T + o_queue, 0, 64, wv->stream) == cudaSuccess;
     if (ok) {
-        pb_wsg_params_t p;
+        pb_depth_params_t p;
         memset(&p, 0, sizeof(p));
         p.topo = v2;
         p.units = (const pb_munit_t *)(T + o_units);
@@ -411,9 +411,8 @@ static int admit_deep(pose_b200_server_t *s)
         p.team_warps = PB_SERVER_DEEP_WARPS;
         p.nbatches = (uint32_t)nbatches;
         p.queue = (unsigned int *)(T + o_queue);
-        const uint32_t need = pb_wsg_smem_bytes(v2.csm, G, PB_SERVER_DEEP_WARPS);
-        ok = pb_dev_label_wsg(&p, grid, 32 * (PB_SERVER_DEEP_WARPS + 1),
-                              s->deep_excl && s->wsg_smem_max > need ? s->wsg_smem_max : need, wv->stream) == 0;
+        const uint32_t need = pb_ws_smem_bytes(v2.csm, G, PB_SERVER_DEEP_WARPS);
+        ok = pb_dev_label_ws(&p, grid, s->deep_excl && s->wsg_smem_max > need ? s->wsg_smem_max : need, wv->stream) == 0;
     }
     /* scratch and chunk seeds are zeroed before the requests count as done */
     ok = ok && cudaMemsetAsync(s->d_arena + off, 0, scratch, wv->stream) == cudaSuccess;
@@ -753,7 +752,7 @@ pose_b200_server_t *pose_b200_server_create(uint64_t scratch_bytes, uint32_t max
         if (e && atoi(e) > 0 && atoi(e) < sms) sms = atoi(e);
         s->sms = (uint32_t)sms;
         uint32_t mx = 0;
-        if (pb_dev_label_wsg_prepare(&mx) != 0) mx = 0; /* no depth kernel: deep requests join waves */
+        if (pb_dev_label_ws_prepare(&mx) != 0) mx = 0; /* no depth kernel: deep requests join waves */
         cudaGetLastError();
         const char *ed = getenv("POSE_B200_SERVER_DEEP"); /* 0: every request joins the waves */
         s->wsg_smem_max = ed && ed[0] == '0' ? 0 : mx;
