@@ -21,7 +21,8 @@ extern "C" {
 /* Schedule of one labeling launch.  Zero fields mean "choose automatically". */
 typedef struct {
     uint32_t team_warps;        /* T: warps that cooperate on one batch (1..16, power of 2) */
-    uint32_t units_per_team;    /* G: chunk copies run in lockstep by one team (1..32, power of 2) */
+    uint32_t units_per_team;    /* G: chunk copies run in lockstep by one team (1..32, power of 2);
+                                   the automatic choice also takes other counts, up to 64 */
     uint32_t max_teams;         /* cap on resident teams (0 = occupancy and memory bound) */
     uint32_t kernel;            /* 0 = automatic, 1 = basic lockstep kernel,
                                    3 = warp-specialised depth kernel (team_warps = hashing warps: 7 or 15);
@@ -132,8 +133,7 @@ typedef struct pose_b200_batch pose_b200_batch_t;
  * beside the first unless flags has POSE_B200_BATCH_ONE_LAUNCH; sched then
  * applies to the rest.  When the deep requests share one topology built with
  * its block-0 table, that launch is the multi-unit depth kernel (1, 2 or 4
- * chunk copies per CTA, at most one CTA per SM; the topology then also keeps
- * a second set of pipelined records, 32 bytes per node, built on first use).
+ * chunk copies per CTA, at most one CTA per SM).
  * Otherwise it is the lockstep kernel with 8-warp teams, units packed up to
  * 4 a team so that they hold about half the SMs' team slots.  The
  * environment variable POSE_B200_DEEP_KERNEL=0 selects the lockstep kernel
@@ -222,10 +222,9 @@ typedef struct pose_b200_server pose_b200_server_t;
 pose_b200_server_t *pose_b200_server_create(uint64_t scratch_bytes, uint32_t max_waves);
 /* Register a session seed (<= 1016 bytes); returns its id, or -1. */
 int pose_b200_server_session(pose_b200_server_t *server, const uint8_t *seed, size_t seed_len);
-/* Build ahead of the first request what requests of this topology need (the
- * depth kernel's 512-slot records, for a deep topology; kept with the
- * topology).  Optional: the first submit of a topology does it otherwise, in
- * the submitting thread.  0 on success, -1 on a bad argument. */
+/* Make ready, ahead of the first request, what requests of this topology
+ * need beyond the topology itself (at present nothing).  Optional.  0 on
+ * success, -1 on a bad argument. */
 int pose_b200_server_prepare(pose_b200_server_t *server, const pose_hbm_topo_t *topo);
 /* Queue one request; returns its ticket, or -1. */
 int64_t pose_b200_server_submit(pose_b200_server_t *server, const pose_hbm_topo_t *topo, int session,

@@ -12,7 +12,8 @@
 extern "C" {
 #endif
 
-/* Largest CTA the labeling kernel is launched with (teams of up to 16 warps). */
+/* Largest CTA the labeling kernels are launched with (lockstep teams of up to
+ * 16 warps; 15 hashing warps and a producer). */
 #define PB_CTA_THREADS 512
 /* Largest CTA of the multi-topology kernel (k_label_multi is compiled for
  * three such CTAs per SM). */
@@ -51,16 +52,16 @@ typedef struct {
     uint64_t team_scratch_bytes; /* G * pool * 32 */
     uint32_t nunits;
     uint32_t copies_log2;
-    uint32_t g_log2;             /* G = 2^g_log2 units per team */
+    uint32_t units_per_team;     /* G: 1 to 32 team_warps */
     uint32_t team_warps;         /* T warps per team */
     uint32_t nbatches;           /* ceil(nunits / G) */
     unsigned int *queue;         /* zeroed work counter */
 } pb_label_params_t;
 
 /* Multi-topology launch (batched sessions): batch b runs units
- * [first_unit, first_unit + count) of topology `topo`, count <= 2^glog. */
+ * [first_unit, first_unit + count) of topology `topo`, count <= G. */
 typedef struct {
-    uint32_t topo, first_unit, count, glog;
+    uint32_t topo, first_unit, count, G;
 } pb_mbatch_t;
 
 typedef struct {
@@ -106,6 +107,9 @@ typedef struct {
     uint32_t desc[8];
 } pb_topo_view2_t;
 
+/* Most chunk copies a CTA of the depth kernel runs. */
+#define PB_WS_MAX_UNITS 8u
+
 /* One launch of the depth kernels k_label_ws and k_label_wsc (label_ws.cu):
  * batch b is units [b * G, min(nunits, (b + 1) * G)), G = units_per_cta.
  * Unit k is entry k of `units`, or, when that is NULL, copy
@@ -123,7 +127,7 @@ typedef struct {
     uint32_t nunits;
     uint8_t *scratch;
     uint64_t unit_scratch_bytes; /* topo.gpool * 32 */
-    uint32_t units_per_cta;      /* G: 1 to 4 */
+    uint32_t units_per_cta;      /* G: 1 to PB_WS_MAX_UNITS */
     uint32_t team_warps;         /* hashing warps: 7 or 15 */
     uint32_t nbatches;           /* ceil(nunits / G) */
     unsigned int *queue;         /* zeroed work counter */

@@ -91,7 +91,7 @@ struct pose_hbm_topo {
     uint64_t dev_bytes;
     pb_topo_view_t view;
     pb_topo_view2_t view2; /* pipelined records (d_recs2 != NULL) */
-    int occ_ws[2];         /* warp-specialised kernel CTAs/SM for 7 and 15 hashing warps */
+    int occ_ws[2][PB_WS_MAX_UNITS + 1]; /* depth kernel CTAs per SM for 7 and 15 hashing warps, by units per CTA */
     /* levels wider than split_width (ascending), shared by a cluster's CTAs */
     uint32_t *d_split, nsplit, split_width;
     int occ_wsc[4];        /* clusters of 2, 4, 8, 16 CTAs (15 hashing warps) the device holds */
@@ -106,11 +106,6 @@ struct pose_hbm_topo {
     size_t sess_alloc;
     unsigned int *d_queue;
     int occ_team[5], sms; /* k_label CTAs (one team of 2^i warps each) per SM */
-    /* pipelined records for a PB_CSM_MULTI-slot shared pool per unit (the
-     * multi-unit depth kernel's), built on first use */
-    void *d_recs2s;
-    pb_topo_view2_t view2s;
-    pthread_mutex_t lazy_mu; /* guards the first-use build of d_recs2s / view2s */
     /* schedule chosen by pose_b200_topo_autotune for calls of tuned_units chunk copies */
     int tuned_ok;
     uint64_t tuned_units;
@@ -118,24 +113,6 @@ struct pose_hbm_topo {
 };
 
 /* ── schedule model ──────────────────────────────────────────────────────── */
-
-/* Model constants: integer lanes an SM retires per clock for this
- * instruction mix, and the dependent latency of one node label in SM clocks.
- * Defaults come from the compression microbenchmark; POSE_B200_INT_LANES and
- * POSE_B200_LABEL_LATENCY override them. */
-static double model_lanes(void)
-{
-    const char *e = getenv("POSE_B200_INT_LANES");
-    double v = e ? atof(e) : 0.0;
-    return v > 0 ? v : 72.0;
-}
-
-static double model_latency(int cv0)
-{
-    const char *e = getenv("POSE_B200_LABEL_LATENCY");
-    double v = e ? atof(e) : 0.0;
-    return v > 0 ? v : (cv0 ? 6000.0 : 7000.0);
-}
 
 typedef struct {
     uint32_t T, G, teams, grid, cta, kernel, smem;
@@ -145,42 +122,29 @@ typedef struct {
     double cost;
 } plan_t;
 
-#define PB_CSM_LATENCY 2048u /* shared-memory label slots per copy in the pipelined records */
-#define PB_CSM_MULTI 512u    /* the same for the multi-unit depth kernel (four pools per CTA) */
+#define PB_CSM 480u /* shared-memory label slots per copy in the pipelined records */
 #define PB_SPLIT_WIDTH 480u  /* levels a depth-kernel cluster shares: wider than one pass of its hashing threads */
 
-static double model_ws_latency(void)
+static uint32_t ws_smem_bytes(const pose_hbm_topo_t *t, uint32_t nc, uint32_t G)
 {
-    const char *e = getenv("POSE_B200_WS_LATENCY");
-    double v = e ? atof(e) : 0.0;
-    return v > 0 ? v : 2700.0;
+    return pb_ws_smem_bytes(t->view2.csm, G, nc);
 }
 
-static uint32_t ws_smem_bytes(const pose_hbm_topo_t *t, uint32_t nc)
+static int ws_occupancy(pose_hbm_topo_t *t, uint32_t nc, uint32_t G)
 {
-    return pb_ws_smem_bytes(t->view2.csm, 1, nc);
-}
-
-static int ws_occupancy(pose_hbm_topo_t *t, uint32_t nc)
-{
-    int i = nc == 7 ? 0 : 1;
-    if (t->occ_ws[i] < 0) {
+    int *cached = &t->occ_ws[nc == 7 ? 0 : 1][G];
+    if (*cached < 0) {
         int occ = 0;
-        uint32_t smem = ws_smem_bytes(t, nc);
-        if (smem > 227u * 1024u || pb_dev_label_ws_occupancy(32 * (nc + 1), smem, &occ) != 0) occ = 0;
+        if (pb_dev_label_ws_occupancy(32 * (nc + 1), ws_smem_bytes(t, nc, G), &occ) != 0) occ = 0;
         cudaGetLastError();
-        t->occ_ws[i] = occ;
+        *cached = occ;
     }
-    return t->occ_ws[i];
+    return *cached;
 }
 
-/* SM clocks a cluster barrier adds to a level (POSE_B200_CLUSTER_SYNC overrides). */
-static double model_cluster_sync(void)
-{
-    const char *e = getenv("POSE_B200_CLUSTER_SYNC");
-    double v = e ? atof(e) : 0.0;
-    return v > 0 ? v : 1500.0;
-}
+/* Clocks the cluster form of the depth kernel adds to a level, and to one
+ * that the cluster shares. */
+static const double wsc_level = 60.0, wsc_split_sync = 1500.0;
 
 /* Clusters of C CTAs of the depth kernel (15 hashing warps) the device holds
  * at once (0 when C is not 2, 4, 8 or 16, or the kernel cannot run so). */
@@ -190,19 +154,12 @@ static int wsc_clusters(pose_hbm_topo_t *t, uint32_t C)
     if (i < 0 || !t->d_split) return 0;
     if (t->occ_wsc[i] < 0) {
         int n = 0;
-        const uint32_t smem = ws_smem_bytes(t, 15);
+        const uint32_t smem = ws_smem_bytes(t, 15, 1);
         if (smem > 227u * 1024u || pb_dev_label_wsc_max_clusters(C, 15, smem, &n) != 0) n = 0;
         cudaGetLastError();
         t->occ_wsc[i] = n;
     }
     return t->occ_wsc[i];
-}
-
-static uint64_t passes_lanes(const pose_hbm_topo_t *t, uint64_t lanes)
-{
-    uint64_t passes = 0;
-    for (uint32_t k = 0; k < t->nw; k++) passes += t->wcnt[k] * ((t->wval[k] + lanes - 1) / lanes);
-    return passes;
 }
 
 static uint64_t passes_for(const pose_hbm_topo_t *t, uint32_t T, uint32_t G)
@@ -217,86 +174,125 @@ static uint64_t passes_for(const pose_hbm_topo_t *t, uint32_t T, uint32_t G)
 
 static int is_pow2(uint32_t v) { return v && !(v & (v - 1)); }
 
-/* One-warp passes of a batch of G units: sum over levels of ceil(G w / 32).
- * Warps without a node of a level skip it, so this is the batch's ALU work
- * in warp-wide node hashes, idle lanes of partly filled warps included. */
-static uint64_t warp_passes(const pose_hbm_topo_t *t, uint32_t G)
+/* Clocks a level costs beyond its hashing on an SM that holds k lockstep
+ * teams, and clocks of a node there.  With one 16-warp team per SM a level of
+ * n nodes measured 2500 + 15.7 n clocks (n = 159, 299, 435 and 636 nodes an
+ * SM, chunk_blocks 2^12 to 2^16: within 1 %); k teams of n / k nodes each
+ * overlap their overheads in part (k = 2, 3, 4, 7: 1.2, 1.4, 1.6, 1.85 of one
+ * team's).  Without the block-0 table a node is three compressions. */
+static double lockstep_overhead(uint64_t k, int cv0) { return (cv0 ? 2500.0 : 3400.0) * pow((double)k, 0.32); }
+static double lockstep_node(int cv0) { return cv0 ? 15.7 : 23.4; }
+/* A pass after a level's first costs its SM this much more, whatever its size
+ * (256 x 16384 super-chunks, 32 units a team, 1024 teams of 1, 2 and 4 warps:
+ * 45.8, 44.0 and 38.8 k clocks a level). */
+static const double lockstep_more = 600.0;
+/* A team's pass over its threads takes at least this long. */
+static double lockstep_pass(int cv0) { return cv0 ? 4400.0 : 5500.0; }
+
+/* One batch of G units on a team of T warps: its passes, and its warp passes
+ * of 32 lanes (a full pass keeps all T warps, the last one of a level only
+ * those with a node). */
+static void lockstep_passes(const pose_hbm_topo_t *t, uint32_t T, uint32_t G, uint64_t *passes, uint64_t *warps)
 {
-    uint64_t passes = 0;
-    for (uint32_t k = 0; k < t->nw; k++) passes += t->wcnt[k] * (((uint64_t)G * t->wval[k] + 31) / 32);
-    return passes;
+    const uint64_t stride = 32ull * T / G;
+    uint64_t p = 0, wp = 0;
+    for (uint32_t k = 0; k < t->nw; k++) {
+        const uint64_t full = t->wval[k] / stride, rest = t->wval[k] % stride;
+        p += t->wcnt[k] * (full + (rest != 0));
+        wp += t->wcnt[k] * (full * T + (rest * G + 31) / 32);
+    }
+    *passes = p;
+    *warps = wp;
 }
 
-/* Throughput model of one launch.  A team's batch takes at least its
- * latency-bound time (every pass of every level waits for a label: t_lat per
- * pass for the basic kernel; the depth kernel's levels cost its per-level
- * time, further passes of a wide level t_lat), and an SM needs at least its
- * ALU time (the warp passes of the teams resident on it, 32 lanes each, at
- * lanes_clk lane-operations per clock).  A launch runs its full waves of the
- * larger of the two, then the rest of the batches spread over the SMs. */
+/* Depth kernel with 15 hashing warps: clocks of a level of n items.  Measured
+ * per level width with one unit (chunk_blocks 2^17) and with up to seven. */
+static double ws_level(double n)
+{
+    if (n <= 32) return 1930.0;
+    if (n <= 64) return 2480.0;
+    if (n <= 120) return 2480.0 + (n - 64.0) * 12.0;
+    return 2864.0 + 1200.0 * (ceil(n / 480.0) - 1.0) + 15.5 * n;
+}
+
+/* Depth kernel: clocks of `batches` batches of G units through R CTAs, one
+ * per SM. */
+static double ws_cost(const pose_hbm_topo_t *t, uint32_t nc, uint32_t G, uint64_t batches, uint64_t R)
+{
+    double sum = 0;
+    for (uint32_t j = 0; j < t->nw; j++) sum += (double)t->wcnt[j] * ws_level((double)t->wval[j] * G * 15.0 / nc);
+    return sum * (double)((batches + R - 1) / R);
+}
+
+/* The schedule of one launch: the cheapest, by the model above, of
+ *   - the lockstep kernel with T warps and G units a team and k teams per SM
+ *     (G a power of two, or what spreads the units evenly over the SMs in one
+ *     to four waves: at 4096 x 2048 super-chunks 28 units a team on 147 SMs
+ *     take 78 ms, 32 on 128 SMs 84 ms), full waves of teams first and then
+ *     the rest of the batches spread over the SMs;
+ *   - the depth kernel with G units per CTA, one CTA per SM, or with a
+ *     cluster of CTAs per unit. */
 static int make_plan(const pose_hbm_topo_t *ct, uint64_t nunits, const pose_b200_sched_t *hint,
                      uint64_t budget, plan_t *best)
 {
     pose_hbm_topo_t *t = (pose_hbm_topo_t *)ct; /* occupancy cache */
-    const double lanes_clk = model_lanes();
-    const double t_lat = model_latency(t->d_cv0 != NULL);
-    const double item_instr = t->d_cv0 ? 1400.0 : 2080.0;
+    const int cv0 = t->d_cv0 != NULL;
     const int want = hint ? (int)hint->kernel : 0;
     memset(best, 0, sizeof(*best));
     best->cost = -1;
-    for (int kernel = 1; kernel <= 1; kernel++) {
-        if (want && want != kernel) continue;
-        /* One team per CTA (its barrier is the CTA's, so a CTA reserves one
-         * hardware barrier and the SM's barriers never cap residency), so
-         * that any number k of teams per SM can be resident.  Teams pull
-         * batches until the queue is empty, and a batch's time is set by
-         * the ALU share of its SM.  Every k is costed; a k below the
-         * occupancy limit is enforced by padding the CTA's shared memory
-         * (pb_dev_label_balance_smem), so that no SM takes k + 1. */
-        const char *fk = getenv("POSE_B200_TEAMS_PER_SM"); /* forces k (tests, sweeps) */
-        const int force_k = fk ? atoi(fk) : 0;
-        for (uint32_t T = 1, ti = 0; T <= 16; T <<= 1, ti++) {
-            if (hint && hint->team_warps && hint->team_warps != T) continue;
-            const uint32_t cta = 32 * T;
-            const int occ = t->occ_team[ti];
-            if (occ <= 0) continue;
-            for (uint32_t G = 1; G <= 32 && G <= 32 * T; G <<= 1) {
-                if (hint && hint->units_per_team && hint->units_per_team != G) continue;
-                uint64_t slots = t->pool;
-                uint64_t team_scratch = (uint64_t)G * slots * 32;
-                uint64_t batches = (nunits + G - 1) / G;
-                uint64_t memcap = budget / team_scratch;
-                uint64_t passes = passes_for(t, T, G);
-                double lat = (double)passes * t_lat;
-                /* one batch's ALU clocks on an SM of its own: its warp passes
-                 * of 32 lanes, idle lanes included */
-                const double alu1 = (double)warp_passes(t, G) * 32.0 * item_instr / lanes_clk;
-                for (int k = occ; k >= 1; k--) {
-                    if (force_k && k != force_k) continue;
-                    uint64_t R = (uint64_t)t->sms * (uint64_t)k;
-                    if (R > memcap) R = memcap;
-                    if (R > batches) R = batches;
-                    if (hint && hint->max_teams && R > hint->max_teams) R = hint->max_teams;
-                    if (R == 0) continue;
-                    uint64_t sbytes = R * team_scratch;
-                    if (sbytes > budget) continue;
-                    /* full waves of R teams, then the rest, spread over the SMs */
-                    const uint64_t full = batches / R, rest = batches - full * R;
-                    const uint64_t teams_sm = (R + t->sms - 1) / t->sms, rest_sm = (rest + t->sms - 1) / t->sms;
-                    const double alu = (double)teams_sm * alu1, alu_rest = (double)rest_sm * alu1;
-                    double cost = (double)full * (lat > alu ? lat : alu);
-                    if (rest) cost += lat > alu_rest ? lat : alu_rest;
-                    if (best->cost < 0 || cost < best->cost * 0.999 ||
-                        (cost <= best->cost * 1.001 && sbytes < best->scratch_bytes)) {
-                        best->T = T; best->G = G; best->teams = (uint32_t)R;
-                        best->grid = (uint32_t)R; best->cta = cta;
-                        best->team_scratch = team_scratch; best->scratch_bytes = sbytes;
-                        best->cost = cost; best->kernel = (uint32_t)kernel;
-                        /* residency cap when fewer than the occupancy limit
-                         * of teams go on every SM */
-                        best->smem = 0;
-                        best->per_sm = R % t->sms == 0 && R / t->sms < (uint64_t)occ ? (uint32_t)(R / t->sms) : 0;
-                    }
+    /* One team per CTA (its barrier is the CTA's, so a CTA reserves one
+     * hardware barrier and the SM's barriers never cap residency).  A k below
+     * the occupancy limit is enforced by padding the CTA's shared memory
+     * (pb_dev_label_balance_smem), so that no SM takes k + 1. */
+    const char *fk = getenv("POSE_B200_TEAMS_PER_SM"); /* forces k (tests, sweeps) */
+    const int force_k = fk ? atoi(fk) : 0;
+    for (uint32_t T = 1, ti = 0; T <= 16 && (!want || want == 1); T <<= 1, ti++) {
+        if (hint && hint->team_warps && hint->team_warps != T) continue;
+        const int occ = t->occ_team[ti];
+        /* power-of-two G, then the even ones for each k */
+        const int nfix = 6, nk = occ < 4 ? occ : 4;
+        for (int c = 0; c < nfix + 4 * nk; c++) {
+            const int even_k = c < nfix ? 0 : (c - nfix) / 4 + 1;
+            const uint64_t even = even_k ? (uint64_t)even_k * t->sms * (uint64_t)((c - nfix) % 4 + 1) : 0;
+            const uint64_t G64 = c < nfix ? 1ull << c : (nunits + even - 1) / even;
+            if (hint && hint->units_per_team && (even_k || hint->units_per_team != G64)) continue;
+            if (G64 > (even_k ? 64 : 32) || G64 > 32ull * T || (even_k && is_pow2((uint32_t)G64))) continue;
+            const uint32_t G = (uint32_t)G64;
+            const uint64_t team_scratch = (uint64_t)G * t->pool * 32;
+            const uint64_t batches = (nunits + G - 1) / G;
+            const uint64_t memcap = budget / team_scratch;
+            uint64_t passes, warps;
+            lockstep_passes(t, T, G, &passes, &warps);
+            const double lat = (double)passes * lockstep_pass(cv0);
+            const double alu1 = (double)warps * 32.0 * lockstep_node(cv0);
+            const double more = (double)(passes - t->L) * lockstep_more;
+            for (int k = occ; k >= 1; k--) {
+                if (force_k && k != force_k) continue;
+                if (even_k && k != even_k) continue;
+                uint64_t R = (uint64_t)t->sms * (uint64_t)k;
+                if (R > memcap) R = memcap;
+                if (R > batches) R = batches;
+                if (hint && hint->max_teams && R > hint->max_teams) R = hint->max_teams;
+                if (R == 0) continue;
+                const uint64_t sbytes = R * team_scratch;
+                const uint64_t full = batches / R, rest = batches - full * R;
+                const uint64_t teams_sm = (R + t->sms - 1) / t->sms, rest_sm = (rest + t->sms - 1) / t->sms;
+                const double wave = t->L * lockstep_overhead(teams_sm, cv0) + more + (double)teams_sm * alu1;
+                double cost = (double)full * (lat > wave ? lat : wave);
+                if (rest) {
+                    const double last = t->L * lockstep_overhead(rest_sm, cv0) + more + (double)rest_sm * alu1;
+                    cost += lat > last ? lat : last;
+                }
+                if (best->cost < 0 || cost < best->cost * 0.999 ||
+                    (cost <= best->cost * 1.001 && sbytes < best->scratch_bytes)) {
+                    best->T = T; best->G = G; best->teams = (uint32_t)R;
+                    best->grid = (uint32_t)R; best->cta = 32 * T;
+                    best->team_scratch = team_scratch; best->scratch_bytes = sbytes;
+                    best->cost = cost; best->kernel = 1;
+                    best->smem = 0;
+                    /* residency cap when fewer than the occupancy limit
+                     * of teams go on every SM */
+                    best->per_sm = R % t->sms == 0 && R / t->sms < (uint64_t)occ ? (uint32_t)(R / t->sms) : 0;
                 }
             }
         }
@@ -317,52 +313,47 @@ static int make_plan(const pose_hbm_topo_t *ct, uint64_t nunits, const pose_b200
         uint64_t team_scratch = (uint64_t)(t->view2.gpool ? t->view2.gpool : 1) * 32;
         uint64_t sbytes = nunits * team_scratch;
         if (sbytes > budget) continue;
-        uint64_t passes = passes_lanes(t, 32ull * nc);
-        /* the cluster form runs every level ~250 clocks slower than the
-         * one-CTA kernel (measured at 2^17: 742 ms against 693 ms with only
-         * 169 shared levels), so it pays only where wide levels dominate */
-        double lat = (double)t->L * (model_ws_latency() + 250.0) + (double)(passes - t->L) * t_lat / C +
-                     2.0 * t->nsplit * model_cluster_sync();
+        double lat = 0;
+        for (uint32_t j = 0; j < t->nw; j++) {
+            const double n = (double)t->wval[j];
+            lat += (double)t->wcnt[j] * (n > t->split_width ? ws_level(n / C > 480.0 ? n / C : 480.0) + wsc_split_sync
+                                                            : ws_level(n) + wsc_level);
+        }
         double cost = lat;
         if (best->cost < 0 || cost < best->cost * 0.999) {
             best->T = nc; best->G = 1; best->teams = (uint32_t)nunits;
             best->grid = (uint32_t)(nunits * C); best->cta = 32 * (nc + 1);
             best->team_scratch = team_scratch; best->scratch_bytes = sbytes;
-            best->cost = cost; best->kernel = 3; best->smem = ws_smem_bytes(t, nc);
+            best->cost = cost; best->kernel = 3; best->smem = ws_smem_bytes(t, nc, 1);
             best->per_sm = 0;
             best->cluster = C;
         }
     }
-    /* warp-specialised kernel: one chunk copy per CTA, NC hashing warps */
+    /* depth kernel: G units per CTA, one CTA of 15 hashing warps per SM (of 7
+     * on request); two CTAs of 7 measured slower at equal units per SM
+     * (chunk_blocks 2^14, 2 units: 3034 against 2714 clocks a level) */
     for (uint32_t nc = 7; nc <= 15 && t->d_recs2 && (!want || want == 3); nc += 8) {
-        if (hint && hint->team_warps && hint->team_warps != nc) continue;
-        if (hint && hint->units_per_team > 1) continue;
-        if (hint && hint->cluster_ctas > 1) continue;
-        int occ = ws_occupancy(t, nc);
-        if (occ <= 0) continue;
-        uint64_t team_scratch = (uint64_t)(t->view2.gpool ? t->view2.gpool : 1) * 32;
-        uint64_t batches = nunits;
-        uint64_t cap = (uint64_t)t->sms * occ;
-        uint64_t memcap = budget / team_scratch;
-        uint64_t R = cap < memcap ? cap : memcap;
-        if (R > batches) R = batches;
-        if (hint && hint->max_teams && R > hint->max_teams) R = hint->max_teams;
-        if (R == 0) continue;
-        uint64_t waves = (batches + R - 1) / R;
-        uint64_t passes = passes_lanes(t, 32ull * nc);
-        double lat = (double)t->L * model_ws_latency() + (double)(passes - t->L) * t_lat;
-        double teams_sm = (double)((R + t->sms - 1) / t->sms);
-        double alu = teams_sm * (double)t->S * item_instr / lanes_clk;
-        double cost = (double)waves * (lat > alu ? lat : alu);
-        uint64_t sbytes = R * team_scratch;
-        if (sbytes > budget) continue;
-        if (best->cost < 0 || cost < best->cost * 0.999) {
-            best->T = nc; best->G = 1; best->teams = (uint32_t)R;
-            best->grid = (uint32_t)R; best->cta = 32 * (nc + 1);
-            best->team_scratch = team_scratch; best->scratch_bytes = sbytes;
-            best->cost = cost; best->kernel = 3; best->smem = ws_smem_bytes(t, nc);
-            best->per_sm = 0;
-            best->cluster = 1;
+        if (hint && hint->team_warps ? hint->team_warps != nc : nc != 15) continue;
+        if (hint && (hint->units_per_team > 1 || hint->cluster_ctas > 1)) continue;
+        for (uint32_t G = 1; G <= PB_WS_MAX_UNITS; G++) {
+            if (hint && hint->units_per_team && hint->units_per_team != G) continue;
+            if (ws_occupancy(t, nc, G) <= 0) continue;
+            const uint64_t team_scratch = (uint64_t)(t->view2.gpool ? t->view2.gpool : 1) * 32 * G;
+            const uint64_t batches = (nunits + G - 1) / G;
+            const uint64_t memcap = budget / team_scratch;
+            uint64_t R = (uint64_t)t->sms < memcap ? (uint64_t)t->sms : memcap;
+            if (R > batches) R = batches;
+            if (hint && hint->max_teams && R > hint->max_teams) R = hint->max_teams;
+            if (R == 0) continue;
+            const double cost = ws_cost(t, nc, G, batches, R);
+            if (best->cost < 0 || cost < best->cost * 0.999) {
+                best->T = nc; best->G = G; best->teams = (uint32_t)R;
+                best->grid = (uint32_t)R; best->cta = 32 * (nc + 1);
+                best->team_scratch = team_scratch; best->scratch_bytes = R * team_scratch;
+                best->cost = cost; best->kernel = 3; best->smem = ws_smem_bytes(t, nc, G);
+                best->per_sm = 0;
+                best->cluster = 1;
+            }
         }
     }
     return best->cost < 0 ? -1 : 0;
@@ -453,7 +444,6 @@ void pose_graph_hbm_topo_free(pose_hbm_topo_t *t)
     if (t->stream) free_workspace(t);
     cudaFree(t->d_recs);
     cudaFree(t->d_recs2);
-    cudaFree(t->d_recs2s);
     cudaFree(t->d_split);
     cudaFree(t->d_cv0);
     cudaFree(t->d_orank);
@@ -464,7 +454,6 @@ void pose_graph_hbm_topo_free(pose_hbm_topo_t *t)
     if (prev >= 0 && prev != t->device) cudaSetDevice(prev);
     free(t->wval);
     free(t->wcnt);
-    pthread_mutex_destroy(&t->lazy_mu);
     free(t);
 }
 
@@ -483,14 +472,13 @@ static pose_hbm_topo_t *pose_b200_topo_build_impl(uint32_t chunk_blocks, int wit
         return NULL;
     }
     pb_topo_host_t h;
-    if (pb_topo_host_build_ex(cb, with_cv0_table ? PB_CSM_LATENCY : 0, &h) != 0) {
+    if (pb_topo_host_build_ex(cb, with_cv0_table ? PB_CSM : 0, &h) != 0) {
         set_err("pose_graph_hbm_topo_build: schedule build failed for chunk_blocks %u", cb);
         return NULL;
     }
     pose_hbm_topo_t *t = (pose_hbm_topo_t *)calloc(1, sizeof(*t));
     uint32_t *ws = NULL;
     if (!t) { set_err("pose_graph_hbm_topo_build: out of host memory"); goto fail_host; }
-    pthread_mutex_init(&t->lazy_mu, NULL);
     cudaGetDevice(&t->device);
     t->cb = cb;
     t->super_bytes = (uint64_t)cb * 32;
@@ -608,7 +596,7 @@ fail:
 fail_host:
     free(ws);
     pb_topo_host_free(&h);
-    if (t) { free(t->wval); free(t->wcnt); pthread_mutex_destroy(&t->lazy_mu); free(t); }
+    if (t) { free(t->wval); free(t->wcnt); free(t); }
     return NULL;
 }
 
@@ -698,6 +686,18 @@ static int autotune_candidates(pose_hbm_topo_t *t, uint64_t nunits, uint64_t bud
             c[n].s.kernel = 1; c[n].s.team_warps = p.T; c[n].s.units_per_team = p.G; c[n].s.max_teams = p.teams;
             c[n].cost = p.cost; c[n].group = T; n++;
         }
+    /* each team size with the G that the model picks, where that is no power
+     * of two (units_per_team 0: a caller's own schedule takes powers of two) */
+    for (uint32_t T = 1; T <= 16 && n < PB_TUNE_MAX - 4; T <<= 1) {
+        pose_b200_sched_t h;
+        memset(&h, 0, sizeof(h));
+        h.kernel = 1; h.team_warps = T;
+        plan_t p;
+        if (make_plan(t, nunits, &h, budget, &p) != 0 || is_pow2(p.G)) continue;
+        memset(&c[n], 0, sizeof(c[n]));
+        c[n].s.kernel = 1; c[n].s.team_warps = T; c[n].s.max_teams = p.teams;
+        c[n].cost = p.cost; c[n].group = T; n++;
+    }
     /* the depth kernel alone and with a cluster of 2, 4 or 8 CTAs per copy */
     for (uint32_t cl = 1; cl <= 8 && n < PB_TUNE_MAX; cl <<= 1) {
         pose_b200_sched_t h;
@@ -707,7 +707,7 @@ static int autotune_candidates(pose_hbm_topo_t *t, uint64_t nunits, uint64_t bud
         plan_t p;
         if (make_plan(t, nunits, &h, budget, &p) != 0) continue;
         memset(&c[n], 0, sizeof(c[n]));
-        c[n].s.kernel = 3; c[n].s.team_warps = p.T; c[n].s.units_per_team = 1; c[n].s.max_teams = p.teams;
+        c[n].s.kernel = 3; c[n].s.team_warps = p.T; c[n].s.units_per_team = p.G == 1 ? 1 : 0; c[n].s.max_teams = p.teams;
         c[n].s.cluster_ctas = p.cluster;
         c[n].cost = p.cost; c[n].group = 0; n++;
     }
@@ -912,7 +912,7 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
             p.team_scratch_bytes = plan.team_scratch;
             p.nunits = (uint32_t)(n * t->copies);
             p.copies_log2 = t->copies == 2 ? 1 : 0;
-            p.g_log2 = (uint32_t)__builtin_ctz(plan.G);
+            p.units_per_team = plan.G;
             p.team_warps = plan.T;
             p.nbatches = (uint32_t)((p.nunits + plan.G - 1) / plan.G);
             p.queue = t->d_queue;
@@ -924,8 +924,8 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
                 pp.topo = t->view2;
                 pp.seeds = p.seeds; pp.persist = p.persist; pp.super_bytes = p.super_bytes;
                 pp.first_super = p.first_super; pp.scratch = p.scratch;
-                pp.unit_scratch_bytes = plan.team_scratch; pp.nunits = p.nunits;
-                pp.copies_log2 = p.copies_log2; pp.units_per_cta = 1; pp.team_warps = p.team_warps;
+                pp.unit_scratch_bytes = plan.team_scratch / plan.G; pp.nunits = p.nunits;
+                pp.copies_log2 = p.copies_log2; pp.units_per_cta = plan.G; pp.team_warps = p.team_warps;
                 pp.nbatches = p.nbatches; pp.queue = p.queue;
                 if (plan.cluster > 1) {
                     pp.cluster = plan.cluster;
@@ -1228,47 +1228,10 @@ int pb_topo_internal(const pose_hbm_topo_t *t, pb_topo_internal_t *out)
     return 0;
 }
 
-int pb_topo_view2_small(const pose_hbm_topo_t *ct, pb_topo_view2_t *out)
+int pb_topo_view2(const pose_hbm_topo_t *t, pb_topo_view2_t *out)
 {
-    pose_hbm_topo_t *t = (pose_hbm_topo_t *)ct; /* the record set is built once and kept */
     if (!t || !out || !t->d_cv0 || !t->d_recs2) return -1;
-    /* several host threads may create batches on one topology at once: the
-     * first one builds the records, the others wait for it and reuse them */
-    pthread_mutex_lock(&t->lazy_mu);
-    if (!t->d_recs2s) {
-        pb_topo_host_t h;
-        if (pb_topo_host_build_ex(t->cb, PB_CSM_MULTI, &h) != 0) {
-            pthread_mutex_unlock(&t->lazy_mu);
-            return -1;
-        }
-        /* the same levels and node order as the default records; only the
-         * pool slots differ */
-        int ok = h.recs2 && h.S == t->S && h.L == t->L;
-        int prev = -1;
-        cudaGetDevice(&prev);
-        if (ok && prev != t->device) ok = cudaSetDevice(t->device) == cudaSuccess;
-        if (ok) ok = pb_dev_malloc(&t->d_recs2s, (size_t)h.S * 32) == cudaSuccess;
-        if (ok) ok = cudaMemcpy(t->d_recs2s, h.recs2, (size_t)h.S * 32, cudaMemcpyHostToDevice) == cudaSuccess;
-        if (ok) {
-            t->view2s = t->view2;
-            t->view2s.recs2 = (const pb_u4 *)t->d_recs2s;
-            t->view2s.csm = h.csm;
-            t->view2s.gpool = h.gpool2;
-            t->dev_bytes += (uint64_t)h.S * 32;
-        } else {
-            cudaFree(t->d_recs2s);
-            t->d_recs2s = NULL;
-            cudaGetLastError();
-        }
-        if (prev >= 0 && prev != t->device) cudaSetDevice(prev);
-        pb_topo_host_free(&h);
-        if (!ok) {
-            pthread_mutex_unlock(&t->lazy_mu);
-            return -1;
-        }
-    }
-    *out = t->view2s;
-    pthread_mutex_unlock(&t->lazy_mu);
+    *out = t->view2;
     return 0;
 }
 

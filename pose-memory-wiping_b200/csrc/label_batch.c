@@ -239,7 +239,7 @@ int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, 
                 bs[q].b.topo = (uint32_t)k;
                 bs[q].b.first_unit = (uint32_t)(ufirst[k] + f);
                 bs[q].b.count = nunits_t[k] - f < G[k] ? nunits_t[k] - f : G[k];
-                bs[q].b.glog = (uint32_t)__builtin_ctz(G[k]);
+                bs[q].b.G = G[k];
                 bs[q].cost = passes;
                 if (passes > out->max_chain) out->max_chain = passes;
                 q++;
@@ -640,7 +640,7 @@ no_split:
             const char *ek = getenv("POSE_B200_DEEP_KERNEL");
             const char *eg = getenv("POSE_B200_DEEP_UNITS");
             if (eg && eg[0] >= '1' && eg[0] <= '4' && !eg[1]) G = (uint32_t)(eg[0] - '0');
-            int wsg = !(ek && ek[0] == '0') && one_topo && pb_topo_view2_small(pd[0].topo, &v2) == 0;
+            int wsg = !(ek && ek[0] == '0') && one_topo && pb_topo_view2(pd[0].topo, &v2) == 0;
             if (wsg) {
                 const uint64_t grid = (dunits + G - 1) / G < sms ? (dunits + G - 1) / G : sms;
                 wsg = grid * ((uint64_t)v2.gpool * 32 * G) <= budget;
@@ -672,7 +672,7 @@ no_split:
                     if (eu && eu[0] >= '1' && eu[0] <= '4' && !eu[1]) G2 = (uint32_t)(eu[0] - '0');
                     const uint32_t left = sms > b->part[1].grid ? sms - b->part[1].grid : 0;
                     uint32_t max_smem2 = 0;
-                    int ok2 = left > 0 && pb_topo_view2_small(pd2[0].topo, &v2b) == 0 &&
+                    int ok2 = left > 0 && pb_topo_view2(pd2[0].topo, &v2b) == 0 &&
                               pb_dev_label_ws_prepare(&max_smem2) == 0 &&
                               pb_ws_smem_bytes(v2b.csm, G2, 15) <= max_smem2;
                     cudaGetLastError();

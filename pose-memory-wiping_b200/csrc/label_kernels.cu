@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128) k_chunk_seeds(const uint8_t *__restrict__
 /* What one thread needs to run its unit through the levels. */
 struct UnitCtx {
     uint4 *tscr;       /* team scratch, label (slot, u) at (slot*G + u)*2 */
-    uint32_t glog, u, q, stride;
+    uint32_t G, u, q, stride; /* G units a team; this thread: unit u, nodes q, q + stride, ... */
     bool valid;
     uint32_t id_off, rank_base, rank_lim;
     uint8_t *out;      /* persisted super-chunk of this unit's chunk */
@@ -202,7 +202,7 @@ __device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const Uni
                 const uint32_t np = (rec.x >> PB_REC_NP_SHIFT) & 3u;
                 uint32_t m[16];
                 if (np >= 1) {
-                    const uint4 *s = c.tscr + (((size_t)rec.y << c.glog) + c.u) * 2;
+                    const uint4 *s = c.tscr + ((size_t)rec.y * c.G + c.u) * 2;
                     uint4 a = s[0], b = s[1];
                     m[0] = a.x; m[1] = a.y; m[2] = a.z; m[3] = a.w;
                     m[4] = b.x; m[5] = b.y; m[6] = b.z; m[7] = b.w;
@@ -211,7 +211,7 @@ __device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const Uni
                     for (int i = 0; i < 8; i++) m[i] = 0;
                 }
                 if (np >= 2) {
-                    const uint4 *s = c.tscr + (((size_t)rec.z << c.glog) + c.u) * 2;
+                    const uint4 *s = c.tscr + ((size_t)rec.z * c.G + c.u) * 2;
                     uint4 a = s[0], b = s[1];
                     m[8] = a.x; m[9] = a.y; m[10] = a.z; m[11] = a.w;
                     m[12] = b.x; m[13] = b.y; m[14] = b.z; m[15] = b.w;
@@ -238,7 +238,7 @@ __device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const Uni
                 compress(cv, m2, 64, kFlagsBlock2);
                 const uint4 o0 = make_uint4(cv[0], cv[1], cv[2], cv[3]);
                 const uint4 o1 = make_uint4(cv[4], cv[5], cv[6], cv[7]);
-                uint4 *d = c.tscr + (((size_t)rec.w << c.glog) + c.u) * 2;
+                uint4 *d = c.tscr + ((size_t)rec.w * c.G + c.u) * 2;
                 d[0] = o0;
                 d[1] = o1;
                 if (rec.x & PB_REC_OUT_BIT) {
@@ -288,17 +288,17 @@ __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant_
     const pb_topo_view_t &tp = p.topo;
     __shared__ uint32_t s_batch[1];
     UnitCtx c;
-    c.glog = p.g_log2;
-    c.u = tt & ((1u << c.glog) - 1);
-    c.q = tt >> c.glog;
-    c.stride = TT >> c.glog;
+    c.G = p.units_per_team;
+    c.q = tt / c.G;
+    c.u = tt - c.q * c.G;
+    c.stride = TT / c.G;
     c.tscr = reinterpret_cast<uint4 *>(p.scratch + gteam * p.team_scratch_bytes);
 
     for (;;) {
         const uint32_t batch = grab_batch<true>(p.queue, T, team, tt, bar_id, TT, s_batch);
         if (batch >= p.nbatches) break;
-        const uint32_t unit = (batch << c.glog) + c.u;
-        c.valid = unit < p.nunits;
+        const uint32_t unit = batch * c.G + c.u;
+        c.valid = c.q < c.stride && unit < p.nunits; /* TT - stride * G threads have no unit */
         const uint32_t chunk = unit >> p.copies_log2;
         const uint32_t copy = unit & ((1u << p.copies_log2) - 1u);
         c.id_off = copy ? tp.S : 0u;
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant_
 }
 
 /* Many topologies in one launch: teams take batches (same topology, up to
- * G = 2^glog units) from a queue sorted longest first, and copy the batch's
+ * G units) from a queue sorted longest first, and copy the batch's
  * topology view into shared memory.  One team of T warps per CTA
  * (blockDim.x == 32 T), ending its levels with the CTA barrier. */
 __global__ void __launch_bounds__(PB_MULTI_CTA_THREADS, 3) k_label_multi(const __grid_constant__ pb_multi_params_t p)
@@ -338,11 +338,11 @@ __global__ void __launch_bounds__(PB_MULTI_CTA_THREADS, 3) k_label_multi(const _
                 reinterpret_cast<const uint32_t *>(p.topos + bd.topo)[tt];
         team_sync<true>(T, bar_id, TT);
         const pb_topo_view_t &tp = s_topo[team];
-        c.glog = bd.glog;
-        c.u = tt & ((1u << c.glog) - 1);
-        c.q = tt >> c.glog;
-        c.stride = TT >> c.glog;
-        c.valid = c.u < bd.count;
+        c.G = bd.G;
+        c.q = tt / c.G;
+        c.u = tt - c.q * c.G;
+        c.stride = TT / c.G;
+        c.valid = c.q < c.stride && c.u < bd.count;
         const pb_munit_t un = p.units[bd.first_unit + (c.valid ? c.u : 0)];
         const uint32_t copy = un.copy;
         c.id_off = copy ? tp.S : 0u;

@@ -139,7 +139,7 @@ extern "C" int pose_b200_topo_label_noalloc(const pose_hbm_topo_t *topo, const u
         p.team_scratch_bytes = plan.team_scratch;
         p.nunits = (uint32_t)(n * ti.copies);
         p.copies_log2 = ti.copies == 2 ? 1 : 0;
-        p.g_log2 = (uint32_t)__builtin_ctz(plan.G);
+        p.units_per_team = plan.G;
         p.team_warps = plan.T;
         p.nbatches = (uint32_t)((p.nunits + plan.G - 1) / plan.G);
         p.queue = na.queue;

@@ -195,20 +195,16 @@ static void arena_give(pose_b200_server_t *s, uint64_t off, uint64_t len)
     }
 }
 
-/* Whether a request runs on the depth kernel: a deep topology whose 512-slot
- * records the multi-unit depth kernel has (built here on first use: call
- * without the server lock held), on a GPU whose CTAs hold the kernel's
- * shared memory, with one chunk copy's scratch fitting the arena
- * (otherwise it joins a wave like the others). */
+/* Whether a request runs on the depth kernel: a deep topology built with its
+ * block-0 table, on a GPU whose CTAs hold the kernel's shared memory, with
+ * one chunk copy's scratch fitting the arena (otherwise it joins a wave like
+ * the others). */
 static int req_is_deep(const pose_b200_server_t *s, const pose_hbm_topo_t *topo)
 {
     pb_topo_internal_t ti;
     pb_topo_view2_t v2;
     if (!s->wsg_smem_max || pb_topo_internal(topo, &ti) != 0 || ti.view.L < s->deep_levels) return 0;
-    if (pb_topo_view2_small(topo, &v2) != 0) {
-        cudaGetLastError();
-        return 0;
-    }
+    if (pb_topo_view2(topo, &v2) != 0) return 0;
     return pb_ws_smem_bytes(v2.csm, 4, PB_SERVER_DEEP_WARPS) <= s->wsg_smem_max &&
            (uint64_t)v2.gpool * 32 <= s->arena_bytes;
 }
@@ -292,7 +288,7 @@ static int admit_deep(pose_b200_server_t *s)
     const pose_hbm_topo_t *topo = s->reqs[i0].topo;
     pb_topo_internal_t ti;
     pb_topo_view2_t v2;
-    if (pb_topo_internal(topo, &ti) != 0 || pb_topo_view2_small(topo, &v2) != 0) return 0;
+    if (pb_topo_internal(topo, &ti) != 0 || pb_topo_view2(topo, &v2) != 0) return 0;
     const uint32_t free_sms = s->deep_ctas < s->sms ? s->sms - s->deep_ctas : 0;
     const uint64_t units0 = (s->reqs[i0].len / ti.super_bytes) * ti.copies;
     size_t pending = 0;
@@ -878,8 +874,7 @@ out:
 int pose_b200_server_prepare(pose_b200_server_t *s, const pose_hbm_topo_t *topo)
 {
     if (!s || !topo) return -1;
-    (void)req_is_deep(s, topo); /* builds the depth kernel's records of a deep topology */
-    return 0;
+    return 0; /* the topology has all that its requests need */
 }
 
 int64_t pose_b200_server_submit(pose_b200_server_t *s, const pose_hbm_topo_t *topo, int session, void *dev_ptr,
@@ -887,7 +882,6 @@ int64_t pose_b200_server_submit(pose_b200_server_t *s, const pose_hbm_topo_t *to
 {
     if (!s || !topo) return -1;
     const double t_submit = now_ms(); /* latency counts from the call, lock wait included */
-    /* before the lock: a deep topology's first request builds its records */
     const int deep = req_is_deep(s, topo);
     pthread_mutex_lock(&s->mu);
     int64_t id = -1;

@@ -9,7 +9,7 @@
  * records, block-0 chaining values and predecessors born earlier — is taken
  * off that path, using the pipelined records of topology.c (PB_REF_*):
  *
- *   CTA = NC hashing warps + 1 producer warp; G (1 to 4) chunk copies of one
+ *   CTA = NC hashing warps + 1 producer warp; G (1 to 8) chunk copies of one
  *   topology ("units") run in lockstep, so a level of width w is w * G items
  *   (item k: node k / G of unit k % G).
  *   During level l the producer
@@ -90,7 +90,9 @@ __device__ __forceinline__ void put8(uint32_t *w, uint4 a, uint4 b)
  *   ctx   [G][2]         UnitCtx of each unit
  *   msg   [G][4]         block 2 of each unit: chunk seed | descriptor
  *   tab   [G][28]        the same laid out for quads (quad_table_entry)
- *   pool  [G][csm][2]    next-level labels of each unit
+ *   pool  [csm][G][2]    next-level labels, slot-major: the G lanes of a node
+ *                        read and write neighbouring entries (one pool after
+ *                        another would put them all on the same banks)
  *   rec   [3][slots][2]  records, ring of three levels
  *   dat   [2][nthr][6]   per item: block-0 value, predecessor 0, predecessor 1
  * with nthr = 32 NC hashing threads and slots = nthr / G staged nodes. */
@@ -104,7 +106,7 @@ struct Layout {
     static constexpr uint32_t zero = 0, hdr = 2;
     __device__ __forceinline__ uint32_t r(uint32_t st, uint32_t j) const { return rec + (st * slots + j) * 2; }
     __device__ __forceinline__ uint32_t d(uint32_t st, uint32_t k) const { return dat + (st * nthr + k) * 6; }
-    __device__ __forceinline__ uint32_t upool(uint32_t u) const { return pool + u * csm * 2; }
+    __device__ __forceinline__ uint32_t upool(uint32_t u) const { return pool + 2 * u; }
 };
 
 struct __align__(16) UnitCtx {
@@ -134,17 +136,18 @@ __device__ __forceinline__ bool from_global(uint32_t ref)
     return (ref & (PB_REF_PREV | PB_REF_SMEM)) == PB_REF_PREV;
 }
 
-__device__ __forceinline__ uint32_t operand_at(uint32_t ref, bool have, uint32_t pool, uint32_t staged)
+__device__ __forceinline__ uint32_t operand_at(uint32_t ref, bool have, uint32_t pool, uint32_t staged, uint32_t G2)
 {
     if (!have) return Layout::zero;
     if (!(ref & PB_REF_PREV)) return staged;
-    return (ref & PB_REF_SMEM) ? pool + (ref & PB_REF_SLOT_MASK) * 2 : Layout::zero;
+    return (ref & PB_REF_SMEM) ? pool + (ref & PB_REF_SLOT_MASK) * G2 : Layout::zero;
 }
 
 /* Descriptor of a staged item: record at smem[rec], operands staged at dat
  * index `item`; an empty one when !ok.  Free of branches, so that its loads
  * and selects fill the issue slots that a compression leaves idle. */
-__device__ __forceinline__ Desc load_desc(const uint4 *smem, bool ok, uint32_t rec, uint32_t item, uint32_t pool)
+__device__ __forceinline__ Desc load_desc(const uint4 *smem, bool ok, uint32_t rec, uint32_t item, uint32_t pool,
+                                          uint32_t G2)
 {
     const uint32_t at = ok ? rec : Layout::zero;
     const uint4 r0 = smem[at];
@@ -157,8 +160,8 @@ __device__ __forceinline__ Desc load_desc(const uint4 *smem, bool ok, uint32_t r
     d.gslot = ok ? r0.w : PB_NO_SLOT;
     d.sslot = ok ? r1.x : PB_NO_SLOT;
     d.rank = r1.y;
-    d.s0 = operand_at(r0.y, np >= 1, pool, item + 2) * 16;
-    d.s1 = operand_at(r0.z, np >= 2, pool, item + 4) * 16;
+    d.s0 = operand_at(r0.y, np >= 1, pool, item + 2, G2) * 16;
+    d.s1 = operand_at(r0.z, np >= 2, pool, item + 4, G2) * 16;
     d.v = item * 16;
     return d;
 }
@@ -289,21 +292,23 @@ __device__ __forceinline__ void lane_hash(const uint4 *smem, uint32_t msg, uint3
 
 /* A label of a directly loaded item: pool is the unit's shared-memory pool
  * (of this CTA, or of the cluster's rank 0). */
-__device__ __forceinline__ void load_label(uint32_t *w, uint32_t ref, const uint4 *pool, const uint4 *gscr)
+__device__ __forceinline__ void load_label(uint32_t *w, uint32_t ref, const uint4 *pool, uint32_t G2,
+                                           const uint4 *gscr)
 {
-    const uint4 *s = (ref & (PB_REF_PREV | PB_REF_SMEM)) == (PB_REF_PREV | PB_REF_SMEM) ? pool : gscr;
-    s += (size_t)(ref & PB_REF_SLOT_MASK) * 2;
+    const uint32_t slot = ref & PB_REF_SLOT_MASK;
+    const uint4 *s = (ref & (PB_REF_PREV | PB_REF_SMEM)) == (PB_REF_PREV | PB_REF_SMEM) ? pool + (size_t)slot * G2
+                                                                                        : gscr + (size_t)slot * 2;
     put8(w, s[0], s[1]);
 }
 
 __device__ __forceinline__ void lane_store(const uint32_t (&cv)[8], uint32_t x, uint32_t gslot, uint32_t sslot,
-                                           uint32_t rank, uint4 *pool, const UnitCtx *cx)
+                                           uint32_t rank, uint4 *pool, uint32_t G2, const UnitCtx *cx)
 {
     const uint4 o0 = make_uint4(cv[0], cv[1], cv[2], cv[3]);
     const uint4 o1 = make_uint4(cv[4], cv[5], cv[6], cv[7]);
     if (sslot != PB_NO_SLOT) {
-        pool[(size_t)sslot * 2] = o0;
-        pool[(size_t)sslot * 2 + 1] = o1;
+        pool[(size_t)sslot * G2] = o0;
+        pool[(size_t)sslot * G2 + 1] = o1;
     }
     if (gslot != PB_NO_SLOT) {
         uint4 *d = cx->gscr + (size_t)gslot * 2;
@@ -329,8 +334,8 @@ __device__ __forceinline__ void load_direct(const P &p, uint32_t pos, const Unit
     const uint32_t np = (r0.x >> PB_REC_NP_SHIFT) & 3u;
 #pragma unroll
     for (int i = 0; i < 16; i++) m[i] = 0;
-    if (np >= 1) load_label(m, r0.y, pool, cx->gscr);
-    if (np >= 2) load_label(m + 8, r0.z, pool, cx->gscr);
+    if (np >= 1) load_label(m, r0.y, pool, 2 * p.units_per_cta, cx->gscr);
+    if (np >= 2) load_label(m + 8, r0.z, pool, 2 * p.units_per_cta, cx->gscr);
     const uint4 *c = p.topo.cv0 + ((size_t)cx->copy * p.topo.S + pos) * 2;
     put8(cv, __ldg(c), __ldg(c + 1));
     x = r0.x; gslot = r0.w; sslot = r1.x; rank = r1.y;
@@ -374,8 +379,8 @@ struct NextLevel {
             d.rank = r1.y;
         } else if (R == 4) {
             const uint32_t np = (r0.x >> PB_REC_NP_SHIFT) & 3u; /* 0 for the empty record */
-            d.s0 = operand_at(r0.y, np >= 1, pool, item + 2) * 16;
-            d.s1 = operand_at(r0.z, np >= 2, pool, item + 4) * 16;
+            d.s0 = operand_at(r0.y, np >= 1, pool, item + 2, 2 * G) * 16;
+            d.s1 = operand_at(r0.z, np >= 2, pool, item + 4, 2 * G) * 16;
             d.v = item * 16 + lane4;
         } else if (R == 5) {
             global = __any_sync(0xFFFFFFFFu, from_global(d.y) || from_global(d.z));
@@ -450,12 +455,12 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
 
     __syncthreads(); /* levels 0 and 1 are staged */
     const auto quad_desc = [&](uint32_t lv, uint32_t st, uint32_t wl) {
-        Desc n = load_desc(smem, ok4 && j4 < wl, o.r(st, j4), o.d(lv & 1, k4), pool4);
+        Desc n = load_desc(smem, ok4 && j4 < wl, o.r(st, j4), o.d(lv & 1, k4), pool4, 2 * G);
         n.v += 4 * q.i;
         return n;
     };
     const auto lane_desc = [&](uint32_t lv, uint32_t st, uint32_t wl) {
-        return load_desc(smem, ok1 && j1 < wl, o.r(st, j1), o.d(lv & 1, c), pool1);
+        return load_desc(smem, ok1 && j1 < wl, o.r(st, j1), o.d(lv & 1, c), pool1, 2 * G);
     };
     /* The level's start and width, this warp's part in it, and the ring stage
      * of the next level. */
@@ -503,8 +508,8 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
                 put8(m, at16(smem, d.s0), at16(smem, d.s0 + 16));
                 put8(m + 8, at16(smem, d.s1), at16(smem, d.s1 + 16));
                 if (global) {
-                    if (from_global(d.y)) load_label(m, d.y, nullptr, gscr4);
-                    if (from_global(d.z)) load_label(m + 8, d.z, nullptr, gscr4);
+                    if (from_global(d.y)) load_label(m, d.y, nullptr, 0, gscr4);
+                    if (from_global(d.z)) load_label(m + 8, d.z, nullptr, 0, gscr4);
                 }
                 NextLevel n;
                 n.smem = smem; n.G = G; n.quad_max = quad_max; n.warp = warp; n.j4 = j4; n.pool = pool4;
@@ -513,7 +518,7 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
                 quad_compress(va, vb, m, kFlagsBlock1, q, n);
                 quad_compress_table(va, vb, tab_first, tab4, kFlagsBlock2, q);
                 if (d.sslot != PB_NO_SLOT) {
-                    uint32_t *t = reinterpret_cast<uint32_t *>(smem + pool4 + d.sslot * 2) + q.i;
+                    uint32_t *t = reinterpret_cast<uint32_t *>(smem + pool4 + d.sslot * 2 * G) + q.i;
                     t[0] = va;
                     t[4] = vb;
                 }
@@ -562,14 +567,14 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
                         put8(m, at16(smem, dl.s0), at16(smem, dl.s0 + 16));
                         put8(m + 8, at16(smem, dl.s1), at16(smem, dl.s1 + 16));
                         put8(cv, at16(smem, dl.v), at16(smem, dl.v + 16));
-                        if (from_global(dl.y)) load_label(m, dl.y, nullptr, cx->gscr);
-                        if (from_global(dl.z)) load_label(m + 8, dl.z, nullptr, cx->gscr);
+                        if (from_global(dl.y)) load_label(m, dl.y, nullptr, 0, cx->gscr);
+                        if (from_global(dl.z)) load_label(m + 8, dl.z, nullptr, 0, cx->gscr);
                         x = dl.x; gslot = dl.gslot; sslot = dl.sslot; rank = dl.rank;
                     } else {
                         load_direct(p, ls + j, cx, smem + pool1, m, cv, x, gslot, sslot, rank);
                     }
                     lane_hash(smem, o.msg + u1 * 4, cv, m);
-                    lane_store(cv, x, gslot, sslot, rank, smem + pool1, cx);
+                    lane_store(cv, x, gslot, sslot, rank, smem + pool1, 2 * G, cx);
                 }
             }
             boundary(w, w1); /* l + 1 */
@@ -644,7 +649,7 @@ __global__ void __launch_bounds__(PB_CTA_THREADS, 1) k_label_wsc(const __grid_co
                 uint32_t m[16], cv[8], x, gslot, sslot, rk;
                 load_direct(p, ls + j, cx, pool, m, cv, x, gslot, sslot, rk);
                 lane_hash(smem, o.msg, cv, m);
-                lane_store(cv, x, gslot, sslot, rk, pool, cx);
+                lane_store(cv, x, gslot, sslot, rk, pool, 2, cx);
             }
         cl.sync(); /* boundary l + 1 */
     }
@@ -684,7 +689,7 @@ extern "C" int pb_dev_label_ws_prepare(uint32_t *max_smem_bytes) { return allow_
 extern "C" int pb_dev_label_ws(const pb_depth_params_t *params, uint32_t grid, uint32_t smem_bytes,
                                cudaStream_t stream)
 {
-    if (params->units_per_cta < 1 || params->units_per_cta > 4 ||
+    if (params->units_per_cta < 1 || params->units_per_cta > PB_WS_MAX_UNITS ||
         (params->team_warps != 7 && params->team_warps != 15) ||
         smem_bytes < pb_ws_smem_bytes(params->topo.csm, params->units_per_cta, params->team_warps))
         return -1;

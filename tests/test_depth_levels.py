@@ -75,3 +75,21 @@ def test_depth_kernel_levels(pkg, cuda, oracle, cb, nsup):
                 assert rc == 0, pkg.last_error()
                 assert (st["kernel"], st["team_warps"], st["cluster_ctas"]) == (3, warps, cluster)
                 assert buf.cpu().numpy().tobytes() == want, (cb, warps, cluster)
+
+
+# units a team or CTA that are no power of two, the last batch ragged
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel,warps,nsup", [(1, 16, 1100), (1, 4, 1100), (1, 8, 3000), (3, 0, 500), (3, 0, 210),
+                                               (3, 0, 700)])
+def test_uneven_units(pkg, cuda, oracle, kernel, warps, nsup):
+    key, cb, rbo = b"\x11" * 32, 33, 33 * 9
+    want = oracle.label_region(key, cb, nsup, rbo, threads=8).tobytes()
+    buf = cuda.zeros(nsup * cb * 32, dtype=cuda.uint8, device="cuda")
+    with pkg.Topology(cb) as topo:
+        s = pkg.Sched()
+        s.kernel, s.team_warps = kernel, warps
+        rc, st = topo.label(key, buf.data_ptr(), buf.numel(), rbo, sched=s, stats=True)
+        assert rc == 0, pkg.last_error()
+        assert st["kernel"] == kernel and st["units_per_team"] > 1
+        assert buf.cpu().numpy().tobytes() == want, st
+        assert topo.residue() == 0
