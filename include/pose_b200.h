@@ -132,15 +132,16 @@ typedef struct pose_b200_batch pose_b200_batch_t;
  * deepest, when the others are shallower, run as a second launch captured
  * beside the first unless flags has POSE_B200_BATCH_ONE_LAUNCH; sched then
  * applies to the rest.  When the deep requests share one topology built with
- * its block-0 table, that launch is the multi-unit depth kernel (1, 2 or 4
- * chunk copies per CTA, at most one CTA per SM).
- * Otherwise it is the lockstep kernel with 8-warp teams, units packed up to
- * 4 a team so that they hold about half the SMs' team slots.  The
- * environment variable POSE_B200_DEEP_KERNEL=0 selects the lockstep kernel
- * in every case.  With the multi-unit depth kernel, the requests of the
+ * its block-0 table, that launch is the depth kernel (1 to 8 chunk copies per
+ * CTA, one CTA per SM).  Otherwise it is the lockstep kernel with 8-warp
+ * teams, units packed up to 4 a team so that they hold about half the SMs'
+ * team slots.  The environment variable POSE_B200_DEEP_KERNEL=0 selects the
+ * lockstep kernel in every case.  With the depth kernel, the requests of the
  * deepest remaining topology, when its chain is at least a third of the
- * deepest, run as a third launch of it (three chunk copies per CTA, on the
- * SMs the second launch leaves, its CTAs looping over their batches);
+ * deepest, run as a third launch of it.  The copies per CTA of both launches
+ * are those with the shortest estimated makespan, the rest filled in behind
+ * them.  Requests that all share one topology run as pose_b200_topo_label
+ * would run that many chunk copies, unless sched fixes something;
  * POSE_B200_DEEP2=0 keeps them with the rest. */
 pose_b200_batch_t *pose_b200_batch_create(const pose_b200_request_t *reqs, size_t n,
                                           const pose_b200_sched_t *sched);

@@ -37,10 +37,13 @@ typedef struct {
 
 /* Plan n requests for teams of T warps with at most gcap units per team;
  * eff_min > 0 packs units per topology up to that lane efficiency, eff_min
- * <= 0 packs them while their chain stays within the launch's longest.
+ * <= 0 packs them while their chain stays within the launch's longest (both
+ * in powers of two).  With target > 0 each topology takes instead the most
+ * units whose batch the schedule model puts within that many clocks, evened
+ * over its batches, and the queue is ordered by those clocks.
  * Unit i's seed index is its job's index.  Returns 0, or -1 with a message on
  * stderr (bad request, devices differ, out of host memory). */
-int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, double eff_min,
+int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, double eff_min, double target,
                      pb_plan_tables_t *out);
 /* Estimated makespan (SM clocks) of a plan run by R resident teams of T warps:
  * the longest batch chain (passes x latency per pass) against the ALU time of

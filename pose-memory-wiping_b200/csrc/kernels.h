@@ -15,9 +15,8 @@ extern "C" {
 /* Largest CTA the labeling kernels are launched with (lockstep teams of up to
  * 16 warps; 15 hashing warps and a producer). */
 #define PB_CTA_THREADS 512
-/* Largest CTA of the multi-topology kernel (k_label_multi is compiled for
- * three such CTAs per SM). */
-#define PB_MULTI_CTA_THREADS 256
+/* Largest CTA of the multi-topology kernel. */
+#define PB_MULTI_CTA_THREADS 512
 /* Dynamic shared memory of k_label / k_label_multi per thread: two staging
  * buffers of one node's record and block-0 chaining value (48 bytes each). */
 #define PB_PREF_BYTES_PER_THREAD 96u
@@ -93,6 +92,7 @@ typedef struct {
 } pb_multi_params_t;
 
 int pb_dev_label_multi(const pb_multi_params_t *params, uint32_t grid, uint32_t cta_threads, cudaStream_t stream);
+/* Once per device before any launch or stream capture of k_label_multi. */
 int pb_dev_label_multi_occupancy(uint32_t cta_threads, int *blocks_per_sm);
 int pb_dev_seed_jobs(const void *jobs, uint32_t njobs, const uint8_t *blob, uint32_t *seeds, cudaStream_t stream);
 

@@ -1235,6 +1235,39 @@ int pb_topo_view2(const pose_hbm_topo_t *t, pb_topo_view2_t *out)
     return 0;
 }
 
+double pb_topo_lockstep_clocks(const pose_hbm_topo_t *t, uint32_t T, uint32_t G)
+{
+    const int cv0 = t->d_cv0 != NULL;
+    uint64_t passes, warps;
+    lockstep_passes(t, T, G, &passes, &warps);
+    const double lat = (double)passes * lockstep_pass(cv0);
+    const double c = t->L * lockstep_overhead(1, cv0) + (double)(passes - t->L) * lockstep_more +
+                     (double)warps * 32.0 * lockstep_node(cv0);
+    return lat > c ? lat : c;
+}
+
+double pb_topo_depth_clocks(const pose_hbm_topo_t *t, uint32_t G)
+{
+    return t->d_recs2 ? ws_cost(t, 15, G, 1, 1) : 0.0;
+}
+
+int pb_topo_auto_plan(const pose_hbm_topo_t *t, uint64_t nunits, uint64_t budget, uint32_t *kernel, uint32_t *T,
+                      uint32_t *G)
+{
+    plan_t p;
+    pose_b200_sched_t h;
+    memset(&h, 0, sizeof(h));
+    if (nunits == 0 || make_plan(t, nunits, NULL, budget, &p) != 0) return -1;
+    if (p.kernel == 3 && p.cluster > 1) { /* without the cluster form */
+        h.cluster_ctas = 1;
+        if (make_plan(t, nunits, &h, budget, &p) != 0) return -1;
+    }
+    *kernel = p.kernel;
+    *T = p.T;
+    *G = p.G;
+    return 0;
+}
+
 uint64_t pb_topo_passes(const pose_hbm_topo_t *t, uint32_t T, uint32_t G)
 {
     return t ? passes_for(t, T, G) : 0;

@@ -121,7 +121,7 @@ void pb_plan_free(pb_plan_tables_t *p)
     memset(p, 0, sizeof(*p));
 }
 
-int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, double eff_min,
+int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, double eff_min, double target,
                      pb_plan_tables_t *out)
 {
     memset(out, 0, sizeof(*out));
@@ -211,7 +211,13 @@ int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, 
     uint64_t nb = 0;
     for (size_t k = 0; k < ntopo; k++) {
         uint32_t g = 1;
-        while (g * 2 <= gcap && g * 2 <= 32 * T && g < nunits_t[k]) {
+        if (target > 0 && nunits_t[k]) {
+            const uint32_t most = gcap < nunits_t[k] ? gcap : nunits_t[k];
+            while (g < most && g < 32 * T && pb_topo_lockstep_clocks(topo_list[k], T, g + 1) <= target) g++;
+            const uint32_t even = (nunits_t[k] + g - 1) / g;
+            g = (nunits_t[k] + even - 1) / even;
+        }
+        while (target <= 0 && g * 2 <= gcap && g * 2 <= 32 * T && g < nunits_t[k]) {
             if (eff_min > 0) {
                 uint64_t passes = pb_topo_passes(topo_list[k], T, g);
                 double eff = (double)g * ti[k].view.S / ((double)passes * 32.0 * T);
@@ -235,12 +241,14 @@ int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, 
         uint64_t q = 0;
         for (size_t k = 0; k < ntopo; k++) {
             uint64_t passes = pb_topo_passes(topo_list[k], T, G[k]);
+            const uint64_t order = target > 0 && nunits_t[k] ? (uint64_t)pb_topo_lockstep_clocks(topo_list[k], T, G[k])
+                                                             : passes;
             for (uint32_t f = 0; f < nunits_t[k]; f += G[k]) {
                 bs[q].b.topo = (uint32_t)k;
                 bs[q].b.first_unit = (uint32_t)(ufirst[k] + f);
                 bs[q].b.count = nunits_t[k] - f < G[k] ? nunits_t[k] - f : G[k];
                 bs[q].b.G = G[k];
-                bs[q].cost = passes;
+                bs[q].cost = order;
                 if (passes > out->max_chain) out->max_chain = passes;
                 q++;
             }
@@ -297,7 +305,7 @@ int pb_plan_rank(const pb_req_t *pr, size_t n, const pose_b200_sched_t *sched, p
     for (uint32_t tT = t_lo; tT <= t_hi; tT <<= 1) {
         for (int e = 0; e < nrules && k < cap; e++) {
             pb_plan_tables_t cand;
-            if (pb_plan_requests(pr, n, tT, gcap, rules[e], &cand) != 0) return -1;
+            if (pb_plan_requests(pr, n, tT, gcap, rules[e], 0.0, &cand) != 0) return -1;
             out[k].T = tT;
             out[k].eff = rules[e];
             out[k].est = pb_plan_makespan(&cand, tT, (uint64_t)cand.sms * 32 / tT);
@@ -379,13 +387,12 @@ static size_t split_second(const pb_req_t *pr, size_t n, uint8_t *deep)
     return n2;
 }
 
-/* Size, allocate and upload one launch of a batch; `slots` caps its resident
- * threads in units of 256 (256 / 32T teams each) and `budget` its scratch.
- * One team per CTA.  Returns 0, or -1 (message on stderr). */
+/* Size, allocate and upload one launch of a batch; `cap` is the most teams it
+ * may hold and `budget` bounds its scratch.  One team per CTA.  Returns 0, or
+ * -1 (message on stderr). */
 static int part_setup(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_tables_t *pl, uint32_t T,
-                      uint64_t slots, uint64_t budget, const pose_b200_sched_t *sched)
+                      uint64_t cap, uint64_t budget, const pose_b200_sched_t *sched)
 {
-    const uint32_t tpc = 256 / (32 * T);
     q->T = T;
     q->nbatches = pl->nbatches;
     q->njobs = pl->njobs;
@@ -395,7 +402,6 @@ static int part_setup(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_table
     q->Gmax = pl->Gmax;
     q->cv0 = pl->all_cv0;
     q->team_scratch = pl->team_scratch;
-    uint64_t cap = slots * tpc;
     uint64_t R = budget / pl->team_scratch;
     if (R > cap) R = cap;
     if (R > pl->nbatches) R = pl->nbatches;
@@ -435,7 +441,7 @@ static int part_setup(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_table
 }
 
 /* The deep part on the multi-unit depth kernel: every unit of pl (one
- * topology, records v2), G (1 to 4) units per CTA, at most one CTA per SM
+ * topology, records v2), G (1 to 8) units per CTA, at most one CTA per SM
  * (`sms` CTAs), 15 hashing warps.  Returns 0, or -1 (message on stderr). */
 static int part_setup_wsg(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_tables_t *pl,
                           const pb_topo_view2_t *v2, uint32_t G, uint32_t sms, uint32_t smem)
@@ -483,12 +489,20 @@ static int part_setup_wsg(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_t
     return 0;
 }
 
-/* Capture one launch onto stream s: seeds, queue reset, labeling, scratch
- * and chunk-seed zeroing (events e0/e1 around the labeling kernel when not
- * NULL).  A replay leaves no label or chunk seed behind; the session seeds
- * stay for the next replay and are zeroed when the batch is destroyed. */
-static int part_capture(const pose_b200_batch_t *b, const batch_part_t *q, cudaStream_t s, cudaEvent_t e0,
-                        cudaEvent_t e1)
+/* Capture what one launch needs first onto stream s: chunk seeds and the
+ * queue reset. */
+static int part_capture_seeds(const pose_b200_batch_t *b, const batch_part_t *q, cudaStream_t s)
+{
+    if (pb_dev_seed_jobs(q->d_jobs, (uint32_t)q->njobs, (const uint8_t *)b->d_blob, (uint32_t *)q->d_seeds, s) != 0)
+        return -1;
+    return cudaMemsetAsync(q->d_queue, 0, 64, s) == cudaSuccess ? 0 : -1;
+}
+
+/* Capture one launch onto stream s: labeling, scratch and chunk-seed zeroing
+ * (events e0/e1 around the labeling kernel when not NULL).  A replay leaves
+ * no label or chunk seed behind; the session seeds stay for the next replay
+ * and are zeroed when the batch is destroyed. */
+static int part_capture(const batch_part_t *q, cudaStream_t s, cudaEvent_t e0, cudaEvent_t e1)
 {
     pb_multi_params_t p;
     memset(&p, 0, sizeof(p));
@@ -501,9 +515,8 @@ static int part_capture(const pose_b200_batch_t *b, const batch_part_t *q, cudaS
     p.nbatches = (uint32_t)q->nbatches;
     p.team_warps = q->T;
     p.queue = (unsigned int *)q->d_queue;
-    int crc = pb_dev_seed_jobs(q->d_jobs, (uint32_t)q->njobs, (const uint8_t *)b->d_blob, (uint32_t *)q->d_seeds, s);
-    if (crc == 0) crc = cudaMemsetAsync(q->d_queue, 0, 64, s) == cudaSuccess ? 0 : -1;
-    if (crc == 0 && e0) crc = cudaEventRecord(e0, s) == cudaSuccess ? 0 : -1;
+    int crc = 0;
+    if (e0) crc = cudaEventRecord(e0, s) == cudaSuccess ? 0 : -1;
     if (crc == 0 && q->kind == 1) {
         pb_depth_params_t w;
         memset(&w, 0, sizeof(w));
@@ -525,6 +538,147 @@ static int part_capture(const pose_b200_batch_t *b, const batch_part_t *q, cudaS
     if (crc == 0) crc = cudaMemsetAsync(q->d_scratch, 0, q->scratch_bytes, s) == cudaSuccess ? 0 : -1;
     if (crc == 0) crc = cudaMemsetAsync(q->d_seeds, 0, (size_t)q->njobs * 32, s) == cudaSuccess ? 0 : -1;
     return crc;
+}
+
+/* Units (chunk copies) of n requests. */
+static uint64_t request_units(const pb_req_t *pr, size_t n)
+{
+    uint64_t u = 0;
+    for (size_t i = 0; i < n; i++) {
+        pb_topo_internal_t x;
+        if (pb_topo_internal(pr[i].topo, &x) == 0) u += (uint64_t)(pr[i].len / x.super_bytes) * x.copies;
+    }
+    return u;
+}
+
+/* The one topology of all requests with something to label, or NULL. */
+static const pose_hbm_topo_t *one_topology(const pb_req_t *pr, size_t n)
+{
+    const pose_hbm_topo_t *t = NULL;
+    for (size_t i = 0; i < n; i++) {
+        pb_topo_internal_t x;
+        if (pb_topo_internal(pr[i].topo, &x) != 0) return NULL;
+        if (pr[i].len < x.super_bytes) continue;
+        if (t && t != pr[i].topo) return NULL;
+        t = pr[i].topo;
+    }
+    return t;
+}
+
+/* SM clocks of n requests on 16-warp lockstep teams of 16 units, and the
+ * longest single unit's; the larger of the latter and the work spread over
+ * the SMs is what they need at least. */
+static double shallow_work(const pb_req_t *pr, size_t n, double *longest, uint32_t *sms)
+{
+    double work = 0;
+    *longest = 0;
+    *sms = 148;
+    const pose_hbm_topo_t *last = NULL;
+    double c16 = 0, c1 = 0;
+    for (size_t i = 0; i < n; i++) {
+        pb_topo_internal_t x;
+        if (pb_topo_internal(pr[i].topo, &x) != 0 || pr[i].len < x.super_bytes) continue;
+        if (pr[i].topo != last) {
+            last = pr[i].topo;
+            c16 = pb_topo_lockstep_clocks(last, 16, 16) / 16.0;
+            c1 = pb_topo_lockstep_clocks(last, 16, 1);
+        }
+        work += (double)(pr[i].len / x.super_bytes) * x.copies * c16;
+        if (c1 > *longest) *longest = c1;
+        if (x.sms > 0) *sms = (uint32_t)x.sms;
+    }
+    return work;
+}
+
+static double shallow_makespan(const pb_req_t *pr, size_t n)
+{
+    double longest;
+    uint32_t sms;
+    const double work = shallow_work(pr, n, &longest, &sms);
+    return longest > work / sms ? longest : work / sms;
+}
+
+static int cmp_double(const void *a, const void *b)
+{
+    const double x = *(const double *)a, y = *(const double *)b;
+    return x < y ? -1 : x > y;
+}
+
+/* Clocks until b1 jobs of t1, then b2 of t2 (each on the SM that is free
+ * first), and `rest` clocks of small work filled in behind them are done. */
+static double deep_makespan(double *load, uint32_t sms, uint64_t b1, double t1, uint64_t b2, double t2, double rest)
+{
+    for (uint32_t i = 0; i < sms; i++) load[i] = t1 * (double)(b1 / sms + (i < b1 % sms));
+    for (uint64_t j = 0; j < b2; j++) {
+        uint32_t m = 0;
+        for (uint32_t i = 1; i < sms; i++)
+            if (load[i] < load[m]) m = i;
+        load[m] += t2;
+    }
+    qsort(load, sms, sizeof(*load), cmp_double);
+    double level = load[0], left = rest;
+    for (uint32_t i = 1; i <= sms; i++) { /* fill the i least loaded SMs up to the next one */
+        const double next = i < sms ? load[i] : 1e300;
+        if ((next - level) * i >= left) {
+            level += left / i;
+            break;
+        }
+        left -= (next - level) * i;
+        level = next;
+    }
+    return level > load[sms - 1] ? level : load[sms - 1];
+}
+
+/* Copies per CTA of the two deep parts (pd: nd requests of one topology; pd2:
+ * nd2 of another, or none) that the schedule model finishes first, with the
+ * other requests ps filled in behind them; fix1, fix2 (nonzero) fix them.
+ * On the 256-session workload that is 4 and 8: 98 CTAs of the 2^17 sessions
+ * and 49 of the 2^16 ones beside them, each SM one CTA.  Returns 0, or -1
+ * when no choice fits the shared memory and the scratch budget. */
+static int plan_deep(const pb_req_t *pd, size_t nd, const pb_req_t *pd2, size_t nd2, const pb_req_t *ps, size_t ns,
+                     uint32_t sms, uint64_t budget, uint32_t fix1, uint32_t fix2, uint32_t *G1, uint32_t *G2,
+                     double *makespan)
+{
+    pb_topo_view2_t v1, v2;
+    uint32_t max_smem = 0, n_sms;
+    double longest;
+    if (pb_topo_view2(pd[0].topo, &v1) != 0 || pb_dev_label_ws_prepare(&max_smem) != 0) return -1;
+    if (nd2 && pb_topo_view2(pd2[0].topo, &v2) != 0) nd2 = 0;
+    const uint64_t u1 = request_units(pd, nd), u2 = nd2 ? request_units(pd2, nd2) : 0;
+    const double rest = shallow_work(ps, ns, &longest, &n_sms);
+    double *load = (double *)malloc(sms * sizeof(*load));
+    if (!load) return -1;
+    double best = -1;
+    for (uint32_t a = 1; a <= PB_WS_MAX_UNITS; a++) {
+        const uint64_t b1 = (u1 + a - 1) / a, s1 = (b1 < sms ? b1 : sms) * (uint64_t)v1.gpool * 32 * a;
+        if ((fix1 && a != fix1) || pb_ws_smem_bytes(v1.csm, a, 15) > max_smem || s1 > budget) continue;
+        const double t1 = pb_topo_depth_clocks(pd[0].topo, a);
+        for (uint32_t c = nd2 ? 1 : 0; c <= (nd2 ? PB_WS_MAX_UNITS : 0); c++) {
+            uint64_t b2 = 0;
+            double t2 = 0;
+            if (c) {
+                b2 = (u2 + c - 1) / c;
+                if ((fix2 && c != fix2) || pb_ws_smem_bytes(v2.csm, c, 15) > max_smem) continue;
+                t2 = pb_topo_depth_clocks(pd2[0].topo, c);
+            }
+            if (b2 > 16ull * sms) continue;
+            const double m = deep_makespan(load, sms, b1, t1, b2, t2, rest);
+            if (best < 0 || m < best) {
+                best = m;
+                *G1 = a;
+                *G2 = c;
+            }
+        }
+        /* more second-part units than the search takes */
+        if (best < 0 && nd2) {
+            best = t1 * (double)((b1 + sms - 1) / sms);
+            *G1 = a;
+            *G2 = fix2 ? fix2 : 4;
+        }
+    }
+    free(load);
+    *makespan = best;
+    return best < 0 ? -1 : 0;
 }
 
 pose_b200_batch_t *pose_b200_batch_create(const pose_b200_request_t *reqs, size_t n,
@@ -598,8 +752,13 @@ no_split:
     if (!b) goto fail_host;
     b->device = dev;
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) goto fail;
-    if (nd && cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking) != cudaSuccess) goto fail;
-    if (nd2 && cudaStreamCreateWithFlags(&b->stream3, cudaStreamNonBlocking) != cudaSuccess) goto fail;
+    {
+        int lo = 0, hi = 0; /* numerically lower is higher */
+        if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess) lo = hi = 0;
+        const int mid = hi < lo ? hi + 1 : hi;
+        if (nd && cudaStreamCreateWithPriority(&b->stream2, cudaStreamNonBlocking, hi) != cudaSuccess) goto fail;
+        if (nd2 && cudaStreamCreateWithPriority(&b->stream3, cudaStreamNonBlocking, mid) != cudaSuccess) goto fail;
+    }
     for (int i = 0; i < 8; i++) if (cudaEventCreate(&b->ev[i]) != cudaSuccess) goto fail;
     b->blob_len = blob_len;
     if (pb_dev_malloc(&b->d_blob, blob_len ? blob_len : 1) != cudaSuccess) {
@@ -610,10 +769,15 @@ no_split:
                      cudaStreamSynchronize(b->stream) != cudaSuccess))
         goto fail;
     {
-        int occ = 0;
+        int occ = 0, occ16 = 0; /* 8- and 16-warp CTAs per SM */
+        if (pb_dev_label_multi_occupancy(512, &occ16) != 0 || occ16 <= 0) occ16 = 1;
         if (pb_dev_label_multi_occupancy(256, &occ) != 0 || occ <= 0) occ = 1;
         uint64_t budget = pb_topo_scratch_budget(reqs[0].topo, sched ? sched->scratch_cap_bytes : 0);
-        uint64_t slots = 0, deep_ctas = 0;
+        uint64_t deep_ctas = 0;
+        /* the caller fixes nothing: the schedule model plans every part */
+        const int open_sched = !sched || (!sched->team_warps && !sched->units_per_team && !sched->max_teams &&
+                                          !sched->lane_efficiency && !sched->flags);
+        double makespan = 0; /* estimated, in clocks, when the deep parts are planned by the model */
         /* deep part: 8-warp teams, units packed (G up to 4) until it holds
          * about half the SMs' team slots */
         if (nd) {
@@ -627,38 +791,27 @@ no_split:
                 sms = (uint32_t)x.sms;
                 if (pd[i].topo != pd[0].topo) one_topo = 0;
             }
-            /* one topology: the multi-unit depth kernel, with the fewest
-             * units per CTA (1, 2 or 4) that fit one CTA per SM: a narrow
-             * level of G units is still one warp pass, while a wide level's
-             * ALU work on the SM grows with G.  (Three units per CTA, 137
-             * CTAs for the 256-session workload's 410 deep units, measured
-             * 2.12 s against 1.62 s for four: the shallow part then has 34
-             * SMs fewer.) */
+            /* one topology: the depth kernel */
             pb_topo_view2_t v2;
-            uint32_t G = 1;
-            while (G < 4 && (dunits + G - 1) / G > sms) G *= 2;
             const char *ek = getenv("POSE_B200_DEEP_KERNEL");
-            const char *eg = getenv("POSE_B200_DEEP_UNITS");
-            if (eg && eg[0] >= '1' && eg[0] <= '4' && !eg[1]) G = (uint32_t)(eg[0] - '0');
+            const char *eg = getenv("POSE_B200_DEEP_UNITS");  /* tuning: copies per CTA, 1 to 8 */
+            const char *eu = getenv("POSE_B200_DEEP2_UNITS"); /* the same for the second deep part */
+            const uint32_t fix1 = eg && eg[0] >= '1' && eg[0] <= '8' && !eg[1] ? (uint32_t)(eg[0] - '0') : 0;
+            const uint32_t fix2 = eu && eu[0] >= '1' && eu[0] <= '8' && !eu[1] ? (uint32_t)(eu[0] - '0') : 0;
+            uint32_t G = 0, G2 = 0;
             int wsg = !(ek && ek[0] == '0') && one_topo && pb_topo_view2(pd[0].topo, &v2) == 0;
             if (wsg) {
-                const uint64_t grid = (dunits + G - 1) / G < sms ? (dunits + G - 1) / G : sms;
-                wsg = grid * ((uint64_t)v2.gpool * 32 * G) <= budget;
-            }
-            if (wsg) {
-                /* a device whose CTAs cannot hold the kernel's shared memory
-                 * keeps the deep part on the lockstep kernel */
-                uint32_t max_smem = 0;
-                wsg = pb_dev_label_ws_prepare(&max_smem) == 0 && pb_ws_smem_bytes(v2.csm, G, 15) <= max_smem;
+                /* copies per CTA of both parts */
+                wsg = plan_deep(pd, nd, pd2, nd2, ps, ns, sms, budget, fix1, fix2, &G, &G2, &makespan) == 0;
                 cudaGetLastError();
             }
             if (wsg) {
                 const uint32_t smem = pb_ws_smem_bytes(v2.csm, G, 15);
-                if (pb_plan_requests(pd, nd, 8, 1, 0.9999, &pl[1]) != 0 || pl[1].nunits == 0) goto fail;
+                if (pb_plan_requests(pd, nd, 8, 1, 0.9999, 0.0, &pl[1]) != 0 || pl[1].nunits == 0) goto fail;
                 if (part_setup_wsg(b, &b->part[1], &pl[1], &v2, G, sms, smem) != 0) goto fail;
                 /* the next-deepest topology's requests: a third launch of the
-                 * depth kernel on the SMs the first leaves, three copies per
-                 * CTA, its CTAs looping over their batches */
+                 * depth kernel, on the SMs the first leaves and then on those
+                 * it is done with */
                 if (nd2) {
                     pb_topo_view2_t v2b;
                     uint64_t du2 = 0;
@@ -667,22 +820,18 @@ no_split:
                         if (pb_topo_internal(pd2[i].topo, &x) != 0) goto fail;
                         du2 += (uint64_t)(pd2[i].len / x.super_bytes) * x.copies;
                     }
-                    uint32_t G2 = 3; /* on the 256-session workload: 3 copies 999 MiB/s, 4 copies 839-845 */
-                    const char *eu = getenv("POSE_B200_DEEP2_UNITS"); /* tuning: copies per CTA, 1 to 4 */
-                    if (eu && eu[0] >= '1' && eu[0] <= '4' && !eu[1]) G2 = (uint32_t)(eu[0] - '0');
-                    const uint32_t left = sms > b->part[1].grid ? sms - b->part[1].grid : 0;
                     uint32_t max_smem2 = 0;
-                    int ok2 = left > 0 && pb_topo_view2(pd2[0].topo, &v2b) == 0 &&
+                    int ok2 = G2 > 0 && pb_topo_view2(pd2[0].topo, &v2b) == 0 &&
                               pb_dev_label_ws_prepare(&max_smem2) == 0 &&
                               pb_ws_smem_bytes(v2b.csm, G2, 15) <= max_smem2;
                     cudaGetLastError();
                     if (ok2) {
-                        const uint64_t g2 = (du2 + G2 - 1) / G2 < left ? (du2 + G2 - 1) / G2 : left;
+                        const uint64_t g2 = (du2 + G2 - 1) / G2 < sms ? (du2 + G2 - 1) / G2 : sms;
                         ok2 = b->part[1].scratch_bytes + g2 * ((uint64_t)v2b.gpool * 32 * G2) <= budget;
                     }
                     if (ok2) {
-                        if (pb_plan_requests(pd2, nd2, 8, 1, 0.9999, &pl[2]) != 0 || pl[2].nunits == 0) goto fail;
-                        if (part_setup_wsg(b, &b->part[2], &pl[2], &v2b, G2, left, pb_ws_smem_bytes(v2b.csm, G2, 15)) !=
+                        if (pb_plan_requests(pd2, nd2, 8, 1, 0.9999, 0.0, &pl[2]) != 0 || pl[2].nunits == 0) goto fail;
+                        if (part_setup_wsg(b, &b->part[2], &pl[2], &v2b, G2, sms, pb_ws_smem_bytes(v2b.csm, G2, 15)) !=
                             0)
                             goto fail;
                     } else {
@@ -693,7 +842,7 @@ no_split:
             } else {
                 uint32_t g = 1;
                 while (g < 4 && 2 * (dunits + g - 1) / g > (uint64_t)sms * occ) g *= 2;
-                if (pb_plan_requests(pd, nd, 8, g, 0.9999, &pl[1]) != 0 || pl[1].nunits == 0) goto fail;
+                if (pb_plan_requests(pd, nd, 8, g, 0.9999, 0.0, &pl[1]) != 0 || pl[1].nunits == 0) goto fail;
                 deep_ctas = pl[1].nbatches;
                 if (deep_ctas * 2 > (uint64_t)pl[1].sms * occ) deep_ctas = (uint64_t)pl[1].sms * occ / 2;
                 if (part_setup(b, &b->part[1], &pl[1], 8, deep_ctas, budget, NULL) != 0) goto fail;
@@ -706,18 +855,54 @@ no_split:
             budget = budget > used ? budget - used : 0;
         }
         const uint32_t gcap = sched && sched->units_per_team ? sched->units_per_team : 32;
-        uint32_t T = 4;
+        uint32_t T = 16;
         double eff = 0.0;
-        if (pb_plan_choose(ps, ns, sched, &T, &eff) != 0) goto fail;
-        if (pb_plan_requests(ps, ns, T, gcap, eff, &pl[0]) != 0) goto fail;
-        if (pl[0].nunits == 0 && !nd) { fprintf(stderr, "pose_b200_batch_create: no super-chunk to label\n"); goto fail; }
-        slots = (uint64_t)pl[0].sms * occ;
-        {
-            const uint64_t taken = (uint64_t)b->part[1].grid + (nd2 ? b->part[2].grid : 0);
-            slots = slots > taken ? slots - taken : 1;
+        const pose_hbm_topo_t *only = NULL;
+        uint32_t ukern = 0, uT = 0, uG = 0;
+        if (open_sched && !nd && (only = one_topology(ps, ns)) != NULL &&
+            pb_topo_auto_plan(only, request_units(ps, ns), budget, &ukern, &uT, &uG) != 0)
+            ukern = 0;
+        pb_topo_view2_t uv2;
+        uint32_t umax = 0;
+        if (ukern == 3 && (pb_topo_view2(only, &uv2) != 0 || pb_dev_label_ws_prepare(&umax) != 0 ||
+                           pb_ws_smem_bytes(uv2.csm, uG, 15) > umax)) {
+            cudaGetLastError();
+            ukern = 0;
         }
-        if (pl[0].nunits) {
-            if (part_setup(b, &b->part[0], &pl[0], T, slots, budget, sched) != 0) goto fail;
+        if (ukern == 3) {
+            /* one topology, few units: the depth kernel, as a single call */
+            pb_topo_internal_t x;
+            if (pb_topo_internal(only, &x) != 0 || pb_plan_requests(ps, ns, 8, 1, 0.9999, 0.0, &pl[0]) != 0) goto fail;
+            T = 15;
+            if (part_setup_wsg(b, &b->part[0], &pl[0], &uv2, uG, (uint32_t)x.sms, pb_ws_smem_bytes(uv2.csm, uG, 15)) != 0)
+                goto fail;
+        } else if (open_sched) {
+            /* 16-warp teams; batches no longer than a third of the deep
+             * parts' makespan (they fill the SMs those leave), or half of
+             * what the requests need on all SMs */
+            double target = ukern == 1 ? 1e30 : makespan / 3.0;
+            if (target <= 0) target = shallow_makespan(ps, ns) / 2.0;
+            if (target <= 0) target = 1.0;
+            if (ukern == 1) T = uT;
+            if (pb_plan_requests(ps, ns, T, ukern == 1 ? uG : 32, 0.0, target, &pl[0]) != 0) goto fail;
+        } else {
+            if (pb_plan_choose(ps, ns, sched, &T, &eff) != 0) goto fail;
+            if (pb_plan_requests(ps, ns, T, gcap, eff, 0.0, &pl[0]) != 0) goto fail;
+        }
+        if (pl[0].nunits == 0 && !nd) { fprintf(stderr, "pose_b200_batch_create: no super-chunk to label\n"); goto fail; }
+        if (pl[0].nunits && ukern != 3) {
+            uint64_t cap;
+            if (open_sched) {
+                int o = 1;
+                if (pb_dev_label_multi_occupancy(32 * T, &o) != 0 || o <= 0) o = 1;
+                cap = (uint64_t)pl[0].sms * (uint64_t)o;
+            } else {
+                const uint64_t taken = (uint64_t)b->part[1].grid + (nd2 ? b->part[2].grid : 0);
+                uint64_t slots = (uint64_t)pl[0].sms * occ;
+                slots = slots > taken ? slots - taken : 1;
+                cap = slots * (256 / (32 * T));
+            }
+            if (part_setup(b, &b->part[0], &pl[0], T, cap, budget, sched) != 0) goto fail;
         }
         b->nparts = nd2 ? 3 : nd ? 2 : 1;
         b->T = T;
@@ -733,23 +918,30 @@ no_split:
         }
         b->cv0 = (pl[0].nunits == 0 || b->part[0].cv0) && (!nd || b->part[1].cv0) && (!nd2 || b->part[2].cv0);
 
-        /* capture: the rest on the batch's stream; the deep part forked onto
-         * a second stream and joined back */
+        /* capture: every launch's seeds on the batch's stream, then the deep
+         * parts forked onto streams of higher priority and the rest behind a
+         * second reset of its queue, so that the deep parts' CTAs, which need
+         * whole SMs and run longest, are placed first */
         if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) goto fail;
         int crc = 0;
-        if (nd) {
+        for (int i = b->nparts - 1; i >= 0 && crc == 0; i--)
+            if (i > 0 || pl[0].nunits) crc = part_capture_seeds(b, &b->part[i], b->stream);
+        if (crc == 0 && nd) {
             crc = cudaEventRecord(b->ev[4], b->stream) == cudaSuccess ? 0 : -1;
             if (crc == 0) crc = cudaStreamWaitEvent(b->stream2, b->ev[4], 0) == cudaSuccess ? 0 : -1;
-            if (crc == 0) crc = part_capture(b, &b->part[1], b->stream2, NULL, NULL);
+            if (crc == 0) crc = part_capture(&b->part[1], b->stream2, NULL, NULL);
             if (crc == 0) crc = cudaEventRecord(b->ev[5], b->stream2) == cudaSuccess ? 0 : -1;
         }
         if (crc == 0 && nd2) {
             crc = cudaEventRecord(b->ev[6], b->stream) == cudaSuccess ? 0 : -1;
             if (crc == 0) crc = cudaStreamWaitEvent(b->stream3, b->ev[6], 0) == cudaSuccess ? 0 : -1;
-            if (crc == 0) crc = part_capture(b, &b->part[2], b->stream3, NULL, NULL);
+            if (crc == 0) crc = part_capture(&b->part[2], b->stream3, NULL, NULL);
             if (crc == 0) crc = cudaEventRecord(b->ev[7], b->stream3) == cudaSuccess ? 0 : -1;
         }
-        if (crc == 0 && pl[0].nunits) crc = part_capture(b, &b->part[0], b->stream, b->ev[1], b->ev[2]);
+        if (crc == 0 && pl[0].nunits) {
+            if (nd) crc = cudaMemsetAsync(b->part[0].d_queue, 0, 64, b->stream) == cudaSuccess ? 0 : -1;
+            if (crc == 0) crc = part_capture(&b->part[0], b->stream, b->ev[1], b->ev[2]);
+        }
         if (crc == 0 && nd) crc = cudaStreamWaitEvent(b->stream, b->ev[5], 0) == cudaSuccess ? 0 : -1;
         if (crc == 0 && nd2) crc = cudaStreamWaitEvent(b->stream, b->ev[7], 0) == cudaSuccess ? 0 : -1;
         cudaError_t ce = cudaStreamEndCapture(b->stream, &b->graph);

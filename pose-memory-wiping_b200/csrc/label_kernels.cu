@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant_
  * G units) from a queue sorted longest first, and copy the batch's
  * topology view into shared memory.  One team of T warps per CTA
  * (blockDim.x == 32 T), ending its levels with the CTA barrier. */
-__global__ void __launch_bounds__(PB_MULTI_CTA_THREADS, 3) k_label_multi(const __grid_constant__ pb_multi_params_t p)
+__global__ void __launch_bounds__(PB_MULTI_CTA_THREADS, 2) k_label_multi(const __grid_constant__ pb_multi_params_t p)
 {
     const uint32_t T = p.team_warps;
     const uint32_t TT = T * 32;
@@ -556,9 +556,13 @@ extern "C" int pb_dev_label_multi(const pb_multi_params_t *params, uint32_t grid
 
 extern "C" int pb_dev_label_multi_occupancy(uint32_t cta_threads, int *blocks_per_sm)
 {
+    /* a 512-thread CTA stages 48 KiB, more than the default limit with the
+     * static shared memory: one value for every caller (idempotent) */
     const size_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pb::k_label_multi, (int)cta_threads, smem) ==
-                   cudaSuccess
+    return cudaFuncSetAttribute(pb::k_label_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(PB_PREF_BYTES_PER_THREAD * PB_MULTI_CTA_THREADS)) == cudaSuccess &&
+                   cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pb::k_label_multi, (int)cta_threads,
+                                                                 smem) == cudaSuccess
                ? 0
                : -1;
 }

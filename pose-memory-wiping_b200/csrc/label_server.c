@@ -482,7 +482,7 @@ static int admit_wave(pose_b200_server_t *s)
     pb_plan_tables_t pl;
     uint32_t Tw = 4;
     double eff = 0.0;
-    if (pb_plan_choose(pr, n, NULL, &Tw, &eff) != 0 || pb_plan_requests(pr, n, Tw, 32, eff, &pl) != 0) {
+    if (pb_plan_choose(pr, n, NULL, &Tw, &eff) != 0 || pb_plan_requests(pr, n, Tw, 32, eff, 0.0, &pl) != 0) {
         free(pr);
         for (size_t i = 0; i < n; i++) { s->reqs[wv->reqs[i]].state = 3; s->reqs[wv->reqs[i]].t_done = now_ms(); }
         pthread_cond_broadcast(&s->cv);

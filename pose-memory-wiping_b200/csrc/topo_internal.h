@@ -41,6 +41,15 @@ int pb_topo_label_raw(const pose_hbm_topo_t *t, const uint8_t *chunk_seeds, void
  * topology built without its block-0 table. */
 int pb_topo_view2(const pose_hbm_topo_t *t, pb_topo_view2_t *out);
 
+/* The schedule model's clocks of one batch of G units on an SM of its own: on
+ * a lockstep team of T warps, and on a depth-kernel CTA of 15 hashing warps
+ * (0 for a topology without the records). */
+double pb_topo_lockstep_clocks(const pose_hbm_topo_t *t, uint32_t T, uint32_t G);
+double pb_topo_depth_clocks(const pose_hbm_topo_t *t, uint32_t G);
+/* The automatic schedule of a call of nunits units: kernel 1 (T, G) or 3 (G). */
+int pb_topo_auto_plan(const pose_hbm_topo_t *t, uint64_t nunits, uint64_t budget, uint32_t *kernel, uint32_t *T,
+                      uint32_t *G);
+
 /* Passes a team of T warps makes over all levels running G units in lockstep. */
 uint64_t pb_topo_passes(const pose_hbm_topo_t *t, uint32_t T, uint32_t G);
 /* Free device memory usable for scratch under an optional cap (the topology's
