@@ -194,10 +194,11 @@ int pose_b200_label_stream(const pose_hbm_topo_t *topo, const uint8_t *session_s
  * scratch arena (the HBM budget given at creation) has room, so work that
  * arrives while other work runs starts as memory frees up and overlaps it on
  * the device:
- *   - requests of deep topologies (chunk_blocks 2^17 and up) run on the
- *     multi-unit depth kernel, the pending ones of one topology together,
- *     three chunk copies per CTA, each CTA holding its SM alone, on
- *     high-priority streams; one that does not fit the free SMs waits;
+ *   - requests of deep topologies (chunk_blocks 2^15 and up) run on the depth
+ *     kernel, the pending ones of one topology together, one to four chunk
+ *     copies per CTA by the load, each CTA holding its SM alone, on
+ *     high-priority streams and at most 7/8 of the SMs; one that does not fit
+ *     the free SMs waits;
  *   - the others run in waves: one persistent multi-topology launch per
  *     wave on its own stream, a request completing as soon as its chunk
  *     copies are in;
@@ -208,8 +209,8 @@ int pose_b200_label_stream(const pose_hbm_topo_t *topo, const uint8_t *session_s
  * CUDA_DEVICE_MAX_CONNECTIONS (8 by default; 32 gives every slot its own)
  * bounds how many run at once.  Tuning variables, read at creation:
  * POSE_B200_SERVER_DEEP_LEVELS (levels from which a topology is deep),
- * POSE_B200_SERVER_DEEP_UNITS (copies per depth CTA; 0 = the fewest that fit
- * an idle GPU), POSE_B200_SERVER_DEEP_EXCL and POSE_B200_SERVER_DEEP_WAIT
+ * POSE_B200_SERVER_DEEP_UNITS (copies per depth CTA; 0 = by the load),
+ * POSE_B200_SERVER_DEEP_GMAX (the most then), POSE_B200_SERVER_DEEP_EXCL and POSE_B200_SERVER_DEEP_WAIT
  * (0: share SMs; 0: join a wave instead of waiting), POSE_B200_SERVER_DEEP=0
  * (every request in waves), POSE_B200_SERVER_DEEP_SMS (SMs the depth kernel
  * may hold).  Each result is byte-identical to labelling the request alone.

@@ -590,12 +590,19 @@ static double shallow_work(const pb_req_t *pr, size_t n, double *longest, uint32
     return work;
 }
 
-static double shallow_makespan(const pb_req_t *pr, size_t n)
+static double shallow_makespan(const pb_req_t *pr, size_t n, uint32_t sms)
 {
     double longest;
-    uint32_t sms;
-    const double work = shallow_work(pr, n, &longest, &sms);
+    uint32_t all;
+    const double work = shallow_work(pr, n, &longest, &all);
+    if (sms == 0 || sms > all) sms = all;
     return longest > work / sms ? longest : work / sms;
+}
+
+int pb_plan_fill(const pb_req_t *reqs, size_t n, uint32_t sms, uint32_t T, pb_plan_tables_t *out)
+{
+    const double target = shallow_makespan(reqs, n, sms) / 2.0;
+    return pb_plan_requests(reqs, n, T, 32, 0.0, target > 0 ? target : 1.0, out);
 }
 
 static int cmp_double(const void *a, const void *b)
@@ -881,7 +888,7 @@ no_split:
              * parts' makespan (they fill the SMs those leave), or half of
              * what the requests need on all SMs */
             double target = ukern == 1 ? 1e30 : makespan / 3.0;
-            if (target <= 0) target = shallow_makespan(ps, ns) / 2.0;
+            if (target <= 0) target = shallow_makespan(ps, ns, 0) / 2.0;
             if (target <= 0) target = 1.0;
             if (ukern == 1) T = uT;
             if (pb_plan_requests(ps, ns, T, ukern == 1 ? uG : 32, 0.0, target, &pl[0]) != 0) goto fail;

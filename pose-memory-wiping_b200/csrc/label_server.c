@@ -22,10 +22,11 @@
  *   - finished waves are reaped and their arena range is zeroed on the device
  *     before it is reused;
  *   - deep requests (topologies of at least PB_SERVER_DEEP_LEVELS levels,
- *     chunk_blocks 2^17 and up) do not join waves: the pending deep requests
- *     of one topology run together on the multi-unit depth kernel
- *     (k_label_ws: a producer warp and 15 hashing warps per CTA, three chunk
- *     copies per CTA) in a slot of their own, on a high-priority stream.
+ *     chunk_blocks 2^15 and up) do not join waves: the pending deep requests
+ *     of one topology run together on the depth kernel (k_label_ws: a
+ *     producer warp and 15 hashing warps per CTA, one to four chunk copies
+ *     per CTA by the load) in a slot of their own, on a high-priority stream;
+ *     an eighth of the SMs stays with the waves.
  *     Each depth CTA holds its SM alone (its shared memory is raised to the
  *     limit), so no lockstep warp slows its chain, and at most one depth CTA
  *     per SM is in flight: a deep request that does not fit the free SMs
@@ -58,15 +59,23 @@
 #define PB_SERVER_MAX_WAVES 16
 /* Concurrent launches of the depth kernel. */
 #define PB_SERVER_MAX_DEEP 16
-/* Requests whose topology has at least this many levels (chunk_blocks 2^17
+/* Requests whose topology has at least this many levels (chunk_blocks 2^15
  * and up) run on the depth kernel instead of joining a wave.  On the
- * 120-request Poisson trace (200 requests/s, chunk_blocks 2^10..2^18), with
- * three chunk copies per depth CTA: 603 MiB/s, against 549 with only 2^18 on
- * the depth kernel and 448 with every request in waves. */
-#define PB_SERVER_DEEP_LEVELS 300000u
-/* Chunk copies per depth CTA under the default policy (measured on the same
- * trace: 3 copies 549-603 MiB/s, 4 copies 515-548, 2 copies 520). */
-#define PB_SERVER_DEEP_UNITS 3u
+ * 120-request Poisson trace (200 requests/s, chunk_blocks 2^10..2^18): 559 to
+ * 632 MiB/s, p50 0.31 to 0.37 s and p99 2.7 to 2.9 s with 2^15 and up, 544
+ * MiB/s, 0.24 and 2.86 s with 2^14 and up, and at most 441 MiB/s with 2^17
+ * and up; with 2^17 and up at three copies a CTA and waves of small teams it
+ * was 591 MiB/s, 1.27 and 2.8 s. */
+#define PB_SERVER_DEEP_LEVELS 90000u
+/* Chunk copies per depth CTA: 0 = as many as there are chunk copies of deep
+ * requests, waiting or running, per SM that the depth kernel may hold, at
+ * most PB_SERVER_DEEP_MOST.  A burst of 48 requests (2^10..2^17) then takes
+ * 491 ms, the chain of one 2^17 copy, against 817 at three copies a CTA; on
+ * the trace, which overloads the GPU three times, at most 3, 4, 5 and 8
+ * copies give 579, 611, 420 and 474 MiB/s: packing more makes the last 2^18
+ * requests too long. */
+#define PB_SERVER_DEEP_UNITS 0u
+#define PB_SERVER_DEEP_MOST 4u
 /* Hashing warps of a depth-kernel CTA. */
 #define PB_SERVER_DEEP_WARPS 15u
 /* A deep request joins a wave instead when more than this many requests
@@ -102,6 +111,7 @@ typedef struct {
     int deep;                  /* deep requests on the depth kernel (complete with the launch) */
     uint32_t chan;             /* the host-to-device work queue its stream maps to (creation order) */
     uint32_t ctas;             /* its CTAs, one SM each */
+    uint64_t units;            /* and chunk copies */
 } wave_t;
 
 struct pose_b200_server {
@@ -126,13 +136,15 @@ struct pose_b200_server {
     wave_t deeps[PB_SERVER_MAX_DEEP]; /* depth-kernel launches, high-priority streams */
     uint32_t max_waves;        /* concurrent multi-topology waves */
     uint32_t deep_ctas;        /* depth-kernel CTAs in flight */
+    uint64_t deep_inflight;    /* chunk copies they were launched for */
     uint32_t deep_queue;       /* deep requests take the depth kernel while at most this many requests wait */
-    uint32_t deep_units;       /* units per depth CTA: 0 = the fewest of 1, 2, 4 that fit the free SMs */
+    uint32_t deep_units;       /* units per depth CTA: 0 = by the load (PB_SERVER_DEEP_UNITS) */
     uint32_t deep_gmax;        /* most units per depth CTA */
     int deep_wait;             /* a deep request that does not fit waits for SMs instead of joining a wave */
     int deep_excl;             /* a depth CTA holds its SM alone (shared memory raised to the limit) */
     uint32_t deep_levels;      /* requests of topologies with at least this many levels are deep */
-    uint32_t sms;
+    uint32_t sms;              /* SMs the depth kernel may hold */
+    uint32_t all_sms;
     uint32_t conns;            /* host-to-device work queues (CUDA_DEVICE_MAX_CONNECTIONS, default 8) */
     uint32_t wsg_smem_max;     /* the depth kernel's shared-memory limit (0: no depth kernel) */
     int occ;
@@ -205,7 +217,7 @@ static int req_is_deep(const pose_b200_server_t *s, const pose_hbm_topo_t *topo)
     pb_topo_view2_t v2;
     if (!s->wsg_smem_max || pb_topo_internal(topo, &ti) != 0 || ti.view.L < s->deep_levels) return 0;
     if (pb_topo_view2(topo, &v2) != 0) return 0;
-    return pb_ws_smem_bytes(v2.csm, 4, PB_SERVER_DEEP_WARPS) <= s->wsg_smem_max &&
+    return pb_ws_smem_bytes(v2.csm, s->deep_gmax, PB_SERVER_DEEP_WARPS) <= s->wsg_smem_max &&
            (uint64_t)v2.gpool * 32 <= s->arena_bytes;
 }
 
@@ -268,15 +280,13 @@ static int chan_busy(const pose_b200_server_t *s, uint32_t chan)
 }
 
 /* With the lock held: launch the pending deep requests of the oldest pending
- * deep request's topology, oldest first, on the multi-unit depth kernel in a
- * free deep slot, one chunk copy per CTA and CTA per SM (the CTAs in flight
- * count against the SMs): the shortest chains.  Requests are taken while
- * their copies fit the free SMs.  When the oldest one does not fit, or more
- * than PB_SERVER_DEEP_QUEUE requests are pending, the GPU is loaded: it joins
- * the next wave instead, where the lockstep kernel packs many copies per SM
- * (on a loaded GPU the depth kernel's one SM per copy costs more throughput
- * than its shorter chain saves).  The requests complete with the launch.  Returns 1 when something was launched, failed
- * or moved to the waves, 0 when nothing could be done. */
+ * deep request's topology, oldest first, on the depth kernel in a free deep
+ * slot, one CTA per SM (the CTAs in flight count against the SMs).  Requests
+ * are taken while their copies fit the free SMs.  When the oldest one does
+ * not fit it waits; with POSE_B200_SERVER_DEEP_WAIT=0, or when more than
+ * PB_SERVER_DEEP_QUEUE requests are pending, it joins the next wave instead.
+ * The requests complete with the launch.  Returns 1 when something was
+ * launched, failed or moved to the waves, 0 when nothing could be done. */
 static int admit_deep(pose_b200_server_t *s)
 {
     size_t i0 = s->next_pending;
@@ -332,25 +342,18 @@ static int admit_deep(pose_b200_server_t *s)
         pthread_cond_broadcast(&s->cv);
         return 1;
     }
-    /* units per CTA: on an otherwise idle depth kernel (nothing of it in
-     * flight, no other deep request waiting) the fewest that fit the free
-     * SMs, for the shortest chains; under load the most, for the most chains
-     * per SM (a narrow level of G units is still one warp pass) */
+    /* units per CTA: by the load, all deep units waiting or running spread
+     * over the SMs the depth kernel may hold */
     uint32_t G = s->deep_units;
     if (!G) {
-        size_t others = 0;
+        uint64_t all = s->deep_inflight;
         for (size_t i = i0; i < s->nreqs; i++) {
             const sreq_t *r = &s->reqs[i];
-            others += r->state == 0 && r->deep;
+            pb_topo_internal_t x;
+            if (r->state == 0 && r->deep && pb_topo_internal(r->topo, &x) == 0) all += (r->len / x.super_bytes) * x.copies;
         }
-        others -= n;
-        if (s->deep_ctas > 0 || others > 0) {
-            G = gmax;
-        } else {
-            G = 1;
-            while (G < gmax && (units + G - 1) / G > free_sms) G *= 2;
-            if (G > gmax) G = gmax;
-        }
+        const uint64_t want = (all + s->sms - 1) / s->sms;
+        G = want < 1 ? 1 : want < gmax ? (uint32_t)want : gmax;
     }
     const uint64_t nbatches = (units + G - 1) / G;
     uint32_t grid = (uint32_t)(nbatches < free_sms ? nbatches : free_sms);
@@ -430,10 +433,12 @@ static int admit_deep(pose_b200_server_t *s)
         wv->busy = 1;
         wv->deep = 1;
         wv->ctas = grid;
+        wv->units = units;
         wv->arena_off = off;
         wv->arena_len = scratch;
         wv->nreqs = n;
         s->deep_ctas += grid;
+        s->deep_inflight += units;
         for (size_t k = 0; k < n; k++) {
             s->reqs[wv->reqs[k]].state = 1;
             s->reqs[wv->reqs[k]].t_start = t;
@@ -459,6 +464,7 @@ static int admit_wave(pose_b200_server_t *s)
     wave_t *wv = &s->waves[w];
     wv->deep = 0;
     wv->ctas = 0;
+    wv->units = 0;
     size_t n = 0;
     for (size_t i = s->next_pending; i < s->nreqs; i++) n += s->reqs[i].state == 0 && !s->reqs[i].deep;
     if (n == 0) return 0;
@@ -480,9 +486,8 @@ static int admit_wave(pose_b200_server_t *s)
         pr[i].seed_len = s->sess_len[r->session];
     }
     pb_plan_tables_t pl;
-    uint32_t Tw = 4;
-    double eff = 0.0;
-    if (pb_plan_choose(pr, n, NULL, &Tw, &eff) != 0 || pb_plan_requests(pr, n, Tw, 32, eff, 0.0, &pl) != 0) {
+    const uint32_t Tw = 16;
+    if (pb_plan_fill(pr, n, s->all_sms - s->deep_ctas, Tw, &pl) != 0) {
         free(pr);
         for (size_t i = 0; i < n; i++) { s->reqs[wv->reqs[i]].state = 3; s->reqs[wv->reqs[i]].t_done = now_ms(); }
         pthread_cond_broadcast(&s->cv);
@@ -502,8 +507,7 @@ static int admit_wave(pose_b200_server_t *s)
     }
     /* teams: as many as fit in the largest free arena range, the GPU and the
      * batches; one team per CTA, every team with its scratch */
-    const uint32_t tpc_max = 256 / (32 * Tw);
-    uint64_t cap = (uint64_t)pl.sms * (s->occ > 0 ? s->occ : 1) * tpc_max;
+    const uint64_t cap = (uint64_t)pl.sms * (s->occ > 0 ? s->occ : 1);
     uint64_t R = arena_largest(s) / pl.team_scratch;
     if (R > cap) R = cap;
     if (R > pl.nbatches) R = pl.nbatches;
@@ -649,7 +653,10 @@ static int reap(pose_b200_server_t *s)
             cudaGetLastError();
         }
         arena_give(s, wv->arena_off, wv->arena_len);
-        if (wv->deep) s->deep_ctas -= wv->ctas;
+        if (wv->deep) {
+            s->deep_ctas -= wv->ctas;
+            s->deep_inflight -= wv->units;
+        }
         wv->busy = 0;
         k++;
     }
@@ -745,8 +752,9 @@ pose_b200_server_t *pose_b200_server_create(uint64_t scratch_bytes, uint32_t max
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device) != cudaSuccess || sms <= 0) sms = 1;
         /* POSE_B200_SERVER_DEEP_SMS caps the SMs the depth kernel may hold (tests, tuning) */
         const char *e = getenv("POSE_B200_SERVER_DEEP_SMS");
-        if (e && atoi(e) > 0 && atoi(e) < sms) sms = atoi(e);
-        s->sms = (uint32_t)sms;
+        s->all_sms = (uint32_t)sms;
+        s->sms = s->all_sms > 8 ? s->all_sms - s->all_sms / 8 : s->all_sms;
+        if (e && atoi(e) > 0 && atoi(e) < sms) s->sms = (uint32_t)atoi(e);
         uint32_t mx = 0;
         if (pb_dev_label_ws_prepare(&mx) != 0) mx = 0; /* no depth kernel: deep requests join waves */
         cudaGetLastError();
@@ -755,7 +763,7 @@ pose_b200_server_t *pose_b200_server_create(uint64_t scratch_bytes, uint32_t max
         /* deep-request policy (tuning): queue threshold, units per CTA, wait or join a wave, SM held alone */
         s->deep_queue = PB_SERVER_DEEP_QUEUE;
         s->deep_units = PB_SERVER_DEEP_UNITS;
-        s->deep_gmax = 4;
+        s->deep_gmax = PB_SERVER_DEEP_MOST;
         s->deep_wait = 1;
         s->deep_excl = 1;
         s->deep_levels = PB_SERVER_DEEP_LEVELS;
@@ -764,15 +772,15 @@ pose_b200_server_t *pose_b200_server_create(uint64_t scratch_bytes, uint32_t max
         const char *e1 = getenv("POSE_B200_SERVER_DEEP_QUEUE");
         if (e1 && e1[0]) s->deep_queue = (uint32_t)atoi(e1);
         const char *e2 = getenv("POSE_B200_SERVER_DEEP_UNITS");
-        if (e2 && atoi(e2) >= 0 && atoi(e2) <= 4) s->deep_units = (uint32_t)atoi(e2);
+        if (e2 && atoi(e2) >= 0 && atoi(e2) <= (int)PB_WS_MAX_UNITS) s->deep_units = (uint32_t)atoi(e2);
         const char *e3 = getenv("POSE_B200_SERVER_DEEP_GMAX");
-        if (e3 && atoi(e3) >= 1 && atoi(e3) <= 4) s->deep_gmax = (uint32_t)atoi(e3);
+        if (e3 && atoi(e3) >= 1 && atoi(e3) <= (int)PB_WS_MAX_UNITS) s->deep_gmax = (uint32_t)atoi(e3);
         const char *e4 = getenv("POSE_B200_SERVER_DEEP_WAIT");
         if (e4 && e4[0]) s->deep_wait = atoi(e4) != 0;
         const char *e5 = getenv("POSE_B200_SERVER_DEEP_EXCL");
         if (e5 && e5[0]) s->deep_excl = atoi(e5) != 0;
     }
-    if (pb_dev_label_multi_occupancy(256, &s->occ) != 0) s->occ = 1;
+    if (pb_dev_label_multi_occupancy(512, &s->occ) != 0) s->occ = 1;
     /* Launch tables and completion counters of every slot, allocated up
      * front: the dispatcher then makes no allocation while kernels run (a
      * cudaFree there waits for the whole device, and the submitters and
