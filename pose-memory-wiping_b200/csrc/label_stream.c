@@ -6,11 +6,15 @@
  * pinned stage and writes it, strictly one after the other
  * (tools/disk-wipe-bench/disk_wipe_bench.cu:646-697).  Here the region is cut
  * into windows of whole super-chunks labelled alternately into two device
- * buffers; a worker thread copies each finished window into one of two pinned
- * host buffers on its own stream and hands it to the sink, while the calling
- * thread already labels the next window.  The sink has the shape of the
- * reference's pose_label_sink_fn (common/include/graph.h:244-245) and, as
- * there, may be called from a worker thread.
+ * buffers; a worker thread copies each finished window into a pinned host
+ * buffer on its own stream and hands it to the sink, while the calling thread
+ * already labels the next ones.  A window of few chunk copies leaves most of
+ * the GPU idle for the length of their chain, so consecutive windows are
+ * labelled in one call until it has some eight copies per SM
+ * (PB_STREAM_UNITS); the sink still gets them one by one, in order.  The sink
+ * has the shape of the reference's pose_label_sink_fn
+ * (common/include/graph.h:244-245) and, as there, may be called from a worker
+ * thread.
  */
 #include "pose_b200.h"
 #include "dev_alloc.h"
@@ -23,10 +27,16 @@
 #include <string.h>
 #include <time.h>
 
+/* Chunk copies of one labelling call.  2048 chunks of 4096 blocks in windows
+ * of 256 chunks, 512 copies: 19.9 ms a call; 1024 copies 28.5, 1536 copies
+ * about 36, 4096 copies 78. */
+#define PB_STREAM_UNITS 1184u
+
 typedef struct {
     pthread_mutex_t mu;
     pthread_cond_t cv;
-    /* job handed to the worker (valid when posted) */
+    /* job handed to the worker (valid when posted): the windows in dev[buf],
+     * len bytes, the first at byte offset off */
     int posted, quit;
     int buf;
     size_t len;
@@ -34,9 +44,10 @@ typedef struct {
     /* per buffer: 1 while the worker still uses it */
     int busy[2];
     int error;
+    size_t window; /* bytes */
     double d2h_ms, sink_ms;
     /* resources */
-    uint8_t *dev[2], *host[2];
+    uint8_t *dev[2], *host;
     cudaStream_t stream;
     int device;
     pose_b200_sink_fn sink;
@@ -50,11 +61,42 @@ static double now_ms(void)
     return 1e3 * (double)ts.tv_sec + 1e-6 * (double)ts.tv_nsec;
 }
 
+/* Copy the windows of one labelling call to the pinned buffer and sink them,
+ * one after the other. */
+static int sink_windows(stream_state_t *s, int i, size_t len, uint64_t off)
+{
+    for (size_t at = 0; at < len; at += s->window) {
+        const size_t n = len - at < s->window ? len - at : s->window;
+        const double t0 = now_ms();
+        if (cudaMemcpyAsync(s->host, s->dev[i] + at, n, cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
+            cudaStreamSynchronize(s->stream) != cudaSuccess) {
+            fprintf(stderr, "pose_b200_label_stream: D2H copy failed: %s\n", cudaGetErrorString(cudaGetLastError()));
+            return -1;
+        }
+        const double t1 = now_ms();
+        if (s->sink(s->ctx, s->host, n, off + at) != 0) {
+            fprintf(stderr, "pose_b200_label_stream: sink failed at offset %llu\n", (unsigned long long)(off + at));
+            return -1;
+        }
+        s->d2h_ms += t1 - t0;
+        s->sink_ms += now_ms() - t1;
+    }
+    return 0;
+}
+
 static void *sink_worker(void *arg)
 {
     stream_state_t *s = (stream_state_t *)arg;
     cudaSetDevice(s->device);
+    /* pinned here, while the first windows are labelled */
+    const int have = cudaMallocHost((void **)&s->host, s->window) == cudaSuccess;
+    if (!have) {
+        cudaGetLastError();
+        s->host = NULL;
+        fprintf(stderr, "pose_b200_label_stream: pinned buffer of %llu bytes failed\n", (unsigned long long)s->window);
+    }
     pthread_mutex_lock(&s->mu);
+    if (!have) s->error = 1;
     for (;;) {
         while (!s->posted && !s->quit) pthread_cond_wait(&s->cv, &s->mu);
         if (!s->posted && s->quit) break;
@@ -63,25 +105,10 @@ static void *sink_worker(void *arg)
         uint64_t off = s->off;
         s->posted = 0;
         pthread_cond_broadcast(&s->cv);
+        const int skip = s->error; /* nothing is sunk after a failure */
         pthread_mutex_unlock(&s->mu);
-
-        int err = 0;
-        double t0 = now_ms();
-        if (cudaMemcpyAsync(s->host[i], s->dev[i], len, cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
-            cudaStreamSynchronize(s->stream) != cudaSuccess) {
-            fprintf(stderr, "pose_b200_label_stream: D2H copy failed: %s\n", cudaGetErrorString(cudaGetLastError()));
-            err = -1;
-        }
-        double t1 = now_ms();
-        if (!err && s->sink(s->ctx, s->host[i], len, off) != 0) {
-            fprintf(stderr, "pose_b200_label_stream: sink failed at offset %llu\n", (unsigned long long)off);
-            err = -1;
-        }
-        double t2 = now_ms();
-
+        const int err = skip ? -1 : sink_windows(s, i, len, off);
         pthread_mutex_lock(&s->mu);
-        s->d2h_ms += t1 - t0;
-        s->sink_ms += t2 - t1;
         if (err) s->error = 1;
         s->busy[i] = 0;
         pthread_cond_broadcast(&s->cv);
@@ -108,6 +135,23 @@ static int pose_b200_label_stream_impl(const pose_hbm_topo_t *topo, const uint8_
     uint64_t W = window_bytes / sb;
     if (W == 0) W = 1;
     if (W > nsuper) W = nsuper;
+    /* windows per labelling call: up to PB_STREAM_UNITS chunk copies, half
+     * the region (the first half is sunk while the second is labelled) and a
+     * quarter of the free device memory; a caller's schedule is for its own
+     * window */
+    uint64_t per = 1;
+    if (!sched) {
+        const uint64_t copies = W * 2, half = (nsuper + W - 1) / W / 2;
+        size_t fr = 0, tot = 0;
+        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+            cudaGetLastError();
+            fr = 0;
+        }
+        per = (PB_STREAM_UNITS + copies - 1) / copies;
+        if (per > half) per = half;
+        while (per > 1 && 2 * per * W * sb > fr / 4) per--;
+        if (per == 0) per = 1;
+    }
     const uint64_t wbytes = W * sb;
 
     stream_state_t s;
@@ -116,6 +160,7 @@ static int pose_b200_label_stream_impl(const pose_hbm_topo_t *topo, const uint8_
     pthread_cond_init(&s.cv, NULL);
     s.sink = sink;
     s.ctx = sink_ctx;
+    s.window = wbytes;
     cudaGetDevice(&s.device);
     int rc = -1, started = 0;
     pthread_t th;
@@ -126,10 +171,18 @@ static int pose_b200_label_stream_impl(const pose_hbm_topo_t *topo, const uint8_
     memset(&last, 0, sizeof(last));
 
     for (int i = 0; i < 2; i++) {
-        if (pb_dev_malloc((void **)&s.dev[i], wbytes) != cudaSuccess ||
-            cudaMallocHost((void **)&s.host[i], wbytes) != cudaSuccess) {
+        const uint64_t cbytes = per * wbytes;
+        if (pb_dev_malloc((void **)&s.dev[i], cbytes) != cudaSuccess) {
+            cudaGetLastError();
+            if (per > 1) { /* one window a call then */
+                per = 1;
+                if (i) cudaFree(s.dev[0]);
+                s.dev[0] = NULL;
+                i = -1;
+                continue;
+            }
             fprintf(stderr, "pose_b200_label_stream: window buffers of %llu bytes failed\n",
-                    (unsigned long long)wbytes);
+                    (unsigned long long)cbytes);
             goto out;
         }
     }
@@ -137,9 +190,9 @@ static int pose_b200_label_stream_impl(const pose_hbm_topo_t *topo, const uint8_
     if (pthread_create(&th, NULL, sink_worker, &s) != 0) goto out;
     started = 1;
 
-    for (uint64_t k = 0, first = 0; first < nsuper; k++, first += W) {
+    for (uint64_t k = 0, first = 0; first < nsuper; k++, first += per * W) {
         const int i = (int)(k & 1);
-        const uint64_t n = nsuper - first < W ? nsuper - first : W;
+        const uint64_t n = nsuper - first < per * W ? nsuper - first : per * W;
         pthread_mutex_lock(&s.mu);
         while (s.busy[i] && !s.error) pthread_cond_wait(&s.cv, &s.mu);
         int err = s.error;
@@ -191,10 +244,8 @@ out:
         stats->nodes = nodes;
         stats->kernel_launches = launches;
     }
-    for (int i = 0; i < 2; i++) {
-        cudaFree(s.dev[i]);
-        if (s.host[i]) cudaFreeHost(s.host[i]);
-    }
+    for (int i = 0; i < 2; i++) cudaFree(s.dev[i]);
+    if (s.host) cudaFreeHost(s.host);
     if (s.stream) cudaStreamDestroy(s.stream);
     pthread_mutex_destroy(&s.mu);
     pthread_cond_destroy(&s.cv);
