@@ -168,7 +168,7 @@ int pb_dev_set_keys(const uint32_t ksrc[8], const uint32_t kint[8], const uint32
 int pb_dev_cv0_table(const void *recs, uint32_t S, uint32_t copies, void *cv0, cudaStream_t stream);
 int pb_dev_chunk_seeds(const uint8_t *d_session_seed, uint32_t seed_len, uint64_t rbo, uint32_t cb,
                        uint32_t nchunks, uint64_t first_super, uint32_t *d_seeds,
-                       cudaStream_t stream);
+                       unsigned int *d_queue, cudaStream_t stream);
 /* smem_bytes: dynamic shared memory per CTA, 0 = the staging area alone
  * (PB_PREF_BYTES_PER_THREAD per thread); more caps residency per SM
  * (pb_dev_label_balance_smem). */

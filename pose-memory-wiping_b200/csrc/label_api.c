@@ -75,6 +75,15 @@ static double now_sec(void)
     return (double)ts.tv_sec + 1e-9 * (double)ts.tv_nsec;
 }
 
+/* One launch as planned. */
+typedef struct {
+    uint32_t T, G, teams, grid, cta, kernel, smem;
+    uint32_t per_sm; /* lockstep kernel: teams per SM to cap residency at (0 = no cap) */
+    uint32_t cluster; /* depth kernel: CTAs per chunk copy (1 = k_label_ws, >1 = k_label_wsc) */
+    uint64_t team_scratch, scratch_bytes;
+    double cost;
+} plan_t;
+
 struct pose_hbm_topo {
     int device;
     uint32_t cb;
@@ -106,6 +115,9 @@ struct pose_hbm_topo {
     size_t sess_alloc;
     unsigned int *d_queue;
     int occ_team[5], sms; /* k_label CTAs (one team of 2^i warps each) per SM */
+    /* the last automatic plan that free memory did not limit, and its units */
+    plan_t plan;
+    uint64_t plan_units;
     /* schedule chosen by pose_b200_topo_autotune for calls of tuned_units chunk copies */
     int tuned_ok;
     uint64_t tuned_units;
@@ -114,13 +126,6 @@ struct pose_hbm_topo {
 
 /* ── schedule model ──────────────────────────────────────────────────────── */
 
-typedef struct {
-    uint32_t T, G, teams, grid, cta, kernel, smem;
-    uint32_t per_sm; /* lockstep kernel: teams per SM to cap residency at (0 = no cap) */
-    uint32_t cluster; /* depth kernel: CTAs per chunk copy (1 = k_label_ws, >1 = k_label_wsc) */
-    uint64_t team_scratch, scratch_bytes;
-    double cost;
-} plan_t;
 
 #define PB_CSM 480u /* shared-memory label slots per copy in the pipelined records */
 #define PB_SPLIT_WIDTH 480u  /* levels a depth-kernel cluster shares: wider than one pass of its hashing threads */
@@ -776,6 +781,33 @@ int pose_b200_topo_autotune(pose_hbm_topo_t *t, const uint8_t *session_seed, siz
     return 0;
 }
 
+/* The schedule of a labelling call.  Asking for the free device memory and
+ * going through the schedules took a tenth of a small call, so the plan that
+ * memory does not limit is made first and, for a call without a schedule,
+ * kept with its number of units; it is used as it is when the workspace
+ * already holds its scratch. */
+static int call_plan(pose_hbm_topo_t *t, uint64_t nunits, const pose_b200_sched_t *sched, uint64_t *budget,
+                     plan_t *plan)
+{
+    const uint64_t cap = sched && sched->scratch_cap_bytes ? sched->scratch_cap_bytes : (uint64_t)1 << 62;
+    const int keep = !sched && !getenv("POSE_B200_TEAMS_PER_SM");
+    if (keep && t->plan_units == nunits && t->plan.scratch_bytes <= t->scratch_alloc) {
+        *plan = t->plan;
+        *budget = plan->scratch_bytes;
+        return 0;
+    }
+    if (make_plan(t, nunits, sched, cap, plan) == 0) {
+        if (keep) {
+            t->plan = *plan;
+            t->plan_units = nunits;
+        }
+        *budget = plan->scratch_bytes;
+        if (plan->scratch_bytes <= t->scratch_alloc) return 0;
+    }
+    *budget = scratch_budget(t, sched);
+    return make_plan(t, nunits, sched, *budget, plan);
+}
+
 /* The labeling call.  Chunk seeds come either from the session seed (derived
  * per super-chunk from its absolute position), or, when raw_seeds is set, are
  * taken as given: raw_seeds holds 32 bytes per super-chunk of the buffer. */
@@ -825,8 +857,8 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
     const uint64_t per_launch = num_super < PB_MAX_CHUNKS_PER_LAUNCH ? num_super : PB_MAX_CHUNKS_PER_LAUNCH;
     plan_t plan;
     if (!sched && t->tuned_ok && t->tuned_units == per_launch * t->copies) sched = &t->tuned;
-    uint64_t budget = scratch_budget(t, sched);
-    if (make_plan(t, per_launch * t->copies, sched, budget, &plan) != 0) {
+    uint64_t budget = 0;
+    if (call_plan(t, per_launch * t->copies, sched, &budget, &plan) != 0) {
         set_err("pose_graph_hbm_topo_label: no schedule fits the scratch budget "
                 "(one copy needs %llu bytes)", (unsigned long long)t->pool * 32ull);
         goto out;
@@ -883,7 +915,7 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
                 CK(cudaStreamSynchronize(t->stream), "seed upload");
             } else if (dev_seeds) {
                 if (pb_dev_chunk_seeds(t->d_sess, (uint32_t)seed_len, rbo, t->cb, (uint32_t)n, first,
-                                       t->d_seeds, t->stream) != 0) {
+                                       t->d_seeds, t->d_queue, t->stream) != 0) {
                     set_err("pose_graph_hbm_topo_label: chunk-seed kernel failed");
                     goto out;
                 }
@@ -900,7 +932,7 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
                    "seed upload");
                 CK(cudaStreamSynchronize(t->stream), "seed upload");
             }
-            CK(cudaMemsetAsync(t->d_queue, 0, 64, t->stream), "queue reset");
+            if (raw_seeds || !dev_seeds) CK(cudaMemsetAsync(t->d_queue, 0, 64, t->stream), "queue reset");
             pb_label_params_t p;
             memset(&p, 0, sizeof(p));
             p.topo = t->view;
@@ -952,10 +984,12 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
             }
             CK(cudaEventRecord(t->ev[2], t->stream), "event");
             launches++;
-            CK(cudaEventSynchronize(t->ev[2]), "label kernel");
-            float ms = 0;
-            if (cudaEventElapsedTime(&ms, t->ev[1], t->ev[2]) != cudaSuccess) { cudaGetLastError(); ms = 0; }
-            kms += ms;
+            if (first + n < num_super) { /* the next launch reuses the events and the seed table */
+                CK(cudaEventSynchronize(t->ev[2]), "label kernel");
+                float ms = 0;
+                if (cudaEventElapsedTime(&ms, t->ev[1], t->ev[2]) != cudaSuccess) { cudaGetLastError(); ms = 0; }
+                kms += ms;
+            }
         }
         /* scratch labels, chunk seeds and the session seed never outlive the
          * call (the reference zeroes its scratch before freeing it,
@@ -965,7 +999,9 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
         if (dev_seeds && seed_len) CK(cudaMemsetAsync(t->d_sess, 0, seed_len, t->stream), "seed zero");
         CK(cudaEventRecord(t->ev[3], t->stream), "event");
         CK(cudaStreamSynchronize(t->stream), "label");
-        float tms = 0;
+        float tms = 0, last = 0;
+        if (cudaEventElapsedTime(&last, t->ev[1], t->ev[2]) != cudaSuccess) { cudaGetLastError(); last = 0; }
+        kms += last;
         if (cudaEventElapsedTime(&tms, t->ev[0], t->ev[3]) != cudaSuccess) { cudaGetLastError(); tms = 0; }
         double elapsed = now_sec() - t0;
         if (stats) {

@@ -92,9 +92,10 @@ __global__ void __launch_bounds__(256) k_cv0_table(const uint4 *__restrict__ rec
 __global__ void __launch_bounds__(128) k_chunk_seeds(const uint8_t *__restrict__ session_seed,
                                                       uint32_t seed_len, uint64_t rbo, uint32_t cb,
                                                       uint32_t nchunks, uint64_t first_super,
-                                                      uint32_t *__restrict__ seeds)
+                                                      uint32_t *__restrict__ seeds, unsigned int *queue)
 {
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j == 0) *queue = 0; /* the work counter of the labeling kernel that follows */
     if (j >= nchunks) return;
     uint64_t idx = (rbo + (first_super + j) * (uint64_t)cb) / cb;
     uint32_t len = seed_len + 8;
@@ -508,12 +509,12 @@ extern "C" int pb_dev_cv0_table(const void *recs, uint32_t S, uint32_t copies, v
 
 extern "C" int pb_dev_chunk_seeds(const uint8_t *d_session_seed, uint32_t seed_len, uint64_t rbo,
                                   uint32_t cb, uint32_t nchunks, uint64_t first_super,
-                                  uint32_t *d_seeds, cudaStream_t stream)
+                                  uint32_t *d_seeds, unsigned int *d_queue, cudaStream_t stream)
 {
     if (nchunks == 0) return 0;
     cudaGetLastError(); /* report only this launch */
     pb::k_chunk_seeds<<<(nchunks + 127) / 128, 128, 0, stream>>>(d_session_seed, seed_len, rbo, cb,
-                                                                  nchunks, first_super, d_seeds);
+                                                                  nchunks, first_super, d_seeds, d_queue);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -124,10 +124,8 @@ extern "C" int pose_b200_topo_label_noalloc(const pose_hbm_topo_t *topo, const u
     for (uint64_t first = 0; first < num_super; first += per_launch) {
         uint64_t n = num_super - first < per_launch ? num_super - first : per_launch;
         if (pb_dev_chunk_seeds(na.session, (uint32_t)seed_len, region_block_offset, ti.cb, (uint32_t)n, first,
-                               na.seeds, s) != 0)
+                               na.seeds, na.queue, s) != 0) /* which zeroes the work counter too */
             goto cuda_fail;
-        /* the work counter must start at zero for every launch */
-        if (cudaMemsetAsync(na.queue, 0, sizeof(unsigned int), s) != cudaSuccess) goto cuda_fail;
         pb_label_params_t p;
         memset(&p, 0, sizeof(p));
         p.topo = ti.view;
