@@ -102,7 +102,7 @@ typedef struct {
     const pb_u4 *cv0;        /* [copies * S * 2] block-0 chaining values (required) */
     const uint32_t *lstart;  /* [L + 1] */
     uint32_t S, L, half_w, retained;
-    uint32_t csm;            /* shared-memory label slots per chunk copy */
+    uint32_t csm;            /* shared-memory label slots used per chunk copy: at most PB_CSM */
     uint32_t gpool;          /* global label slots per chunk copy */
     uint32_t desc[8];
 } pb_topo_view2_t;
@@ -139,9 +139,9 @@ typedef struct {
     uint32_t nsplit;
 } pb_depth_params_t;
 
-/* Dynamic shared memory of a CTA: G label pools of csm slots and the staging
- * areas of team_warps hashing warps. */
-uint32_t pb_ws_smem_bytes(uint32_t csm, uint32_t units_per_cta, uint32_t team_warps);
+/* Dynamic shared memory of a CTA: G label pools of PB_CSM slots and the
+ * staging areas of team_warps hashing warps. */
+uint32_t pb_ws_smem_bytes(uint32_t units_per_cta, uint32_t team_warps);
 /* Raise k_label_ws's dynamic shared memory limit to the most a CTA can have
  * and report it; once per device before any launch or stream capture of it. */
 int pb_dev_label_ws_prepare(uint32_t *max_smem_bytes);

@@ -127,20 +127,14 @@ struct pose_hbm_topo {
 /* ── schedule model ──────────────────────────────────────────────────────── */
 
 
-#define PB_CSM 480u /* shared-memory label slots per copy in the pipelined records */
 #define PB_SPLIT_WIDTH 480u  /* levels a depth-kernel cluster shares: wider than one pass of its hashing threads */
-
-static uint32_t ws_smem_bytes(const pose_hbm_topo_t *t, uint32_t nc, uint32_t G)
-{
-    return pb_ws_smem_bytes(t->view2.csm, G, nc);
-}
 
 static int ws_occupancy(pose_hbm_topo_t *t, uint32_t nc, uint32_t G)
 {
     int *cached = &t->occ_ws[nc == 7 ? 0 : 1][G];
     if (*cached < 0) {
         int occ = 0;
-        if (pb_dev_label_ws_occupancy(32 * (nc + 1), ws_smem_bytes(t, nc, G), &occ) != 0) occ = 0;
+        if (pb_dev_label_ws_occupancy(32 * (nc + 1), pb_ws_smem_bytes(G, nc), &occ) != 0) occ = 0;
         cudaGetLastError();
         *cached = occ;
     }
@@ -159,7 +153,7 @@ static int wsc_clusters(pose_hbm_topo_t *t, uint32_t C)
     if (i < 0 || !t->d_split) return 0;
     if (t->occ_wsc[i] < 0) {
         int n = 0;
-        const uint32_t smem = ws_smem_bytes(t, 15, 1);
+        const uint32_t smem = pb_ws_smem_bytes(1, 15);
         if (smem > 227u * 1024u || pb_dev_label_wsc_max_clusters(C, 15, smem, &n) != 0) n = 0;
         cudaGetLastError();
         t->occ_wsc[i] = n;
@@ -329,7 +323,7 @@ static int make_plan(const pose_hbm_topo_t *ct, uint64_t nunits, const pose_b200
             best->T = nc; best->G = 1; best->teams = (uint32_t)nunits;
             best->grid = (uint32_t)(nunits * C); best->cta = 32 * (nc + 1);
             best->team_scratch = team_scratch; best->scratch_bytes = sbytes;
-            best->cost = cost; best->kernel = 3; best->smem = ws_smem_bytes(t, nc, 1);
+            best->cost = cost; best->kernel = 3; best->smem = pb_ws_smem_bytes(1, nc);
             best->per_sm = 0;
             best->cluster = C;
         }
@@ -355,7 +349,7 @@ static int make_plan(const pose_hbm_topo_t *ct, uint64_t nunits, const pose_b200
                 best->T = nc; best->G = G; best->teams = (uint32_t)R;
                 best->grid = (uint32_t)R; best->cta = 32 * (nc + 1);
                 best->team_scratch = team_scratch; best->scratch_bytes = R * team_scratch;
-                best->cost = cost; best->kernel = 3; best->smem = ws_smem_bytes(t, nc, G);
+                best->cost = cost; best->kernel = 3; best->smem = pb_ws_smem_bytes(G, nc);
                 best->per_sm = 0;
                 best->cluster = 1;
             }

@@ -465,7 +465,7 @@ static int part_setup_wsg(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_t
     q->team_scratch = (uint64_t)G * v2->gpool * 32;
     q->scratch_bytes = (uint64_t)q->grid * q->team_scratch;
     uint32_t max_smem = 0;
-    if (pb_dev_label_ws_prepare(&max_smem) != 0 || pb_ws_smem_bytes(v2->csm, G, NC) > max_smem) {
+    if (pb_dev_label_ws_prepare(&max_smem) != 0 || pb_ws_smem_bytes(G, NC) > max_smem) {
         fprintf(stderr, "pose_b200_batch_create: shared memory attribute: %s\n", cudaGetErrorString(cudaGetLastError()));
         return -1;
     }
@@ -658,14 +658,14 @@ static int plan_deep(const pb_req_t *pd, size_t nd, const pb_req_t *pd2, size_t 
     double best = -1;
     for (uint32_t a = 1; a <= PB_WS_MAX_UNITS; a++) {
         const uint64_t b1 = (u1 + a - 1) / a, s1 = (b1 < sms ? b1 : sms) * (uint64_t)v1.gpool * 32 * a;
-        if ((fix1 && a != fix1) || pb_ws_smem_bytes(v1.csm, a, 15) > max_smem || s1 > budget) continue;
+        if ((fix1 && a != fix1) || pb_ws_smem_bytes(a, 15) > max_smem || s1 > budget) continue;
         const double t1 = pb_topo_depth_clocks(pd[0].topo, a);
         for (uint32_t c = nd2 ? 1 : 0; c <= (nd2 ? PB_WS_MAX_UNITS : 0); c++) {
             uint64_t b2 = 0;
             double t2 = 0;
             if (c) {
                 b2 = (u2 + c - 1) / c;
-                if ((fix2 && c != fix2) || pb_ws_smem_bytes(v2.csm, c, 15) > max_smem) continue;
+                if ((fix2 && c != fix2) || pb_ws_smem_bytes(c, 15) > max_smem) continue;
                 t2 = pb_topo_depth_clocks(pd2[0].topo, c);
             }
             if (b2 > 16ull * sms) continue;
@@ -813,7 +813,7 @@ no_split:
                 cudaGetLastError();
             }
             if (wsg) {
-                const uint32_t smem = pb_ws_smem_bytes(v2.csm, G, 15);
+                const uint32_t smem = pb_ws_smem_bytes(G, 15);
                 if (pb_plan_requests(pd, nd, 8, 1, 0.9999, 0.0, &pl[1]) != 0 || pl[1].nunits == 0) goto fail;
                 if (part_setup_wsg(b, &b->part[1], &pl[1], &v2, G, sms, smem) != 0) goto fail;
                 /* the next-deepest topology's requests: a third launch of the
@@ -830,7 +830,7 @@ no_split:
                     uint32_t max_smem2 = 0;
                     int ok2 = G2 > 0 && pb_topo_view2(pd2[0].topo, &v2b) == 0 &&
                               pb_dev_label_ws_prepare(&max_smem2) == 0 &&
-                              pb_ws_smem_bytes(v2b.csm, G2, 15) <= max_smem2;
+                              pb_ws_smem_bytes(G2, 15) <= max_smem2;
                     cudaGetLastError();
                     if (ok2) {
                         const uint64_t g2 = (du2 + G2 - 1) / G2 < sms ? (du2 + G2 - 1) / G2 : sms;
@@ -838,7 +838,7 @@ no_split:
                     }
                     if (ok2) {
                         if (pb_plan_requests(pd2, nd2, 8, 1, 0.9999, 0.0, &pl[2]) != 0 || pl[2].nunits == 0) goto fail;
-                        if (part_setup_wsg(b, &b->part[2], &pl[2], &v2b, G2, sms, pb_ws_smem_bytes(v2b.csm, G2, 15)) !=
+                        if (part_setup_wsg(b, &b->part[2], &pl[2], &v2b, G2, sms, pb_ws_smem_bytes(G2, 15)) !=
                             0)
                             goto fail;
                     } else {
@@ -872,7 +872,7 @@ no_split:
         pb_topo_view2_t uv2;
         uint32_t umax = 0;
         if (ukern == 3 && (pb_topo_view2(only, &uv2) != 0 || pb_dev_label_ws_prepare(&umax) != 0 ||
-                           pb_ws_smem_bytes(uv2.csm, uG, 15) > umax)) {
+                           pb_ws_smem_bytes(uG, 15) > umax)) {
             cudaGetLastError();
             ukern = 0;
         }
@@ -881,7 +881,7 @@ no_split:
             pb_topo_internal_t x;
             if (pb_topo_internal(only, &x) != 0 || pb_plan_requests(ps, ns, 8, 1, 0.9999, 0.0, &pl[0]) != 0) goto fail;
             T = 15;
-            if (part_setup_wsg(b, &b->part[0], &pl[0], &uv2, uG, (uint32_t)x.sms, pb_ws_smem_bytes(uv2.csm, uG, 15)) != 0)
+            if (part_setup_wsg(b, &b->part[0], &pl[0], &uv2, uG, (uint32_t)x.sms, pb_ws_smem_bytes(uG, 15)) != 0)
                 goto fail;
         } else if (open_sched) {
             /* 16-warp teams; batches no longer than a third of the deep

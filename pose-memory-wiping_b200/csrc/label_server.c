@@ -217,7 +217,7 @@ static int req_is_deep(const pose_b200_server_t *s, const pose_hbm_topo_t *topo)
     pb_topo_view2_t v2;
     if (!s->wsg_smem_max || pb_topo_internal(topo, &ti) != 0 || ti.view.L < s->deep_levels) return 0;
     if (pb_topo_view2(topo, &v2) != 0) return 0;
-    return pb_ws_smem_bytes(v2.csm, s->deep_gmax, PB_SERVER_DEEP_WARPS) <= s->wsg_smem_max &&
+    return pb_ws_smem_bytes(s->deep_gmax, PB_SERVER_DEEP_WARPS) <= s->wsg_smem_max &&
            (uint64_t)v2.gpool * 32 <= s->arena_bytes;
 }
 
@@ -410,7 +410,7 @@ static int admit_deep(pose_b200_server_t *s)
         p.team_warps = PB_SERVER_DEEP_WARPS;
         p.nbatches = (uint32_t)nbatches;
         p.queue = (unsigned int *)(T + o_queue);
-        const uint32_t need = pb_ws_smem_bytes(v2.csm, G, PB_SERVER_DEEP_WARPS);
+        const uint32_t need = pb_ws_smem_bytes(G, PB_SERVER_DEEP_WARPS);
         ok = pb_dev_label_ws(&p, grid, s->deep_excl && s->wsg_smem_max > need ? s->wsg_smem_max : need, wv->stream) == 0;
     }
     /* scratch and chunk seeds are zeroed before the requests count as done */

@@ -85,25 +85,26 @@ __device__ __forceinline__ void put8(uint32_t *w, uint4 a, uint4 b)
 }
 
 /* Dynamic shared memory, in uint4 units from smem[0]:
- *   zero  [2]            an absent predecessor
+ *   empty [2]            the record of no node
  *   hdr   [3]            (level start, width) of each ring stage
  *   ctx   [G][2]         UnitCtx of each unit
  *   msg   [G][4]         block 2 of each unit: chunk seed | descriptor
  *   tab   [G][28]        the same laid out for quads (quad_table_entry)
- *   pool  [csm][G][2]    next-level labels, slot-major: the G lanes of a node
- *                        read and write neighbouring entries (one pool after
- *                        another would put them all on the same banks)
+ *   pool  [PB_CSM + 1][G][2]  next-level labels, slot-major: the G lanes of a
+ *                        node read and write neighbouring entries (one pool
+ *                        after another would put them all on the same banks);
+ *                        the last slot is zero, an absent predecessor
  *   rec   [3][slots][2]  records, ring of three levels
  *   dat   [2][nthr][6]   per item: block-0 value, predecessor 0, predecessor 1
  * with nthr = 32 NC hashing threads and slots = nthr / G staged nodes. */
 struct Layout {
-    uint32_t nthr, slots, G, ctx, msg, tab, pool, rec, dat, csm;
-    __device__ __forceinline__ Layout(uint32_t nthr_, uint32_t G_, uint32_t csm_)
+    uint32_t nthr, slots, G, ctx, msg, tab, pool, rec, dat;
+    __device__ __forceinline__ Layout(uint32_t nthr_, uint32_t G_)
         : nthr(nthr_), slots(nthr_ / G_), G(G_), ctx(5), msg(5 + 2 * G_), tab(5 + 6 * G_), pool(5 + 34 * G_),
-          rec(5 + 34 * G_ + 2 * G_ * csm_), dat(5 + 34 * G_ + 2 * G_ * csm_ + 6 * (nthr_ / G_)), csm(csm_)
+          rec(pool + 2 * G_ * (PB_CSM + 1)), dat(rec + 6 * (nthr_ / G_))
     {
     }
-    static constexpr uint32_t zero = 0, hdr = 2;
+    static constexpr uint32_t empty = 0, hdr = 2;
     __device__ __forceinline__ uint32_t r(uint32_t st, uint32_t j) const { return rec + (st * slots + j) * 2; }
     __device__ __forceinline__ uint32_t d(uint32_t st, uint32_t k) const { return dat + (st * nthr + k) * 6; }
     __device__ __forceinline__ uint32_t upool(uint32_t u) const { return pool + 2 * u; }
@@ -120,10 +121,11 @@ static_assert(sizeof(UnitCtx) == 32, "two uint4 a unit");
 
 /* A thread's item of a level: its record, and where its operands are in
  * shared memory (byte offsets, so that nothing is left to compute when the
- * level begins): predecessors (the zero area for an absent one or one that
- * is in the global pool) and block-0 value. */
+ * level begins): predecessors (a zero entry for an absent one or one that is
+ * in the global pool) and block-0 value. */
 struct Desc {
     uint32_t x, y, z, gslot, sslot, rank, s0, s1, v;
+    uint32_t global; /* nonzero when a predecessor is in the global pool */
 };
 
 __device__ __forceinline__ uint4 at16(const uint4 *smem, uint32_t off)
@@ -136,11 +138,10 @@ __device__ __forceinline__ bool from_global(uint32_t ref)
     return (ref & (PB_REF_PREV | PB_REF_SMEM)) == PB_REF_PREV;
 }
 
-__device__ __forceinline__ uint32_t operand_at(uint32_t ref, bool have, uint32_t pool, uint32_t staged, uint32_t G2)
+/* Where an operand is: staged at `staged`, or in the unit's pool. */
+__device__ __forceinline__ uint32_t operand_at(uint32_t place, uint32_t pool, uint32_t staged, uint32_t G2)
 {
-    if (!have) return Layout::zero;
-    if (!(ref & PB_REF_PREV)) return staged;
-    return (ref & PB_REF_SMEM) ? pool + (ref & PB_REF_SLOT_MASK) * G2 : Layout::zero;
+    return (place & PB_PLACE_STAGED) ? staged : pool + (place & PB_PLACE_SLOT_MASK) * G2;
 }
 
 /* Descriptor of a staged item: record at smem[rec], operands staged at dat
@@ -149,20 +150,19 @@ __device__ __forceinline__ uint32_t operand_at(uint32_t ref, bool have, uint32_t
 __device__ __forceinline__ Desc load_desc(const uint4 *smem, bool ok, uint32_t rec, uint32_t item, uint32_t pool,
                                           uint32_t G2)
 {
-    const uint32_t at = ok ? rec : Layout::zero;
-    const uint4 r0 = smem[at];
-    const uint2 r1 = *reinterpret_cast<const uint2 *>(&smem[at + 1]);
-    const uint32_t np = (r0.x >> PB_REC_NP_SHIFT) & 3u; /* 0 for the empty one */
+    const uint32_t at = ok ? rec : Layout::empty;
+    const uint4 r0 = smem[at], r1 = smem[at + 1];
     Desc d;
     d.x = r0.x;
     d.y = r0.y;
     d.z = r0.z;
-    d.gslot = ok ? r0.w : PB_NO_SLOT;
-    d.sslot = ok ? r1.x : PB_NO_SLOT;
+    d.gslot = r0.w;
+    d.sslot = r1.x;
     d.rank = r1.y;
-    d.s0 = operand_at(r0.y, np >= 1, pool, item + 2, G2) * 16;
-    d.s1 = operand_at(r0.z, np >= 2, pool, item + 4, G2) * 16;
+    d.s0 = operand_at(r1.z, pool, item + 2, G2) * 16;
+    d.s1 = operand_at(r1.w, pool, item + 4, G2) * 16;
     d.v = item * 16;
+    d.global = (r1.z | r1.w) & PB_PLACE_GLOBAL;
     return d;
 }
 
@@ -238,7 +238,9 @@ __device__ __forceinline__ void setup_units(const pb_depth_params_t &p, uint4 *s
                                             uint32_t cnt, uint32_t pools, uint32_t t, uint32_t nt)
 {
     const pb_topo_view2_t &tp = p.topo;
-    if (t < 2) smem[Layout::zero + t] = make_uint4(0, 0, 0, 0);
+    if (t == 0) smem[Layout::empty] = make_uint4(0, 0, 0, PB_NO_SLOT);
+    if (t == 1) smem[Layout::empty + 1] = make_uint4(PB_NO_SLOT, PB_NO_RANK, PB_CSM, PB_CSM);
+    for (uint32_t k = t; k < 2 * o.G; k += nt) smem[o.pool + 2 * o.G * PB_CSM + k] = make_uint4(0, 0, 0, 0);
     for (uint32_t k = t; k < cnt * 28; k += nt) {
         const uint32_t u = k / 28, e = k - u * 28;
         const uint32_t unit = batch * o.G + u;
@@ -352,8 +354,7 @@ struct NextLevel {
     uint32_t ls, w, global;
     bool quads, busy;
     Desc d;
-    uint4 h, r0;
-    uint2 r1;
+    uint4 h, r0, r1;
 
     template <int R>
     __device__ __forceinline__ void at()
@@ -366,24 +367,23 @@ struct NextLevel {
         } else if (R == 2) {
             quads = w * G <= quad_max;
             busy = quads && warp * 8 < w * G;
-            ok = ok && quads && j4 < w;
-            const uint32_t from = ok ? rec : Layout::zero;
+            const uint32_t from = ok && quads && j4 < w ? rec : Layout::empty;
             r0 = smem[from];
-            r1 = *reinterpret_cast<const uint2 *>(&smem[from + 1]);
+            r1 = smem[from + 1];
         } else if (R == 3) {
             d.x = r0.x;
             d.y = r0.y;
             d.z = r0.z;
-            d.gslot = ok ? r0.w : PB_NO_SLOT;
-            d.sslot = ok ? r1.x : PB_NO_SLOT;
+            d.gslot = r0.w;
+            d.sslot = r1.x;
             d.rank = r1.y;
         } else if (R == 4) {
-            const uint32_t np = (r0.x >> PB_REC_NP_SHIFT) & 3u; /* 0 for the empty record */
-            d.s0 = operand_at(r0.y, np >= 1, pool, item + 2, 2 * G) * 16;
-            d.s1 = operand_at(r0.z, np >= 2, pool, item + 4, 2 * G) * 16;
+            d.s0 = operand_at(r1.z, pool, item + 2, 2 * G) * 16;
+            d.s1 = operand_at(r1.w, pool, item + 4, 2 * G) * 16;
             d.v = item * 16 + lane4;
+            d.global = (r1.z | r1.w) & PB_PLACE_GLOBAL;
         } else if (R == 5) {
-            global = __any_sync(0xFFFFFFFFu, from_global(d.y) || from_global(d.z));
+            global = __any_sync(0xFFFFFFFFu, d.global != 0);
         }
     }
 };
@@ -474,7 +474,7 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
         st1 = st == 2 ? 0 : st + 1;
         busy = w * G <= quad_max && warp * 8 < w * G;
         d = w * G <= quad_max ? quad_desc(lv, st, w) : lane_desc(lv, st, w);
-        global = __any_sync(0xFFFFFFFFu, from_global(d.y) || from_global(d.z));
+        global = __any_sync(0xFFFFFFFFu, d.global != 0);
     };
     const bool skips = warp >= PB_NARROW_WARPS;
     if (CLUSTER && uniform(smem[Layout::hdr].y) > sw) cg::this_cluster().sync(); /* boundary 0 */
@@ -551,7 +551,7 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
                 d = lane_desc(l + 1, st1, w1);
             } else if (busy) {
                 d = quad_desc(l + 1, st1, w1);
-                global = __any_sync(0xFFFFFFFFu, from_global(d.y) || from_global(d.z));
+                global = __any_sync(0xFFFFFFFFu, d.global != 0);
             }
             if (w * G > quad_max) {
                 uint32_t lim = ok1 ? w : 0;
@@ -567,8 +567,8 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
                         put8(m, at16(smem, dl.s0), at16(smem, dl.s0 + 16));
                         put8(m + 8, at16(smem, dl.s1), at16(smem, dl.s1 + 16));
                         put8(cv, at16(smem, dl.v), at16(smem, dl.v + 16));
-                        if (from_global(dl.y)) load_label(m, dl.y, nullptr, 0, cx->gscr);
-                        if (from_global(dl.z)) load_label(m + 8, dl.z, nullptr, 0, cx->gscr);
+                        if (dl.global && from_global(dl.y)) load_label(m, dl.y, nullptr, 0, cx->gscr);
+                        if (dl.global && from_global(dl.z)) load_label(m + 8, dl.z, nullptr, 0, cx->gscr);
                         x = dl.x; gslot = dl.gslot; sslot = dl.sslot; rank = dl.rank;
                     } else {
                         load_direct(p, ls + j, cx, smem + pool1, m, cv, x, gslot, sslot, rank);
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(PB_CTA_THREADS, 1) k_label_ws(const __grid_con
     extern __shared__ uint4 smem[];
     __shared__ uint32_t s_batch;
     const uint32_t G = p.units_per_cta;
-    const Layout o(p.team_warps * 32, G, p.topo.csm);
+    const Layout o(p.team_warps * 32, G);
     for (;;) {
         if (threadIdx.x == 0) s_batch = atomicAdd(p.queue, 1u);
         __syncthreads();
@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(PB_CTA_THREADS, 1) k_label_wsc(const __grid_co
     const uint32_t C = p.cluster;
     const uint32_t rank = cl.block_rank();
     const uint32_t unit = blockIdx.x / C;
-    const Layout o(p.team_warps * 32, 1, tp.csm);
+    const Layout o(p.team_warps * 32, 1);
     setup_units(p, smem, o, unit, 1, unit, threadIdx.x, blockDim.x);
     __syncthreads();
     if (rank == 0) {
@@ -657,10 +657,10 @@ __global__ void __launch_bounds__(PB_CTA_THREADS, 1) k_label_wsc(const __grid_co
 
 } /* namespace pb */
 
-extern "C" uint32_t pb_ws_smem_bytes(uint32_t csm, uint32_t units_per_cta, uint32_t team_warps)
+extern "C" uint32_t pb_ws_smem_bytes(uint32_t units_per_cta, uint32_t team_warps)
 {
     const uint32_t nthr = 32u * team_warps, slots = nthr / units_per_cta;
-    return (5u + 34u * units_per_cta + 2u * units_per_cta * csm + 6u * slots + 12u * nthr) * 16u;
+    return (5u + 34u * units_per_cta + 2u * units_per_cta * (PB_CSM + 1u) + 6u * slots + 12u * nthr) * 16u;
 }
 
 /* Allow a depth kernel the largest dynamic shared memory a CTA can have (the
@@ -691,7 +691,7 @@ extern "C" int pb_dev_label_ws(const pb_depth_params_t *params, uint32_t grid, u
 {
     if (params->units_per_cta < 1 || params->units_per_cta > PB_WS_MAX_UNITS ||
         (params->team_warps != 7 && params->team_warps != 15) ||
-        smem_bytes < pb_ws_smem_bytes(params->topo.csm, params->units_per_cta, params->team_warps))
+        params->topo.csm > PB_CSM || smem_bytes < pb_ws_smem_bytes(params->units_per_cta, params->team_warps))
         return -1;
     cudaGetLastError(); /* report only this launch */
     pb::k_label_ws<<<grid, 32u * (params->team_warps + 1), smem_bytes, stream>>>(*params);
@@ -721,7 +721,8 @@ extern "C" int pb_dev_label_wsc(const pb_depth_params_t *params, uint32_t smem_b
 {
     const uint32_t C = params->cluster;
     if (C < 2 || C > 16 || (params->team_warps != 7 && params->team_warps != 15) || params->nunits == 0 ||
-        params->units_per_cta != 1 || smem_bytes < pb_ws_smem_bytes(params->topo.csm, 1, params->team_warps) ||
+        params->units_per_cta != 1 || params->topo.csm > PB_CSM ||
+        smem_bytes < pb_ws_smem_bytes(1, params->team_warps) ||
         wsc_allow(C) != 0)
         return -1;
     cudaLaunchConfig_t cfg = {};

@@ -234,13 +234,19 @@ static int build_pipelined(uint32_t S, uint32_t L, const uint8_t *np, const uint
     }
     for (uint32_t p = 0; p < S; p++) {
         uint32_t id = order[p], k = np[id], *r = recs + (size_t)8 * p;
-        uint32_t ref[2] = {0, 0};
+        uint32_t ref[2] = {0, 0}, place[2] = {PB_CSM, PB_CSM};
         for (uint32_t e = 0; e < k; e++) {
             uint32_t q = e == 0 ? p0[id] : p1[id];
-            if (lvl[q] + 1 == lvl[id])
-                ref[e] = PB_REF_PREV | (ss[q] != PB_NO_SLOT ? (PB_REF_SMEM | ss[q]) : gs[q]);
-            else
+            if (lvl[q] + 1 != lvl[id]) {
                 ref[e] = gs[q];
+                place[e] = PB_PLACE_STAGED;
+            } else if (ss[q] != PB_NO_SLOT) {
+                ref[e] = PB_REF_PREV | PB_REF_SMEM | ss[q];
+                place[e] = ss[q];
+            } else {
+                ref[e] = PB_REF_PREV | gs[q];
+                place[e] = PB_PLACE_GLOBAL | PB_CSM;
+            }
         }
         r[0] = id | (k << PB_REC_NP_SHIFT) | (rank_of[id] != PB_NO_RANK ? PB_REC_OUT_BIT : 0);
         r[1] = ref[0];
@@ -248,8 +254,8 @@ static int build_pipelined(uint32_t S, uint32_t L, const uint8_t *np, const uint
         r[3] = gs[id];
         r[4] = ss[id];
         r[5] = rank_of[id];
-        r[6] = 0;
-        r[7] = 0;
+        r[6] = place[0];
+        r[7] = place[1];
     }
     t->recs2 = recs;
     recs = NULL;

@@ -42,7 +42,11 @@ extern "C" {
  *       memory)
  *   [4] shared-memory slot this node is copied to, PB_NO_SLOT if none
  *   [5] local output rank, PB_NO_RANK if not an output
- *   [6], [7] zero
+ *   [6], [7] where the depth kernel finds predecessor 0 and 1 as their level
+ *       begins: PB_PLACE_STAGED = staged for the node; else a slot of the
+ *       shared-memory pool, PB_CSM (the entry after the pool, all zero) for an
+ *       absent predecessor and, with PB_PLACE_GLOBAL, for one that is read
+ *       from the global pool instead
  * A node's shared-memory copy lives for its own level and the next; nodes
  * whose level has more next-level-read labels than the pool holds fall back
  * to the global pool. */
@@ -50,6 +54,12 @@ extern "C" {
 #define PB_REF_SMEM (1u << 30)
 #define PB_REF_SLOT_MASK 0x3FFFFFFFu
 #define PB_NO_SLOT 0xFFFFFFFFu
+#define PB_PLACE_STAGED (1u << 31)
+#define PB_PLACE_GLOBAL (1u << 30)
+#define PB_PLACE_SLOT_MASK 0xFFFFu
+/* Shared-memory label slots per copy of the records that the kernels run on
+ * (8 copies a CTA still fit its shared memory). */
+#define PB_CSM 480u
 
 typedef struct pb_topo_host {
     uint32_t cb;        /* chunk_blocks (m) */
