@@ -84,6 +84,7 @@ typedef struct {
     uint32_t nbatches;
     uint32_t team_warps;
     unsigned int *queue;
+    uint32_t table; /* 1: every topology of the launch has its block-0 table */
     /* optional completion signal: when a batch finishes, each of its units
      * adds 1 to req_done[unit_req[unit]] (system-scope, after a system
      * fence), so the host sees every request end as it happens */

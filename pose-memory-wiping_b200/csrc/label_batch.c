@@ -515,6 +515,7 @@ static int part_capture(const batch_part_t *q, cudaStream_t s, cudaEvent_t e0, c
     p.nbatches = (uint32_t)q->nbatches;
     p.team_warps = q->T;
     p.queue = (unsigned int *)q->d_queue;
+    p.table = q->cv0;
     int crc = 0;
     if (e0) crc = cudaEventRecord(e0, s) == cudaSuccess ? 0 : -1;
     if (crc == 0 && q->kind == 1) {

@@ -169,6 +169,44 @@ __device__ __forceinline__ uint4 staged(uint32_t b, uint32_t k)
     return s_stage[((size_t)b * 3 + k) * blockDim.x + threadIdx.x];
 }
 
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+/* Where slot `slot`'s label of this thread's unit is. */
+__device__ __forceinline__ const uint4 *label_at(const UnitCtx &c, uint32_t slot)
+{
+    return c.tscr + ((size_t)slot * c.G + c.u) * 2;
+}
+
+/* Message block 1: the predecessors' labels, zeros for absent ones. */
+__device__ __forceinline__ void pred_words(uint32_t (&m)[16], const UnitCtx &c, uint4 rec, uint32_t np)
+{
+    if (np >= 1) {
+        const uint4 *s = label_at(c, rec.y);
+        const uint4 a = s[0], b = s[1];
+        m[0] = a.x; m[1] = a.y; m[2] = a.z; m[3] = a.w;
+        m[4] = b.x; m[5] = b.y; m[6] = b.z; m[7] = b.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) m[i] = 0;
+    }
+    if (np >= 2) {
+        const uint4 *s = label_at(c, rec.z);
+        const uint4 a = s[0], b = s[1];
+        m[8] = a.x; m[9] = a.y; m[10] = a.z; m[11] = a.w;
+        m[12] = b.x; m[13] = b.y; m[14] = b.z; m[15] = b.w;
+    } else {
+#pragma unroll
+        for (int i = 8; i < 16; i++) m[i] = 0;
+    }
+}
+
+/* Message block 2. */
+__device__ __forceinline__ void seed_words(uint32_t (&m)[16], const pb_topo_view_t &tp, const UnitCtx &c)
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++) { m[i] = c.seed[i]; m[8 + i] = tp.desc[i]; }
+}
+
 /* All levels of one batch: thread (q, u) hashes nodes q, q+stride, ... of
  * every level for unit u; the team syncs between levels.
  *
@@ -177,8 +215,10 @@ __device__ __forceinline__ uint4 staged(uint32_t b, uint32_t k)
  * ahead (cp.async, double-buffered per thread), and the level bounds are read
  * two levels ahead, so that a level's dependent chain is only the
  * predecessor loads, the two compressions and the barrier.  Each thread
- * reads back only its own staging slots, after waiting for its own copies. */
-template <bool CTA_TEAM>
+ * reads back only its own staging slots, after waiting for its own copies.
+ * TABLE: every topology of the launch has its block-0 table (a kernel without
+ * the other path runs 1 % faster than one that has it and does not use it). */
+template <bool TABLE, bool CTA_TEAM>
 __device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const UnitCtx &c, uint32_t T,
                                              uint32_t bar_id, uint32_t TT)
 {
@@ -201,42 +241,39 @@ __device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const Uni
                 const bool first = j == c.q;
                 const uint4 rec = first ? staged(cur, 0) : __ldg(tp.recs + pos);
                 const uint32_t np = (rec.x >> PB_REC_NP_SHIFT) & 3u;
-                uint32_t m[16];
-                if (np >= 1) {
-                    const uint4 *s = c.tscr + ((size_t)rec.y * c.G + c.u) * 2;
-                    uint4 a = s[0], b = s[1];
-                    m[0] = a.x; m[1] = a.y; m[2] = a.z; m[3] = a.w;
-                    m[4] = b.x; m[5] = b.y; m[6] = b.z; m[7] = b.w;
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) m[i] = 0;
-                }
-                if (np >= 2) {
-                    const uint4 *s = c.tscr + ((size_t)rec.z * c.G + c.u) * 2;
-                    uint4 a = s[0], b = s[1];
-                    m[8] = a.x; m[9] = a.y; m[10] = a.z; m[11] = a.w;
-                    m[12] = b.x; m[13] = b.y; m[14] = b.z; m[15] = b.w;
-                } else {
-#pragma unroll
-                    for (int i = 8; i < 16; i++) m[i] = 0;
-                }
-                uint32_t cv[8];
-                if (c.cv0) {
+                uint32_t cv[8], m[16];
+                if (TABLE || c.cv0) {
+                    pred_words(m, c, rec, np);
                     const uint4 c0 = first ? staged(cur, 1) : __ldg(c.cv0 + 2 * (size_t)pos);
                     const uint4 c1 = first ? staged(cur, 2) : __ldg(c.cv0 + 2 * (size_t)pos + 1);
                     cv[0] = c0.x; cv[1] = c0.y; cv[2] = c0.z; cv[3] = c0.w;
                     cv[4] = c1.x; cv[5] = c1.y; cv[6] = c1.z; cv[7] = c1.w;
+                    uint32_t m2[16];
+                    seed_words(m2, tp, c);
+                    compress(cv, m, 64, kFlagsBlock1);
+                    compress(cv, m2, 64, kFlagsBlock2);
                 } else {
-                    uint32_t m0[16];
+                    /* three blocks through one copy of the compression: three
+                     * copies (38 KB) are more than an SM's 32 KB instruction
+                     * cache holds, and a lone warp then runs at half speed.
+                     * The predecessors come in while block 0 is hashed. */
+                    if (np >= 1) prefetch_l1(label_at(c, rec.y));
+                    if (np >= 2) prefetch_l1(label_at(c, rec.z));
                     key_words(cv, np == 0);
-                    block0_words(m0, (rec.x & PB_REC_ID_MASK) + c.id_off);
-                    compress(cv, m0, 64, kFlagsBlock0);
+                    block0_words(m, (rec.x & PB_REC_ID_MASK) + c.id_off);
+                    uint32_t flags = kFlagsBlock0;
+#pragma unroll 1
+                    for (uint32_t b = 0; b <= 2 * opaque_one(); b++) { /* a known count would be unrolled */
+                        compress(cv, m, 64, flags);
+                        if (b == 0) {
+                            flags = kFlagsBlock1;
+                            pred_words(m, c, rec, np);
+                        } else {
+                            flags = kFlagsBlock2;
+                            seed_words(m, tp, c);
+                        }
+                    }
                 }
-                uint32_t m2[16];
-#pragma unroll
-                for (int i = 0; i < 8; i++) { m2[i] = c.seed[i]; m2[8 + i] = tp.desc[i]; }
-                compress(cv, m, 64, kFlagsBlock1);
-                compress(cv, m2, 64, kFlagsBlock2);
                 const uint4 o0 = make_uint4(cv[0], cv[1], cv[2], cv[3]);
                 const uint4 o1 = make_uint4(cv[4], cv[5], cv[6], cv[7]);
                 uint4 *d = c.tscr + ((size_t)rec.w * c.G + c.u) * 2;
@@ -278,6 +315,7 @@ __device__ __forceinline__ uint32_t grab_batch(unsigned int *queue, uint32_t T, 
 
 /* The lockstep kernel for one topology: one team of T warps per CTA
  * (blockDim.x == 32 T), so any number of teams can be resident per SM. */
+template <bool TABLE>
 __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant__ pb_label_params_t p)
 {
     const uint32_t T = p.team_warps;
@@ -309,7 +347,7 @@ __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant_
         c.cv0 = tp.cv0 ? tp.cv0 + (uint64_t)copy * tp.S * 2 : nullptr;
 #pragma unroll
         for (int i = 0; i < 8; i++) c.seed[i] = c.valid ? p.seeds[8 * (size_t)chunk + i] : 0u;
-        label_levels<true>(tp, c, T, bar_id, TT);
+        label_levels<TABLE, true>(tp, c, T, bar_id, TT);
     }
 }
 
@@ -317,6 +355,7 @@ __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant_
  * G units) from a queue sorted longest first, and copy the batch's
  * topology view into shared memory.  One team of T warps per CTA
  * (blockDim.x == 32 T), ending its levels with the CTA barrier. */
+template <bool TABLE>
 __global__ void __launch_bounds__(PB_MULTI_CTA_THREADS, 2) k_label_multi(const __grid_constant__ pb_multi_params_t p)
 {
     const uint32_t T = p.team_warps;
@@ -353,7 +392,7 @@ __global__ void __launch_bounds__(PB_MULTI_CTA_THREADS, 2) k_label_multi(const _
         c.cv0 = tp.cv0 ? tp.cv0 + (uint64_t)copy * tp.S * 2 : nullptr;
 #pragma unroll
         for (int i = 0; i < 8; i++) c.seed[i] = c.valid ? p.seeds[8 * (size_t)un.seed + i] : 0u;
-        label_levels<true>(tp, c, T, bar_id, TT);
+        label_levels<TABLE, true>(tp, c, T, bar_id, TT);
         /* label_levels ended with a team barrier, so every persisted label of
          * the batch is ordered before this fence */
         if (p.req_done != nullptr && tt < bd.count) {
@@ -518,12 +557,40 @@ extern "C" int pb_dev_chunk_seeds(const uint8_t *d_session_seed, uint32_t seed_l
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-/* k_label's 512-thread CTAs stage 48 KiB, which with the static shared
- * memory is above the default per-CTA limit: opt in (idempotent). */
-static void allow_stage_smem()
+/* k_label with and without the block-0 tables. */
+typedef void (*label_kernel_t)(pb_label_params_t);
+static label_kernel_t const k_label_forms[2] = {pb::k_label<false>, pb::k_label<true>};
+
+/* k_label's 512-thread CTAs stage 48 KiB, which with the static shared memory
+ * is above the default per-CTA limit, and padding takes more
+ * (pb_dev_label_balance_smem): allow the device's most, one value for every
+ * caller (idempotent). */
+static int allow_stage_smem()
 {
-    const int bytes = (int)(PB_PREF_BYTES_PER_THREAD * PB_CTA_THREADS);
-    cudaFuncSetAttribute(pb::k_label, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    int dev = 0, optin = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return -1;
+    for (int i = 0; i < 2; i++) {
+        cudaFuncAttributes fa;
+        if (cudaFuncGetAttributes(&fa, k_label_forms[i]) != cudaSuccess ||
+            cudaFuncSetAttribute(k_label_forms[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 optin - (int)fa.sharedSizeBytes) != cudaSuccess)
+            return -1;
+    }
+    return 0;
+}
+
+/* CTAs that an SM holds: the fewest and the most of the two forms. */
+static int label_residency(uint32_t cta_threads, size_t smem, int *least, int *most)
+{
+    int a = 0, b = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_label_forms[0], (int)cta_threads, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_label_forms[1], (int)cta_threads, smem) != cudaSuccess)
+        return -1;
+    *least = a < b ? a : b;
+    *most = a < b ? b : a;
+    return 0;
 }
 
 extern "C" int pb_dev_label(const pb_label_params_t *params, uint32_t grid, uint32_t cta_threads,
@@ -532,16 +599,11 @@ extern "C" int pb_dev_label(const pb_label_params_t *params, uint32_t grid, uint
     if (cta_threads != 32u * params->team_warps || cta_threads > PB_CTA_THREADS) return -1; /* one team per CTA */
     cudaGetLastError(); /* report only this launch */
     uint32_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
-    if (smem_bytes > smem) {
-        if (cudaFuncSetAttribute(pb::k_label, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) !=
-            cudaSuccess)
-            return -1;
-        smem = smem_bytes;
-    } else if (smem > 48 * 1024 - 1024) {
-        allow_stage_smem();
-    }
+    if (smem_bytes > smem) smem = smem_bytes;
+    if (smem > 48 * 1024 - 1024 && allow_stage_smem() != 0) return -1;
     cudaGetLastError();
-    pb::k_label<<<grid, cta_threads, smem, stream>>>(*params);
+    if (params->topo.cv0) pb::k_label<true><<<grid, cta_threads, smem, stream>>>(*params);
+    else pb::k_label<false><<<grid, cta_threads, smem, stream>>>(*params);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -551,7 +613,8 @@ extern "C" int pb_dev_label_multi(const pb_multi_params_t *params, uint32_t grid
     if (cta_threads != 32u * params->team_warps || cta_threads > PB_MULTI_CTA_THREADS) return -1; /* one team per CTA */
     cudaGetLastError(); /* report only this launch */
     const uint32_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
-    pb::k_label_multi<<<grid, cta_threads, smem, stream>>>(*params);
+    if (params->table) pb::k_label_multi<true><<<grid, cta_threads, smem, stream>>>(*params);
+    else pb::k_label_multi<false><<<grid, cta_threads, smem, stream>>>(*params);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -560,12 +623,19 @@ extern "C" int pb_dev_label_multi_occupancy(uint32_t cta_threads, int *blocks_pe
     /* a 512-thread CTA stages 48 KiB, more than the default limit with the
      * static shared memory: one value for every caller (idempotent) */
     const size_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
-    return cudaFuncSetAttribute(pb::k_label_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(PB_PREF_BYTES_PER_THREAD * PB_MULTI_CTA_THREADS)) == cudaSuccess &&
-                   cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pb::k_label_multi, (int)cta_threads,
-                                                                 smem) == cudaSuccess
-               ? 0
-               : -1;
+    const int bytes = (int)(PB_PREF_BYTES_PER_THREAD * PB_MULTI_CTA_THREADS);
+    int a = 0, b = 0;
+    if (cudaFuncSetAttribute(pb::k_label_multi<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(pb::k_label_multi<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, pb::k_label_multi<false>, (int)cta_threads, smem) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, pb::k_label_multi<true>, (int)cta_threads, smem) !=
+            cudaSuccess)
+        return -1;
+    *blocks_per_sm = a < b ? a : b;
+    return 0;
 }
 
 extern "C" int pb_dev_seed_jobs(const void *jobs, uint32_t njobs, const uint8_t *blob, uint32_t *seeds,
@@ -596,18 +666,15 @@ extern "C" int pb_dev_label_balance_smem(uint32_t cta_threads, uint32_t per_sm, 
     if (pb_dev_label_occupancy(cta_threads, &occ) != 0) return -1;
     if ((uint32_t)occ <= per_sm) return 0;
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, pb::k_label) != cudaSuccess) return -1;
+    if (cudaFuncGetAttributes(&fa, pb::k_label<true>) != cudaSuccess) return -1;
     /* largest multiple of 1 KiB with per_sm CTAs fitting the SM's shared memory */
     int64_t each = (int64_t)cap / per_sm - resv - (int64_t)fa.sharedSizeBytes;
     each -= each % 1024;
     if (each > optin - (int64_t)fa.sharedSizeBytes) each = optin - (int64_t)fa.sharedSizeBytes;
     if (each < (int64_t)base) return 0;
     for (; each >= (int64_t)base; each -= 1024) {
-        int m = 0;
-        if (cudaFuncSetAttribute(pb::k_label, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)each) !=
-                cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, pb::k_label, (int)cta_threads, each) != cudaSuccess)
-            return -1;
+        int least = 0, m = 0;
+        if (label_residency(cta_threads, (size_t)each, &least, &m) != 0) return -1;
         if ((uint32_t)m == per_sm) {
             *smem_bytes = (uint32_t)each;
             return 0;
@@ -619,12 +686,10 @@ extern "C" int pb_dev_label_balance_smem(uint32_t cta_threads, uint32_t per_sm, 
 
 extern "C" int pb_dev_label_occupancy(uint32_t cta_threads, int *blocks_per_sm)
 {
-    const size_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
-    allow_stage_smem();
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pb::k_label, (int)cta_threads, smem) ==
-                   cudaSuccess
-               ? 0
-               : -1;
+    int most = 0;
+    return allow_stage_smem() == 0 ? label_residency(cta_threads, PB_PREF_BYTES_PER_THREAD * cta_threads,
+                                                     blocks_per_sm, &most)
+                                   : -1;
 }
 
 extern "C" int pb_dev_label_single(uint32_t *d_out, int is_source, uint64_t node_index,

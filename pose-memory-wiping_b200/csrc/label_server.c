@@ -573,6 +573,7 @@ static int admit_wave(pose_b200_server_t *s)
     p.nbatches = (uint32_t)pl.nbatches;
     p.team_warps = Tw;
     p.queue = (unsigned int *)(T + o_queue);
+    p.table = pl.all_cv0;
     p.unit_req = (const uint32_t *)(T + o_ureq);
     p.req_done = wv->d_done;
     if (ok) ok = pb_dev_label_multi(&p, g2, 32 * Tw, wv->stream) == 0;

@@ -93,3 +93,22 @@ def test_uneven_units(pkg, cuda, oracle, kernel, warps, nsup):
         assert st["kernel"] == kernel and st["units_per_team"] > 1
         assert buf.cpu().numpy().tobytes() == want, st
         assert topo.residue() == 0
+
+
+# a multi-topology launch: all topologies with the block-0 table, some, none
+@pytest.mark.gpu
+@pytest.mark.parametrize("tables", [(True, True), (True, False), (False, False)])
+def test_tables_in_one_launch(pkg, cuda, oracle, tables):
+    sizes = [(33, 70), (300, 5)]
+    topos = [pkg.Topology(cb, cv0_table=t) for (cb, _), t in zip(sizes, tables)]
+    bufs = [cuda.zeros(n * cb * 32, dtype=cuda.uint8, device="cuda") for cb, n in sizes]
+    with pkg.Batch([(t, b"\x22" * 32, b.data_ptr(), b.numel(), 3 * cb)
+                    for t, b, (cb, _) in zip(topos, bufs, sizes)]) as batch:
+        rc, st = batch.run()
+    assert rc == 0, pkg.last_error()
+    assert st["used_cv0_table"] == all(tables)
+    for b, (cb, n) in zip(bufs, sizes):
+        assert b.cpu().numpy().tobytes() == oracle.label_region(b"\x22" * 32, cb, n, 3 * cb, threads=8).tobytes()
+    for t in topos:
+        assert t.residue() == 0
+        t.free()
