@@ -40,7 +40,8 @@ typedef struct {
  * <= 0 packs them while their chain stays within the launch's longest (both
  * in powers of two).  With target > 0 each topology takes instead the most
  * units whose batch the schedule model puts within that many clocks, evened
- * over its batches, and the queue is ordered by those clocks.
+ * over its batches, and the queue is ordered by those clocks; with target < 0
+ * the rule of eff_min holds, within -target clocks a batch.
  * Unit i's seed index is its job's index.  Returns 0, or -1 with a message on
  * stderr (bad request, devices differ, out of host memory). */
 int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, double eff_min, double target,

@@ -92,9 +92,10 @@ typedef struct {
     unsigned int *req_done;
 } pb_multi_params_t;
 
-int pb_dev_label_multi(const pb_multi_params_t *params, uint32_t grid, uint32_t cta_threads, cudaStream_t stream);
+int pb_dev_label_multi(const pb_multi_params_t *params, uint32_t grid, uint32_t cta_threads, uint32_t smem_bytes,
+                       cudaStream_t stream);
 /* Once per device before any launch or stream capture of k_label_multi. */
-int pb_dev_label_multi_occupancy(uint32_t cta_threads, int *blocks_per_sm);
+int pb_dev_label_multi_occupancy(uint32_t cta_threads, int *blocks_per_sm, uint32_t *alone_smem);
 int pb_dev_seed_jobs(const void *jobs, uint32_t njobs, const uint8_t *blob, uint32_t *seeds, cudaStream_t stream);
 
 /* Device view of the pipelined records (topology.h, PB_REF_*). */

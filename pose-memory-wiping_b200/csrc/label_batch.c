@@ -202,7 +202,10 @@ int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, 
      * efficiency G*S / (passes * 32T) reaches eff_min.  eff_min <= 0: pack
      * units as long as the batch's chain of passes stays within the longest
      * chain of the launch at G = 1 (the deepest topology sets the makespan;
-     * packing shallower ones costs no time and fills partial warps). */
+     * packing shallower ones costs no time and fills partial warps).
+     * target > 0 replaces both rules: as many units as a batch finishes in
+     * that many clocks, spread evenly.  target < 0 keeps the rule, within
+     * -target clocks a batch. */
     uint64_t chain_cap = 0;
     for (size_t k = 0; k < ntopo; k++) {
         uint64_t p1 = pb_topo_passes(topo_list[k], T, 1);
@@ -225,6 +228,7 @@ int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, 
             } else if (pb_topo_passes(topo_list[k], T, g * 2) > chain_cap) {
                 break;
             }
+            if (target < 0 && pb_topo_lockstep_clocks(topo_list[k], T, g * 2) > -target) break;
             g *= 2;
         }
         G[k] = g;
@@ -533,7 +537,7 @@ static int part_capture(const batch_part_t *q, cudaStream_t s, cudaEvent_t e0, c
         w.queue = (unsigned int *)q->d_queue;
         crc = pb_dev_label_ws(&w, q->grid, q->smem, s);
     } else if (crc == 0) {
-        crc = pb_dev_label_multi(&p, q->grid, q->cta_threads, s);
+        crc = pb_dev_label_multi(&p, q->grid, q->cta_threads, q->smem, s);
     }
     if (crc == 0 && e1) crc = cudaEventRecord(e1, s) == cudaSuccess ? 0 : -1;
     if (crc == 0) crc = cudaMemsetAsync(q->d_scratch, 0, q->scratch_bytes, s) == cudaSuccess ? 0 : -1;
@@ -606,42 +610,54 @@ int pb_plan_fill(const pb_req_t *reqs, size_t n, uint32_t sms, uint32_t T, pb_pl
     return pb_plan_requests(reqs, n, T, 32, 0.0, target > 0 ? target : 1.0, out);
 }
 
-static int cmp_double(const void *a, const void *b)
-{
-    const double x = *(const double *)a, y = *(const double *)b;
-    return x < y ? -1 : x > y;
-}
+/* Batches of the other requests, beside deep parts, take at most this part of
+ * the whole's estimate. */
+#define PB_FILL_PART (1.0 / 3.0)
 
-/* Clocks until b1 jobs of t1, then b2 of t2 (each on the SM that is free
- * first), and `rest` clocks of small work filled in behind them are done. */
-static double deep_makespan(double *load, uint32_t sms, uint64_t b1, double t1, uint64_t b2, double t2, double rest)
+/* Add n jobs of t clocks to the SMs' loads, each on the one free first. */
+static void place_jobs(double *load, uint32_t sms, uint64_t n, double t)
 {
-    for (uint32_t i = 0; i < sms; i++) load[i] = t1 * (double)(b1 / sms + (i < b1 % sms));
-    for (uint64_t j = 0; j < b2; j++) {
+    for (uint64_t j = 0; j < n; j++) {
         uint32_t m = 0;
         for (uint32_t i = 1; i < sms; i++)
             if (load[i] < load[m]) m = i;
-        load[m] += t2;
+        load[m] += t;
     }
-    qsort(load, sms, sizeof(*load), cmp_double);
-    double level = load[0], left = rest;
-    for (uint32_t i = 1; i <= sms; i++) { /* fill the i least loaded SMs up to the next one */
-        const double next = i < sms ? load[i] : 1e300;
-        if ((next - level) * i >= left) {
-            level += left / i;
-            break;
-        }
-        left -= (next - level) * i;
-        level = next;
-    }
-    return level > load[sms - 1] ? level : load[sms - 1];
+}
+
+static double most_loaded(const double *load, uint32_t sms)
+{
+    double m = load[0];
+    for (uint32_t i = 1; i < sms; i++)
+        if (load[i] > m) m = load[i];
+    return m;
+}
+
+/* Clocks until b1 jobs of t1, then b2 of t2 (each on the SM that is free
+ * first), and `rest` clocks of other work behind them are done.  That work
+ * comes in batches of PB_FILL_PART of an even fill's makespan, which is
+ * *even: a choice that leaves the SMs to the deep parts until the end pays
+ * for the last batches (256 sessions of 2^12..2^17 blocks, 4 and 5 copies a
+ * CTA on 103 and 45 SMs: 1602 ms, 5 and 5 on 82 and 66: 1203). */
+static double deep_makespan(double *load, uint32_t sms, uint64_t b1, double t1, uint64_t b2, double t2, double rest,
+                            double *even)
+{
+    for (uint32_t i = 0; i < sms; i++) load[i] = t1 * (double)(b1 / sms + (i < b1 % sms));
+    place_jobs(load, sms, b2, t2);
+    double sum = rest;
+    for (uint32_t i = 0; i < sms; i++) sum += load[i];
+    *even = most_loaded(load, sms);
+    if (sum / sms > *even) *even = sum / sms;
+    if (rest > 0) place_jobs(load, sms, (uint64_t)(rest / (*even * PB_FILL_PART)) + 1, *even * PB_FILL_PART);
+    return most_loaded(load, sms);
 }
 
 /* Copies per CTA of the two deep parts (pd: nd requests of one topology; pd2:
  * nd2 of another, or none) that the schedule model finishes first, with the
  * other requests ps filled in behind them; fix1, fix2 (nonzero) fix them.
- * On the 256-session workload that is 4 and 8: 98 CTAs of the 2^17 sessions
- * and 49 of the 2^16 ones beside them, each SM one CTA.  Returns 0, or -1
+ * Among choices that finish together the one with the least work on the SMs.
+ * On the 256-session workload that is 5 and 8: 82 CTAs of the 2^17 sessions
+ * and 49 of the 2^16 ones beside them.  Returns 0, or -1
  * when no choice fits the shared memory and the scratch budget. */
 static int plan_deep(const pb_req_t *pd, size_t nd, const pb_req_t *pd2, size_t nd2, const pb_req_t *ps, size_t ns,
                      uint32_t sms, uint64_t budget, uint32_t fix1, uint32_t fix2, uint32_t *G1, uint32_t *G2,
@@ -656,7 +672,7 @@ static int plan_deep(const pb_req_t *pd, size_t nd, const pb_req_t *pd2, size_t 
     const double rest = shallow_work(ps, ns, &longest, &n_sms);
     double *load = (double *)malloc(sms * sizeof(*load));
     if (!load) return -1;
-    double best = -1;
+    double best = -1, best_busy = 0;
     for (uint32_t a = 1; a <= PB_WS_MAX_UNITS; a++) {
         const uint64_t b1 = (u1 + a - 1) / a, s1 = (b1 < sms ? b1 : sms) * (uint64_t)v1.gpool * 32 * a;
         if ((fix1 && a != fix1) || pb_ws_smem_bytes(a, 15) > max_smem || s1 > budget) continue;
@@ -670,23 +686,31 @@ static int plan_deep(const pb_req_t *pd, size_t nd, const pb_req_t *pd2, size_t 
                 t2 = pb_topo_depth_clocks(pd2[0].topo, c);
             }
             if (b2 > 16ull * sms) continue;
-            const double m = deep_makespan(load, sms, b1, t1, b2, t2, rest);
-            if (best < 0 || m < best) {
+            double even, busy = t1 * (double)b1 + t2 * (double)b2;
+            const double m = deep_makespan(load, sms, b1, t1, b2, t2, rest, &even);
+            if (best < 0 || m < 0.999 * best || (m < 1.001 * best && busy < best_busy)) {
                 best = m;
+                best_busy = busy;
+                *makespan = even;
                 *G1 = a;
                 *G2 = c;
             }
         }
         /* more second-part units than the search takes */
         if (best < 0 && nd2) {
-            best = t1 * (double)((b1 + sms - 1) / sms);
+            best = *makespan = t1 * (double)((b1 + sms - 1) / sms);
             *G1 = a;
             *G2 = fix2 ? fix2 : 4;
         }
     }
     free(load);
-    *makespan = best;
     return best < 0 ? -1 : 0;
+}
+
+/* The caller fixes nothing: the schedule model plans every part. */
+static int open_schedule(const pose_b200_sched_t *s)
+{
+    return !s || (!s->team_warps && !s->units_per_team && !s->max_teams && !s->lane_efficiency && !s->flags);
 }
 
 pose_b200_batch_t *pose_b200_batch_create(const pose_b200_request_t *reqs, size_t n,
@@ -777,14 +801,15 @@ no_split:
                      cudaStreamSynchronize(b->stream) != cudaSuccess))
         goto fail;
     {
-        int occ = 0, occ16 = 0; /* 8- and 16-warp CTAs per SM */
-        if (pb_dev_label_multi_occupancy(512, &occ16) != 0 || occ16 <= 0) occ16 = 1;
-        if (pb_dev_label_multi_occupancy(256, &occ) != 0 || occ <= 0) occ = 1;
+        int occ = 0; /* 8-warp CTAs per SM */
+        uint32_t alone_smem = 0;
+        if (pb_dev_label_multi_occupancy(256, &occ, &alone_smem) != 0 || occ <= 0) {
+            occ = 1;
+            alone_smem = 64 * 1024;
+        }
         uint64_t budget = pb_topo_scratch_budget(reqs[0].topo, sched ? sched->scratch_cap_bytes : 0);
         uint64_t deep_ctas = 0;
-        /* the caller fixes nothing: the schedule model plans every part */
-        const int open_sched = !sched || (!sched->team_warps && !sched->units_per_team && !sched->max_teams &&
-                                          !sched->lane_efficiency && !sched->flags);
+        const int open_sched = open_schedule(sched);
         double makespan = 0; /* estimated, in clocks, when the deep parts are planned by the model */
         /* deep part: 8-warp teams, units packed (G up to 4) until it holds
          * about half the SMs' team slots */
@@ -888,25 +913,41 @@ no_split:
             /* 16-warp teams; batches no longer than a third of the deep
              * parts' makespan (they fill the SMs those leave), or half of
              * what the requests need on all SMs */
-            double target = ukern == 1 ? 1e30 : makespan / 3.0;
+            double target = ukern == 1 ? 1e30 : makespan * PB_FILL_PART;
             if (target <= 0) target = shallow_makespan(ps, ns, 0) / 2.0;
             if (target <= 0) target = 1.0;
             if (ukern == 1) T = uT;
             if (pb_plan_requests(ps, ns, T, ukern == 1 ? uG : 32, 0.0, target, &pl[0]) != 0) goto fail;
         } else {
+            /* beside depth CTAs, which hold their SMs, the rest starts late:
+             * its batches are bounded as above, and chain-bounded packing
+             * fills them up to that.  (64 requests of 2^10..2^14 blocks,
+             * 4-warp teams: 90-157 ms unbounded, 56 bounded.) */
+            const double bound = makespan * PB_FILL_PART;
             if (pb_plan_choose(ps, ns, sched, &T, &eff) != 0) goto fail;
-            if (pb_plan_requests(ps, ns, T, gcap, eff, 0.0, &pl[0]) != 0) goto fail;
+            if (pb_plan_requests(ps, ns, T, gcap, eff, eff > 0 ? -bound : bound, &pl[0]) != 0) goto fail;
         }
         if (pl[0].nunits == 0 && !nd) { fprintf(stderr, "pose_b200_batch_create: no super-chunk to label\n"); goto fail; }
         if (pl[0].nunits && ukern != 3) {
             uint64_t cap;
-            if (open_sched) {
+            if (makespan > 0) {
+                /* beside deep parts 16 warps an SM: two 16-warp teams would
+                 * both start on the first SM that the deep parts leave and
+                 * end when the second one could have ended elsewhere (256
+                 * sessions, 5 and 8 copies a CTA: 1284 against 1181 ms) */
+                const uint32_t per_sm = 16 / T;
+                b->part[0].smem = per_sm == 1 ? alone_smem : alone_smem / per_sm - 2048;
+                cap = (uint64_t)pl[0].sms * per_sm;
+            } else if (open_sched) {
                 int o = 1;
-                if (pb_dev_label_multi_occupancy(32 * T, &o) != 0 || o <= 0) o = 1;
+                if (pb_dev_label_multi_occupancy(32 * T, &o, NULL) != 0 || o <= 0) o = 1;
                 cap = (uint64_t)pl[0].sms * (uint64_t)o;
             } else {
+                /* 24 warps an SM: with 32 the batches that run longest share
+                 * their SM with more others (256 requests in one launch of
+                 * 8-warp teams: 444 teams 1910 ms, 582 teams 2218-2409) */
                 const uint64_t taken = (uint64_t)b->part[1].grid + (nd2 ? b->part[2].grid : 0);
-                uint64_t slots = (uint64_t)pl[0].sms * occ;
+                uint64_t slots = (uint64_t)pl[0].sms * (occ < 3 ? occ : 3);
                 slots = slots > taken ? slots - taken : 1;
                 cap = slots * (256 / (32 * T));
             }

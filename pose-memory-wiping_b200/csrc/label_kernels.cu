@@ -608,33 +608,40 @@ extern "C" int pb_dev_label(const pb_label_params_t *params, uint32_t grid, uint
 }
 
 extern "C" int pb_dev_label_multi(const pb_multi_params_t *params, uint32_t grid, uint32_t cta_threads,
-                                  cudaStream_t stream)
+                                  uint32_t smem_bytes, cudaStream_t stream)
 {
     if (cta_threads != 32u * params->team_warps || cta_threads > PB_MULTI_CTA_THREADS) return -1; /* one team per CTA */
     cudaGetLastError(); /* report only this launch */
-    const uint32_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
+    uint32_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
+    if (smem_bytes > smem) smem = smem_bytes;
     if (params->table) pb::k_label_multi<true><<<grid, cta_threads, smem, stream>>>(*params);
     else pb::k_label_multi<false><<<grid, cta_threads, smem, stream>>>(*params);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-extern "C" int pb_dev_label_multi_occupancy(uint32_t cta_threads, int *blocks_per_sm)
+extern "C" int pb_dev_label_multi_occupancy(uint32_t cta_threads, int *blocks_per_sm, uint32_t *alone_smem)
 {
     /* a 512-thread CTA stages 48 KiB, more than the default limit with the
-     * static shared memory: one value for every caller (idempotent) */
+     * static shared memory, and one that holds its SM alone has the device's
+     * most: one value for every caller (idempotent) */
     const size_t smem = PB_PREF_BYTES_PER_THREAD * cta_threads;
-    const int bytes = (int)(PB_PREF_BYTES_PER_THREAD * PB_MULTI_CTA_THREADS);
-    int a = 0, b = 0;
-    if (cudaFuncSetAttribute(pb::k_label_multi<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(pb::k_label_multi<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, pb::k_label_multi<false>, (int)cta_threads, smem) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, pb::k_label_multi<true>, (int)cta_threads, smem) !=
-            cudaSuccess)
+    void (*const forms[2])(pb_multi_params_t) = {pb::k_label_multi<false>, pb::k_label_multi<true>};
+    int dev = 0, optin = 0, least = 1 << 30;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
         return -1;
-    *blocks_per_sm = a < b ? a : b;
+    for (int i = 0; i < 2; i++) {
+        cudaFuncAttributes fa;
+        int m = 0;
+        if (cudaFuncGetAttributes(&fa, forms[i]) != cudaSuccess ||
+            cudaFuncSetAttribute(forms[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 optin - (int)fa.sharedSizeBytes) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, forms[i], (int)cta_threads, smem) != cudaSuccess)
+            return -1;
+        if (m < least) least = m;
+        if (alone_smem) *alone_smem = (uint32_t)(optin - (int)fa.sharedSizeBytes);
+    }
+    *blocks_per_sm = least;
     return 0;
 }
 

@@ -576,7 +576,7 @@ static int admit_wave(pose_b200_server_t *s)
     p.table = pl.all_cv0;
     p.unit_req = (const uint32_t *)(T + o_ureq);
     p.req_done = wv->d_done;
-    if (ok) ok = pb_dev_label_multi(&p, g2, 32 * Tw, wv->stream) == 0;
+    if (ok) ok = pb_dev_label_multi(&p, g2, 32 * Tw, 0, wv->stream) == 0;
     /* the scratch range and the chunk seeds are zeroed before the wave
      * counts as done */
     if (ok) ok = cudaMemsetAsync(s->d_arena + off, 0, scratch, wv->stream) == cudaSuccess;
@@ -781,7 +781,7 @@ pose_b200_server_t *pose_b200_server_create(uint64_t scratch_bytes, uint32_t max
         const char *e5 = getenv("POSE_B200_SERVER_DEEP_EXCL");
         if (e5 && e5[0]) s->deep_excl = atoi(e5) != 0;
     }
-    if (pb_dev_label_multi_occupancy(512, &s->occ) != 0) s->occ = 1;
+    if (pb_dev_label_multi_occupancy(512, &s->occ, NULL) != 0) s->occ = 1;
     /* Launch tables and completion counters of every slot, allocated up
      * front: the dispatcher then makes no allocation while kernels run (a
      * cudaFree there waits for the whole device, and the submitters and
