@@ -464,8 +464,8 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
     };
     /* The level's start and width, this warp's part in it, and the ring stage
      * of the next level. */
-    uint32_t ls, w, st1, global;
-    bool busy; /* this warp has a quad with an item */
+    uint32_t ls = 0, w = 0, st1 = 0, global = 0;
+    bool busy = false; /* this warp has a quad with an item */
     Desc d;
     const auto enter = [&](uint32_t lv) {
         const uint32_t st = lv % 3;
@@ -477,8 +477,14 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
         global = __any_sync(0xFFFFFFFFu, d.global != 0);
     };
     const bool skips = warp >= PB_NARROW_WARPS;
-    if (CLUSTER && uniform(smem[Layout::hdr].y) > sw) cg::this_cluster().sync(); /* boundary 0 */
-    enter(0);
+    /* A warp reads the ring only at levels whose next boundary it passes: past
+     * one that it skips the producer may already have refilled the stage
+     * (level 0's in level 1).  A warp that skips level 0 knows its width from
+     * the level offsets, as it does further on. */
+    const uint32_t w0 = uniform(__ldg(tp.lstart + 1) - __ldg(tp.lstart));
+    if (CLUSTER && w0 > sw) cg::this_cluster().sync(); /* boundary 0 */
+    if (skips && !all_hands(w0)) w = w0;
+    else enter(0);
 #pragma unroll 1
     for (uint32_t l = 0; l < L;) {
         if (skips && !all_hands(w)) {
