@@ -100,7 +100,11 @@ struct pose_hbm_topo {
     uint64_t dev_bytes;
     pb_topo_view_t view;
     pb_topo_view2_t view2; /* pipelined records (d_recs2 != NULL) */
-    int occ_ws[2][PB_WS_MAX_UNITS + 1]; /* depth kernel CTAs per SM for 7 and 15 hashing warps, by units per CTA */
+    /* what planning asks of the device, all known once the topology is built,
+     * so that a plan only reads the topology (batches may be created on it
+     * from several threads): depth kernel CTAs per SM for 7 and 15 hashing
+     * warps, by units per CTA */
+    int occ_ws[2][PB_WS_MAX_UNITS + 1];
     /* levels wider than split_width (ascending), shared by a cluster's CTAs */
     uint32_t *d_split, nsplit, split_width;
     int occ_wsc[4];        /* clusters of 2, 4, 8, 16 CTAs (15 hashing warps) the device holds */
@@ -129,17 +133,7 @@ struct pose_hbm_topo {
 
 #define PB_SPLIT_WIDTH 480u  /* levels a depth-kernel cluster shares: wider than one pass of its hashing threads */
 
-static int ws_occupancy(pose_hbm_topo_t *t, uint32_t nc, uint32_t G)
-{
-    int *cached = &t->occ_ws[nc == 7 ? 0 : 1][G];
-    if (*cached < 0) {
-        int occ = 0;
-        if (pb_dev_label_ws_occupancy(32 * (nc + 1), pb_ws_smem_bytes(G, nc), &occ) != 0) occ = 0;
-        cudaGetLastError();
-        *cached = occ;
-    }
-    return *cached;
-}
+static int ws_occupancy(const pose_hbm_topo_t *t, uint32_t nc, uint32_t G) { return t->occ_ws[nc == 7 ? 0 : 1][G]; }
 
 /* Clocks the cluster form of the depth kernel adds to a level, and to one
  * that the cluster shares. */
@@ -147,18 +141,23 @@ static const double wsc_level = 60.0, wsc_split_sync = 1500.0;
 
 /* Clusters of C CTAs of the depth kernel (15 hashing warps) the device holds
  * at once (0 when C is not 2, 4, 8 or 16, or the kernel cannot run so). */
-static int wsc_clusters(pose_hbm_topo_t *t, uint32_t C)
+static int wsc_clusters(const pose_hbm_topo_t *t, uint32_t C)
 {
     const int i = C == 2 ? 0 : C == 4 ? 1 : C == 8 ? 2 : C == 16 ? 3 : -1;
-    if (i < 0 || !t->d_split) return 0;
-    if (t->occ_wsc[i] < 0) {
-        int n = 0;
-        const uint32_t smem = pb_ws_smem_bytes(1, 15);
-        if (smem > 227u * 1024u || pb_dev_label_wsc_max_clusters(C, 15, smem, &n) != 0) n = 0;
-        cudaGetLastError();
-        t->occ_wsc[i] = n;
-    }
-    return t->occ_wsc[i];
+    return i < 0 || !t->d_split ? 0 : t->occ_wsc[i];
+}
+
+/* Fill occ_ws and occ_wsc (0 where the device cannot run the form). */
+static void query_depth_occupancy(pose_hbm_topo_t *t)
+{
+    for (uint32_t i = 0; i < 2 && t->d_recs2; i++)
+        for (uint32_t G = 1, nc = i ? 15 : 7; G <= PB_WS_MAX_UNITS; G++)
+            if (pb_dev_label_ws_occupancy(32 * (nc + 1), pb_ws_smem_bytes(G, nc), &t->occ_ws[i][G]) != 0)
+                t->occ_ws[i][G] = 0;
+    for (uint32_t i = 0; i < 4 && t->d_split; i++)
+        if (pb_dev_label_wsc_max_clusters(2u << i, 15, pb_ws_smem_bytes(1, 15), &t->occ_wsc[i]) != 0)
+            t->occ_wsc[i] = 0;
+    cudaGetLastError();
 }
 
 static uint64_t passes_for(const pose_hbm_topo_t *t, uint32_t T, uint32_t G)
@@ -231,10 +230,9 @@ static double ws_cost(const pose_hbm_topo_t *t, uint32_t nc, uint32_t G, uint64_
  *     the rest of the batches spread over the SMs;
  *   - the depth kernel with G units per CTA, one CTA per SM, or with a
  *     cluster of CTAs per unit. */
-static int make_plan(const pose_hbm_topo_t *ct, uint64_t nunits, const pose_b200_sched_t *hint,
+static int make_plan(const pose_hbm_topo_t *t, uint64_t nunits, const pose_b200_sched_t *hint,
                      uint64_t budget, plan_t *best)
 {
-    pose_hbm_topo_t *t = (pose_hbm_topo_t *)ct; /* occupancy cache */
     const int cv0 = t->d_cv0 != NULL;
     const int want = hint ? (int)hint->kernel : 0;
     memset(best, 0, sizeof(*best));
@@ -560,8 +558,6 @@ static pose_hbm_topo_t *pose_b200_topo_build_impl(uint32_t chunk_blocks, int wit
         t->view2.S = h.S; t->view2.L = h.L; t->view2.half_w = h.half_w;
         t->view2.retained = h.retained; t->view2.csm = h.csm; t->view2.gpool = h.gpool2;
         memcpy(t->view2.desc, t->view.desc, sizeof(t->view2.desc));
-        memset(t->occ_ws, 0xFF, sizeof(t->occ_ws));
-        memset(t->occ_wsc, 0xFF, sizeof(t->occ_wsc));
         if (t->d_recs2) {
             /* the levels a cluster of the depth kernel shares: wider than
              * split_width (POSE_B200_SPLIT_WIDTH overrides the default, the
@@ -584,6 +580,7 @@ static pose_hbm_topo_t *pose_b200_topo_build_impl(uint32_t chunk_blocks, int wit
                 t->dev_bytes += (uint64_t)n * 4;
             }
         }
+        query_depth_occupancy(t);
     }
     pb_topo_host_free(&h);
     return t;

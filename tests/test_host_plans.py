@@ -1,0 +1,93 @@
+"""The host side's plans on a CUDA runtime that does nothing (fake_cuda.c): what
+is allocated and what is launched, with which sizes."""
+from __future__ import annotations
+
+import ctypes as C
+import importlib.util
+import os
+import subprocess
+import time
+
+import pytest
+
+from conftest import PKG_DIR, ROOT
+
+CSRC = os.path.join(PKG_DIR, "csrc")
+CUDA_INC = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+LABEL, MULTI, DEPTH, CLUSTER = 1, 2, 3, 4
+
+
+class Launch(C.Structure):
+    _fields_ = [("kind", C.c_uint32), ("grid", C.c_uint32), ("warps", C.c_uint32), ("units_per", C.c_uint32),
+                ("nunits", C.c_uint32), ("nbatches", C.c_uint32), ("smem", C.c_uint32), ("scratch", C.c_uint64)]
+
+
+class Fake:
+    """The package on the fake library."""
+
+    def __init__(self, path):
+        spec = importlib.util.spec_from_file_location("pose_b200_fake", os.path.join(PKG_DIR, "__init__.py"),
+                                                      submodule_search_locations=[PKG_DIR])
+        self.pkg = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(self.pkg)
+        self.pkg.LIB_PATH = path
+        self.lib = self.pkg.load()
+        self.lib.fake_set_free.argtypes = [C.c_uint64]
+        self.lib.fake_live.restype = C.c_uint64
+        self.topos = {}
+
+    def topo(self, cb, **kw):
+        key = (cb, tuple(kw.items()))
+        if key not in self.topos:
+            self.topos[key] = self.pkg.Topology(cb, **kw)
+        return self.topos[key]
+
+    def launches(self):
+        a = (Launch * 4096)()
+        n = self.lib.fake_launches(a, 4096)
+        return [a[i] for i in range(n)]
+
+    def copy_bytes(self, topo):
+        """Scratch of one chunk copy on the lockstep kernel and on the depth kernel."""
+        out = []
+        for kernel in (1, 3):
+            s = self.pkg.Sched()
+            s.kernel, s.units_per_team, s.max_teams = kernel, 1, 1
+            s.cluster_ctas = 1 if kernel == 3 else 0
+            out.append(topo.plan(1, s).scratch_cap_bytes)
+        return out
+
+    def sched(self, **kw):
+        s = self.pkg.Sched()
+        for k, v in kw.items():
+            setattr(s, k, v)
+        return s
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    if not os.path.exists(os.path.join(CUDA_INC, "cuda_runtime_api.h")):
+        pytest.skip("no CUDA headers")
+    so = str(tmp_path_factory.mktemp("fake") / "libpose_fake.so")
+    src = [os.path.join(CSRC, f) for f in ("label_api.c", "label_batch.c", "label_server.c", "label_stream.c",
+                                           "label_verify.c", "topology.c", "b3_host.c")]
+    src.append(os.path.join(ROOT, "tests", "fake_cuda.c"))
+    subprocess.run(["gcc", "-O2", "-std=c11", "-fPIC", "-shared", "-D_GNU_SOURCE", "-I" + CUDA_INC,
+                    "-I" + os.path.join(ROOT, "include"), "-I" + CSRC, "-o", so, *src, "-lpthread", "-lm", "-ldl"],
+                   check=True)
+    return Fake(so)
+
+
+def requests(topo, n, chunks=1, first=0):
+    sb = topo.super_bytes
+    return [(topo, b"k" * 32, 1 << 40, chunks * sb, (first + i) * topo.chunk_blocks * chunks) for i in range(n)]
+
+
+def test_planning_only_reads_the_topology(fake):
+    topo = fake.topo(2048)
+    fake.lib.fake_reset()
+    topo.plan(16)
+    topo.plan(16, fake.sched(kernel=3, team_warps=7))
+    with fake.pkg.Batch(requests(topo, 16)):
+        pass
+    assert fake.lib.fake_occupancy_queries() == 0
