@@ -1279,7 +1279,7 @@ double pb_topo_depth_clocks(const pose_hbm_topo_t *t, uint32_t G)
 }
 
 int pb_topo_auto_plan(const pose_hbm_topo_t *t, uint64_t nunits, uint64_t budget, uint32_t *kernel, uint32_t *T,
-                      uint32_t *G)
+                      uint32_t *G, uint32_t *teams)
 {
     plan_t p;
     pose_b200_sched_t h;
@@ -1292,6 +1292,7 @@ int pb_topo_auto_plan(const pose_hbm_topo_t *t, uint64_t nunits, uint64_t budget
     *kernel = p.kernel;
     *T = p.T;
     *G = p.G;
+    *teams = p.teams;
     return 0;
 }
 

@@ -444,11 +444,12 @@ static int part_setup(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_table
     return 0;
 }
 
-/* The deep part on the multi-unit depth kernel: every unit of pl (one
- * topology, records v2), G (1 to 8) units per CTA, at most one CTA per SM
- * (`sms` CTAs), 15 hashing warps.  Returns 0, or -1 (message on stderr). */
+/* A part on the depth kernel: every unit of pl (one topology, records v2), G
+ * (1 to 8) units per CTA, at most `ctas` CTAs, 15 hashing warps.  The caller
+ * bounds ctas by the SMs and the scratch budget.  Returns 0, or -1 (message
+ * on stderr). */
 static int part_setup_wsg(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_tables_t *pl,
-                          const pb_topo_view2_t *v2, uint32_t G, uint32_t sms, uint32_t smem)
+                          const pb_topo_view2_t *v2, uint32_t G, uint32_t ctas, uint32_t smem)
 {
     const uint32_t NC = 15;
     q->kind = 1;
@@ -462,7 +463,7 @@ static int part_setup_wsg(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_t
     q->Gmax = G;
     q->cv0 = 1;
     q->nbatches = (pl->nunits + G - 1) / G;
-    q->grid = (uint32_t)(q->nbatches < sms ? q->nbatches : sms);
+    q->grid = (uint32_t)(q->nbatches < ctas ? q->nbatches : ctas);
     q->teams = q->grid;
     q->cta_threads = 32 * (NC + 1);
     q->smem = smem;
@@ -891,9 +892,9 @@ no_split:
         uint32_t T = 16;
         double eff = 0.0;
         const pose_hbm_topo_t *only = NULL;
-        uint32_t ukern = 0, uT = 0, uG = 0;
+        uint32_t ukern = 0, uT = 0, uG = 0, uteams = 0;
         if (open_sched && !nd && (only = one_topology(ps, ns)) != NULL &&
-            pb_topo_auto_plan(only, request_units(ps, ns), budget, &ukern, &uT, &uG) != 0)
+            pb_topo_auto_plan(only, request_units(ps, ns), budget, &ukern, &uT, &uG, &uteams) != 0)
             ukern = 0;
         pb_topo_view2_t uv2;
         uint32_t umax = 0;
@@ -904,11 +905,9 @@ no_split:
         }
         if (ukern == 3) {
             /* one topology, few units: the depth kernel, as a single call */
-            pb_topo_internal_t x;
-            if (pb_topo_internal(only, &x) != 0 || pb_plan_requests(ps, ns, 8, 1, 0.9999, 0.0, &pl[0]) != 0) goto fail;
+            if (pb_plan_requests(ps, ns, 8, 1, 0.9999, 0.0, &pl[0]) != 0) goto fail;
             T = 15;
-            if (part_setup_wsg(b, &b->part[0], &pl[0], &uv2, uG, (uint32_t)x.sms, pb_ws_smem_bytes(uG, 15)) != 0)
-                goto fail;
+            if (part_setup_wsg(b, &b->part[0], &pl[0], &uv2, uG, uteams, pb_ws_smem_bytes(uG, 15)) != 0) goto fail;
         } else if (open_sched) {
             /* 16-warp teams; batches no longer than a third of the deep
              * parts' makespan (they fill the SMs those leave), or half of

@@ -46,9 +46,10 @@ int pb_topo_view2(const pose_hbm_topo_t *t, pb_topo_view2_t *out);
  * (0 for a topology without the records). */
 double pb_topo_lockstep_clocks(const pose_hbm_topo_t *t, uint32_t T, uint32_t G);
 double pb_topo_depth_clocks(const pose_hbm_topo_t *t, uint32_t G);
-/* The automatic schedule of a call of nunits units: kernel 1 (T, G) or 3 (G). */
+/* The automatic schedule of a call of nunits units: kernel 1 (T, G) or 3 (G),
+ * and the teams (CTAs) whose scratch fits `budget`. */
 int pb_topo_auto_plan(const pose_hbm_topo_t *t, uint64_t nunits, uint64_t budget, uint32_t *kernel, uint32_t *T,
-                      uint32_t *G);
+                      uint32_t *G, uint32_t *teams);
 
 /* Passes a team of T warps makes over all levels running G units in lockstep. */
 uint64_t pb_topo_passes(const pose_hbm_topo_t *t, uint32_t T, uint32_t G);

@@ -91,3 +91,34 @@ def test_planning_only_reads_the_topology(fake):
     with fake.pkg.Batch(requests(topo, 16)):
         pass
     assert fake.lib.fake_occupancy_queries() == 0
+
+
+# a cap on the scratch of a batch of one topology: plans on the depth kernel
+# (few copies) and on the lockstep kernel (many), and the challenge call
+@pytest.mark.parametrize("cb,n,kind,copies", [(2048, 16, DEPTH, 3), (2048, 700, None, 10), (64, 4096, MULTI, 2820)])
+def test_one_topology_batch_keeps_its_cap(fake, cb, n, kind, copies):
+    topo = fake.topo(cb)
+    cap = copies * max(fake.copy_bytes(topo))
+    fake.lib.fake_reset()
+    before = fake.lib.fake_live()
+    with fake.pkg.Batch(requests(topo, n), fake.sched(scratch_cap_bytes=cap)) as b:
+        rc, st = b.run()
+        assert rc == 0 and st["scratch_bytes"] <= cap
+        ran = fake.launches()
+        assert kind is None or [x.kind for x in ran] == [kind]
+        assert 0 < sum(x.scratch for x in ran) <= cap
+    assert fake.lib.fake_live() == before
+    rc, _, st = topo.challenge_blocks(b"k" * 32, [i * cb for i in range(n)], fake.sched(scratch_cap_bytes=cap))
+    assert rc == 0 and 0 < st["scratch_bytes"] <= cap
+
+
+def test_one_topology_batch_fits_free_memory(fake):
+    topo = fake.topo(2048)
+    copy = fake.copy_bytes(topo)[1]
+    fake.lib.fake_set_free(fake.lib.fake_live() + (2 << 30) + 5 * copy)
+    try:
+        with fake.pkg.Batch(requests(topo, 16)) as b:
+            rc, st = b.run()
+            assert rc == 0 and st["scratch_bytes"] <= 5 * copy
+    finally:
+        fake.lib.fake_set_free(170 << 30)
