@@ -52,8 +52,9 @@ int pb_plan_requests(const pb_req_t *reqs, size_t n, uint32_t T, uint32_t gcap, 
 double pb_plan_makespan(const pb_plan_tables_t *p, uint32_t T, uint64_t R);
 void pb_plan_free(pb_plan_tables_t *p);
 /* Plan n requests for teams of T warps that fill `sms` SMs: batches no longer
- * than what the requests need there, or the longest single unit's. */
-int pb_plan_fill(const pb_req_t *reqs, size_t n, uint32_t sms, uint32_t T, pb_plan_tables_t *out);
+ * than what the requests need there, or the longest single unit's, and a
+ * team's scratch no larger than `room` (unless one unit's is). */
+int pb_plan_fill(const pb_req_t *reqs, size_t n, uint32_t sms, uint32_t T, uint64_t room, pb_plan_tables_t *out);
 /* A schedule candidate: team size, packing rule (eff_min of
  * pb_plan_requests) and its estimated makespan. */
 typedef struct {

@@ -605,10 +605,23 @@ static double shallow_makespan(const pb_req_t *pr, size_t n, uint32_t sms)
     return longest > work / sms ? longest : work / sms;
 }
 
-int pb_plan_fill(const pb_req_t *reqs, size_t n, uint32_t sms, uint32_t T, pb_plan_tables_t *out)
+/* pb_plan_requests with at most gcap units a team, fewer where a team's
+ * scratch would not fit `room` (one unit at the least). */
+static int plan_within(const pb_req_t *pr, size_t n, uint32_t T, uint32_t gcap, double eff, double target,
+                       uint64_t room, pb_plan_tables_t *out)
+{
+    while (pb_plan_requests(pr, n, T, gcap, eff, target, out) == 0) {
+        if (out->team_scratch <= room || gcap == 1) return 0;
+        pb_plan_free(out);
+        gcap /= 2;
+    }
+    return -1;
+}
+
+int pb_plan_fill(const pb_req_t *reqs, size_t n, uint32_t sms, uint32_t T, uint64_t room, pb_plan_tables_t *out)
 {
     const double target = shallow_makespan(reqs, n, sms) / 2.0;
-    return pb_plan_requests(reqs, n, T, 32, 0.0, target > 0 ? target : 1.0, out);
+    return plan_within(reqs, n, T, 32, 0.0, target > 0 ? target : 1.0, room, out);
 }
 
 /* Batches of the other requests, beside deep parts, take at most this part of
@@ -916,7 +929,7 @@ no_split:
             if (target <= 0) target = shallow_makespan(ps, ns, 0) / 2.0;
             if (target <= 0) target = 1.0;
             if (ukern == 1) T = uT;
-            if (pb_plan_requests(ps, ns, T, ukern == 1 ? uG : 32, 0.0, target, &pl[0]) != 0) goto fail;
+            if (plan_within(ps, ns, T, ukern == 1 ? uG : 32, 0.0, target, budget, &pl[0]) != 0) goto fail;
         } else {
             /* beside depth CTAs, which hold their SMs, the rest starts late:
              * its batches are bounded as above, and chain-bounded packing
@@ -924,7 +937,9 @@ no_split:
              * 4-warp teams: 90-157 ms unbounded, 56 bounded.) */
             const double bound = makespan * PB_FILL_PART;
             if (pb_plan_choose(ps, ns, sched, &T, &eff) != 0) goto fail;
-            if (pb_plan_requests(ps, ns, T, gcap, eff, eff > 0 ? -bound : bound, &pl[0]) != 0) goto fail;
+            /* a caller's own units per team are kept, and refused when they do not fit */
+            const uint64_t room = sched && sched->units_per_team ? UINT64_MAX : budget;
+            if (plan_within(ps, ns, T, gcap, eff, eff > 0 ? -bound : bound, room, &pl[0]) != 0) goto fail;
         }
         if (pl[0].nunits == 0 && !nd) { fprintf(stderr, "pose_b200_batch_create: no super-chunk to label\n"); goto fail; }
         if (pl[0].nunits && ukern != 3) {

@@ -487,7 +487,7 @@ static int admit_wave(pose_b200_server_t *s)
     }
     pb_plan_tables_t pl;
     const uint32_t Tw = 16;
-    if (pb_plan_fill(pr, n, s->all_sms - s->deep_ctas, Tw, &pl) != 0) {
+    if (pb_plan_fill(pr, n, s->all_sms - s->deep_ctas, Tw, s->arena_bytes, &pl) != 0) {
         free(pr);
         for (size_t i = 0; i < n; i++) { s->reqs[wv->reqs[i]].state = 3; s->reqs[wv->reqs[i]].t_done = now_ms(); }
         pthread_cond_broadcast(&s->cv);

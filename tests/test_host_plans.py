@@ -122,3 +122,43 @@ def test_one_topology_batch_fits_free_memory(fake):
             assert rc == 0 and st["scratch_bytes"] <= 5 * copy
     finally:
         fake.lib.fake_set_free(170 << 30)
+
+
+# a cap below the scratch of the teams that the requests would otherwise be
+# packed into: smaller teams
+@pytest.mark.parametrize("copies", [1, 5, 40])
+def test_mixed_batch_packs_within_its_cap(fake, copies):
+    a, b = fake.topo(300), fake.topo(512)  # equally deep: one launch
+    cap = copies * max(fake.copy_bytes(t)[0] for t in (a, b))
+    with fake.pkg.Batch(requests(a, 2000) + requests(b, 2000), fake.sched(scratch_cap_bytes=cap)) as batch:
+        rc, st = batch.run()
+    assert rc == 0 and 0 < st["scratch_bytes"] <= cap
+
+
+def wait_all(fake, server, tickets, seconds=20):
+    """All tickets done; a server that holds some back for good is left alone
+    (closing it would wait for them too)."""
+    end = time.time() + seconds
+    while time.time() < end and any(server.query(t) == 0 for t in tickets):
+        time.sleep(0.01)
+    left = [t for t in tickets if server.query(t) != 1]
+    if left:
+        server.handle = None
+    return left
+
+
+@pytest.mark.parametrize("copies", [1, 6])
+def test_server_packs_within_its_arena(fake, copies):
+    topo = fake.topo(512)
+    arena = max(256, copies * fake.copy_bytes(topo)[0])
+    server = fake.pkg.Server(scratch_bytes=arena)
+    sid = server.session(b"k" * 32)
+    # the first request holds the arena until the others are all pending
+    fake.lib.fake_hold_events()
+    tickets = [server.submit(topo, sid, 1 << 40, 4 * topo.super_bytes, 0)]
+    while server.stats()["waves"] == 0:
+        time.sleep(0.01)
+    tickets += [server.submit(topo, sid, 1 << 40, 4 * topo.super_bytes, 0) for _ in range(600)]
+    fake.lib.fake_finish_events()
+    assert not wait_all(fake, server, tickets)
+    server.close()
