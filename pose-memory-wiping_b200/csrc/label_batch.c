@@ -29,6 +29,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 #include <cuda_runtime_api.h>
+#include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -444,6 +445,9 @@ static int part_setup(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_table
     return 0;
 }
 
+/* Scratch of one chunk copy on the depth kernel. */
+static uint64_t depth_copy_bytes(const pb_topo_view2_t *v) { return (uint64_t)(v->gpool ? v->gpool : 1) * 32; }
+
 /* A part on the depth kernel: every unit of pl (one topology, records v2), G
  * (1 to 8) units per CTA, at most `ctas` CTAs, 15 hashing warps.  The caller
  * bounds ctas by the SMs and the scratch budget.  Returns 0, or -1 (message
@@ -467,7 +471,7 @@ static int part_setup_wsg(pose_b200_batch_t *b, batch_part_t *q, const pb_plan_t
     q->teams = q->grid;
     q->cta_threads = 32 * (NC + 1);
     q->smem = smem;
-    q->team_scratch = (uint64_t)G * v2->gpool * 32;
+    q->team_scratch = (uint64_t)G * depth_copy_bytes(v2);
     q->scratch_bytes = (uint64_t)q->grid * q->team_scratch;
     uint32_t max_smem = 0;
     if (pb_dev_label_ws_prepare(&max_smem) != 0 || pb_ws_smem_bytes(G, NC) > max_smem) {
@@ -628,9 +632,30 @@ int pb_plan_fill(const pb_req_t *reqs, size_t n, uint32_t sms, uint32_t T, uint6
  * the whole's estimate. */
 #define PB_FILL_PART (1.0 / 3.0)
 
-/* Add n jobs of t clocks to the SMs' loads, each on the one free first. */
+/* Add n jobs of t clocks to the SMs' loads, each on the one free first: job
+ * k of an SM starts at its load + k t, and the n jobs take the n earliest
+ * starts.  Of many jobs all but a few are placed at once, those that start
+ * before a time that fewer than n do. */
 static void place_jobs(double *load, uint32_t sms, uint64_t n, double t)
 {
+    if (n > 4ull * sms && t > 0) {
+        double lo = 0, hi = t;
+        for (uint32_t i = 0; i < sms; i++)
+            if (load[i] + t * ((double)n / sms + 1.0) > hi) hi = load[i] + t * ((double)n / sms + 1.0);
+        for (int k = 0; k < 40; k++) {
+            const double mid = 0.5 * (lo + hi);
+            double starts = 0;
+            for (uint32_t i = 0; i < sms; i++) starts += load[i] < mid ? ceil((mid - load[i]) / t) : 0.0;
+            if (starts <= (double)n) lo = mid;
+            else hi = mid;
+        }
+        for (uint32_t i = 0; i < sms; i++) {
+            uint64_t k = load[i] < lo ? (uint64_t)ceil((lo - load[i]) / t) : 0;
+            if (k > n) k = n;
+            load[i] += t * (double)k;
+            n -= k;
+        }
+    }
     for (uint64_t j = 0; j < n; j++) {
         uint32_t m = 0;
         for (uint32_t i = 1; i < sms; i++)
@@ -647,17 +672,24 @@ static double most_loaded(const double *load, uint32_t sms)
     return m;
 }
 
-/* Clocks until b1 jobs of t1, then b2 of t2 (each on the SM that is free
- * first), and `rest` clocks of other work behind them are done.  That work
- * comes in batches of PB_FILL_PART of an even fill's makespan, which is
- * *even: a choice that leaves the SMs to the deep parts until the end pays
- * for the last batches (256 sessions of 2^12..2^17 blocks, 4 and 5 copies a
- * CTA on 103 and 45 SMs: 1602 ms, 5 and 5 on 82 and 66: 1203). */
-static double deep_makespan(double *load, uint32_t sms, uint64_t b1, double t1, uint64_t b2, double t2, double rest,
-                            double *even)
+/* One deep part: G copies per CTA on `ctas` CTAs (0: no such part). */
+typedef struct {
+    uint32_t G, ctas;
+} deep_part_t;
+
+/* Clocks until b1 jobs of t1 on c1 CTAs, then b2 of t2 on c2 CTAs (each on the
+ * SM that is free first), and `rest` clocks of other work behind them are
+ * done.  That work comes in batches of PB_FILL_PART of an even fill's
+ * makespan, which is *even: a choice that leaves the SMs to the deep parts
+ * until the end pays for the last batches (256 sessions of 2^12..2^17 blocks,
+ * 4 and 5 copies a CTA on 103 and 45 SMs: 1602 ms, 5 and 5 on 82 and 66:
+ * 1203). */
+static double deep_makespan(double *load, uint32_t sms, uint32_t c1, uint64_t b1, double t1, uint32_t c2, uint64_t b2,
+                            double t2, double rest, double *even)
 {
-    for (uint32_t i = 0; i < sms; i++) load[i] = t1 * (double)(b1 / sms + (i < b1 % sms));
-    place_jobs(load, sms, b2, t2);
+    for (uint32_t i = 0; i < sms; i++) load[i] = i < c1 ? t1 * (double)(b1 / c1 + (i < b1 % c1)) : 0.0;
+    /* the c2 least loaded SMs are the last ones */
+    if (c2) place_jobs(load + (sms - c2), c2, b2, t2);
     double sum = rest;
     for (uint32_t i = 0; i < sms; i++) sum += load[i];
     *even = most_loaded(load, sms);
@@ -666,55 +698,79 @@ static double deep_makespan(double *load, uint32_t sms, uint64_t b1, double t1, 
     return most_loaded(load, sms);
 }
 
+/* The most scratch that one chunk copy of n requests takes on the lockstep
+ * kernel. */
+static uint64_t lockstep_copy_bytes(const pb_req_t *pr, size_t n)
+{
+    uint64_t most = 0;
+    for (size_t i = 0; i < n; i++) {
+        pb_topo_internal_t x;
+        if (pb_topo_internal(pr[i].topo, &x) != 0 || pr[i].len < x.super_bytes) continue;
+        if ((uint64_t)x.view.pool * 32 > most) most = (uint64_t)x.view.pool * 32;
+    }
+    return most;
+}
+
+/* CTAs of a depth part: one per batch and SM, as many as `room` holds. */
+static uint32_t depth_ctas(uint64_t batches, uint32_t sms, uint64_t room, uint64_t cta_bytes)
+{
+    uint64_t c = room / cta_bytes;
+    if (c > batches) c = batches;
+    return (uint32_t)(c < sms ? c : sms);
+}
+
 /* Copies per CTA of the two deep parts (pd: nd requests of one topology; pd2:
  * nd2 of another, or none) that the schedule model finishes first, with the
  * other requests ps filled in behind them; fix1, fix2 (nonzero) fix them.
+ * Both parts and one copy of the others fit the scratch budget; a part that
+ * memory limits has fewer CTAs, which loop over its batches.
  * Among choices that finish together the one with the least work on the SMs.
  * On the 256-session workload that is 5 and 8: 82 CTAs of the 2^17 sessions
- * and 49 of the 2^16 ones beside them.  Returns 0, or -1
- * when no choice fits the shared memory and the scratch budget. */
+ * and 49 of the 2^16 ones beside them.  Where no choice has room for both
+ * parts the second is left to the others.  Returns 0, or -1 when no choice
+ * fits the shared memory and the budget. */
 static int plan_deep(const pb_req_t *pd, size_t nd, const pb_req_t *pd2, size_t nd2, const pb_req_t *ps, size_t ns,
-                     uint32_t sms, uint64_t budget, uint32_t fix1, uint32_t fix2, uint32_t *G1, uint32_t *G2,
+                     uint32_t sms, uint64_t budget, uint32_t fix1, uint32_t fix2, deep_part_t part[2],
                      double *makespan)
 {
     pb_topo_view2_t v1, v2;
     uint32_t max_smem = 0, n_sms;
     double longest;
     if (pb_topo_view2(pd[0].topo, &v1) != 0 || pb_dev_label_ws_prepare(&max_smem) != 0) return -1;
-    if (nd2 && pb_topo_view2(pd2[0].topo, &v2) != 0) nd2 = 0;
-    const uint64_t u1 = request_units(pd, nd), u2 = nd2 ? request_units(pd2, nd2) : 0;
-    const double rest = shallow_work(ps, ns, &longest, &n_sms);
     double *load = (double *)malloc(sms * sizeof(*load));
     if (!load) return -1;
+    const uint64_t u1 = request_units(pd, nd), u2 = nd2 ? request_units(pd2, nd2) : 0;
+    double rest = shallow_work(ps, ns, &longest, &n_sms);
+    uint64_t keep = lockstep_copy_bytes(ps, ns);
     double best = -1, best_busy = 0;
-    for (uint32_t a = 1; a <= PB_WS_MAX_UNITS; a++) {
-        const uint64_t b1 = (u1 + a - 1) / a, s1 = (b1 < sms ? b1 : sms) * (uint64_t)v1.gpool * 32 * a;
-        if ((fix1 && a != fix1) || pb_ws_smem_bytes(a, 15) > max_smem || s1 > budget) continue;
-        const double t1 = pb_topo_depth_clocks(pd[0].topo, a);
-        for (uint32_t c = nd2 ? 1 : 0; c <= (nd2 ? PB_WS_MAX_UNITS : 0); c++) {
-            uint64_t b2 = 0;
-            double t2 = 0;
-            if (c) {
-                b2 = (u2 + c - 1) / c;
-                if ((fix2 && c != fix2) || pb_ws_smem_bytes(c, 15) > max_smem) continue;
-                t2 = pb_topo_depth_clocks(pd2[0].topo, c);
-            }
-            if (b2 > 16ull * sms) continue;
-            double even, busy = t1 * (double)b1 + t2 * (double)b2;
-            const double m = deep_makespan(load, sms, b1, t1, b2, t2, rest, &even);
-            if (best < 0 || m < 0.999 * best || (m < 1.001 * best && busy < best_busy)) {
-                best = m;
-                best_busy = busy;
-                *makespan = even;
-                *G1 = a;
-                *G2 = c;
-            }
+    for (int second = nd2 && pb_topo_view2(pd2[0].topo, &v2) == 0; second >= 0 && best < 0; second--) {
+        if (!second && nd2) { /* with the others */
+            const uint64_t copy = lockstep_copy_bytes(pd2, nd2);
+            rest += shallow_work(pd2, nd2, &longest, &n_sms);
+            if (copy > keep) keep = copy;
         }
-        /* more second-part units than the search takes */
-        if (best < 0 && nd2) {
-            best = *makespan = t1 * (double)((b1 + sms - 1) / sms);
-            *G1 = a;
-            *G2 = fix2 ? fix2 : 4;
+        const uint64_t room = budget > keep ? budget - keep : 0;
+        for (uint32_t a = 1; a <= PB_WS_MAX_UNITS; a++) {
+            if ((fix1 && a != fix1) || pb_ws_smem_bytes(a, 15) > max_smem) continue;
+            const uint64_t b1 = (u1 + a - 1) / a, m1 = depth_copy_bytes(&v1) * a;
+            const double t1 = pb_topo_depth_clocks(pd[0].topo, a);
+            for (uint32_t c = second ? 1 : 0; c <= (second ? PB_WS_MAX_UNITS : 0); c++) {
+                if (c && ((fix2 && c != fix2) || pb_ws_smem_bytes(c, 15) > max_smem)) continue;
+                const uint64_t b2 = c ? (u2 + c - 1) / c : 0, m2 = c ? depth_copy_bytes(&v2) * c : 0;
+                const double t2 = c ? pb_topo_depth_clocks(pd2[0].topo, c) : 0;
+                const uint32_t c1 = depth_ctas(b1, sms, room > m2 ? room - m2 : 0, m1);
+                const uint32_t c2 = c1 && c ? depth_ctas(b2, sms, room - c1 * m1, m2) : 0;
+                if (!c1 || (c && !c2)) continue;
+                double even, busy = t1 * (double)b1 + t2 * (double)b2;
+                const double m = deep_makespan(load, sms, c1, b1, t1, c2, b2, t2, rest, &even);
+                if (best < 0 || m < 0.999 * best || (m < 1.001 * best && busy < best_busy)) {
+                    best = m;
+                    best_busy = busy;
+                    *makespan = even;
+                    part[0] = (deep_part_t){a, c1};
+                    part[1] = (deep_part_t){c, c2};
+                }
+            }
         }
     }
     free(load);
@@ -845,56 +901,42 @@ no_split:
             const char *eu = getenv("POSE_B200_DEEP2_UNITS"); /* the same for the second deep part */
             const uint32_t fix1 = eg && eg[0] >= '1' && eg[0] <= '8' && !eg[1] ? (uint32_t)(eg[0] - '0') : 0;
             const uint32_t fix2 = eu && eu[0] >= '1' && eu[0] <= '8' && !eu[1] ? (uint32_t)(eu[0] - '0') : 0;
-            uint32_t G = 0, G2 = 0;
+            deep_part_t dp[2] = {{0, 0}, {0, 0}};
             int wsg = !(ek && ek[0] == '0') && one_topo && pb_topo_view2(pd[0].topo, &v2) == 0;
             if (wsg) {
                 /* copies per CTA of both parts */
-                wsg = plan_deep(pd, nd, pd2, nd2, ps, ns, sms, budget, fix1, fix2, &G, &G2, &makespan) == 0;
+                wsg = plan_deep(pd, nd, pd2, nd2, ps, ns, sms, budget, fix1, fix2, dp, &makespan) == 0;
                 cudaGetLastError();
             }
             if (wsg) {
-                const uint32_t smem = pb_ws_smem_bytes(G, 15);
                 if (pb_plan_requests(pd, nd, 8, 1, 0.9999, 0.0, &pl[1]) != 0 || pl[1].nunits == 0) goto fail;
-                if (part_setup_wsg(b, &b->part[1], &pl[1], &v2, G, sms, smem) != 0) goto fail;
+                if (part_setup_wsg(b, &b->part[1], &pl[1], &v2, dp[0].G, dp[0].ctas, pb_ws_smem_bytes(dp[0].G, 15)) !=
+                    0)
+                    goto fail;
                 /* the next-deepest topology's requests: a third launch of the
                  * depth kernel, on the SMs the first leaves and then on those
                  * it is done with */
-                if (nd2) {
+                if (dp[1].ctas) {
                     pb_topo_view2_t v2b;
-                    uint64_t du2 = 0;
-                    for (size_t i = 0; i < nd2; i++) {
-                        pb_topo_internal_t x;
-                        if (pb_topo_internal(pd2[i].topo, &x) != 0) goto fail;
-                        du2 += (uint64_t)(pd2[i].len / x.super_bytes) * x.copies;
-                    }
-                    uint32_t max_smem2 = 0;
-                    int ok2 = G2 > 0 && pb_topo_view2(pd2[0].topo, &v2b) == 0 &&
-                              pb_dev_label_ws_prepare(&max_smem2) == 0 &&
-                              pb_ws_smem_bytes(G2, 15) <= max_smem2;
-                    cudaGetLastError();
-                    if (ok2) {
-                        const uint64_t g2 = (du2 + G2 - 1) / G2 < sms ? (du2 + G2 - 1) / G2 : sms;
-                        ok2 = b->part[1].scratch_bytes + g2 * ((uint64_t)v2b.gpool * 32 * G2) <= budget;
-                    }
-                    if (ok2) {
-                        if (pb_plan_requests(pd2, nd2, 8, 1, 0.9999, 0.0, &pl[2]) != 0 || pl[2].nunits == 0) goto fail;
-                        if (part_setup_wsg(b, &b->part[2], &pl[2], &v2b, G2, sms, pb_ws_smem_bytes(G2, 15)) !=
-                            0)
-                            goto fail;
-                    } else {
-                        for (size_t i = 0; i < nd2; i++) ps[ns++] = pd2[i];
-                        nd2 = 0;
-                    }
+                    if (pb_topo_view2(pd2[0].topo, &v2b) != 0 ||
+                        pb_plan_requests(pd2, nd2, 8, 1, 0.9999, 0.0, &pl[2]) != 0 || pl[2].nunits == 0)
+                        goto fail;
+                    if (part_setup_wsg(b, &b->part[2], &pl[2], &v2b, dp[1].G, dp[1].ctas,
+                                       pb_ws_smem_bytes(dp[1].G, 15)) != 0)
+                        goto fail;
                 }
             } else {
                 uint32_t g = 1;
                 while (g < 4 && 2 * (dunits + g - 1) / g > (uint64_t)sms * occ) g *= 2;
-                if (pb_plan_requests(pd, nd, 8, g, 0.9999, 0.0, &pl[1]) != 0 || pl[1].nunits == 0) goto fail;
+                /* one copy of the others has to fit beside it */
+                const uint64_t k1 = lockstep_copy_bytes(ps, ns), k2 = lockstep_copy_bytes(pd2, nd2);
+                const uint64_t keep = k1 > k2 ? k1 : k2, room = budget > keep ? budget - keep : 0;
+                if (plan_within(pd, nd, 8, g, 0.9999, 0.0, room, &pl[1]) != 0 || pl[1].nunits == 0) goto fail;
                 deep_ctas = pl[1].nbatches;
                 if (deep_ctas * 2 > (uint64_t)pl[1].sms * occ) deep_ctas = (uint64_t)pl[1].sms * occ / 2;
-                if (part_setup(b, &b->part[1], &pl[1], 8, deep_ctas, budget, NULL) != 0) goto fail;
+                if (part_setup(b, &b->part[1], &pl[1], 8, deep_ctas, room, NULL) != 0) goto fail;
             }
-            if (nd2 && !wsg) { /* the lockstep deep part: the next-deepest requests stay with the rest */
+            if (nd2 && !dp[1].ctas) { /* the next-deepest requests stay with the rest */
                 for (size_t i = 0; i < nd2; i++) ps[ns++] = pd2[i];
                 nd2 = 0;
             }

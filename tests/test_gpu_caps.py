@@ -35,3 +35,25 @@ def test_one_topology_batch_under_a_cap(pkg, cuda, oracle, cb, n, copies):
         rc, labels, st = topo.challenge_blocks(KEY, blocks, s)
         assert rc == 0 and st["scratch_bytes"] <= s.scratch_cap_bytes
         assert labels == b"".join(want[32 * (x - rbo):32 * (x - rbo) + 32] for x in blocks)
+
+
+# two deep parts and the rest under one cap, on the depth and the lockstep kernel
+@pytest.mark.parametrize("kernel", ["1", "0"])
+@pytest.mark.parametrize("copies", [0, 20])
+def test_deep_parts_under_a_cap(pkg, cuda, oracle, monkeypatch, kernel, copies):
+    monkeypatch.setenv("POSE_B200_DEEP_KERNEL", kernel)
+    sizes = [(4096, 5), (2048, 9), (256, 20)]
+    topos = [pkg.Topology(cb) for cb, _ in sizes]
+    bufs = [cuda.zeros(n * cb * 32, dtype=cuda.uint8, device="cuda") for cb, n in sizes]
+    lock, depth = ([copy_bytes(pkg, t, k) for t in topos] for k in (1, 3))
+    s = pkg.Sched()
+    least = depth[0] + depth[1] + lock[2] if kernel == "1" else lock[0] + max(lock[1:])
+    s.scratch_cap_bytes = least + copies * lock[1]
+    with pkg.Batch([(t, KEY, b.data_ptr(), b.numel(), 4 * cb) for t, b, (cb, _) in zip(topos, bufs, sizes)],
+                   s) as batch:
+        rc, st = batch.run()
+    assert rc == 0 and st["scratch_bytes"] <= s.scratch_cap_bytes
+    for b, (cb, n) in zip(bufs, sizes):
+        assert b.cpu().numpy().tobytes() == oracle.label_region(KEY, cb, n, 4 * cb, threads=8).tobytes()
+    for t in topos:
+        t.free()

@@ -162,3 +162,34 @@ def test_server_packs_within_its_arena(fake, copies):
     fake.lib.fake_finish_events()
     assert not wait_all(fake, server, tickets)
     server.close()
+
+
+# more copies of the second deep part than the makespan search once took: the
+# first part then ran one copy a CTA, eight times one after the other
+def test_second_deep_part_of_any_size(fake):
+    deep, second = fake.topo(4096), fake.topo(2048)
+    fake.lib.fake_reset()
+    with fake.pkg.Batch(requests(deep, 1, 600) + requests(second, 1, 12000)):
+        pass
+    first = fake.launches()[0]
+    assert first.kind == DEPTH and first.nunits == 1200 and first.units_per > 1
+
+
+# the deep parts, the second one's CTAs too, and the rest share the cap, down
+# to one copy of each
+@pytest.mark.parametrize("kernel", ["1", "0"])
+@pytest.mark.parametrize("part", [2.0, 0.6, 0.3, 0.05, 0.02, 0])
+def test_deep_parts_keep_the_cap(fake, monkeypatch, part, kernel):
+    monkeypatch.setenv("POSE_B200_DEEP_KERNEL", kernel)
+    deep, second, small = fake.topo(4096), fake.topo(2048), fake.topo(256)
+    reqs = requests(deep, 40, 2) + requests(second, 60, 4) + requests(small, 20, 4)
+    d, s, r = (fake.copy_bytes(t) for t in (deep, second, small))
+    least = d[1] + s[1] + r[0] if kernel == "1" else d[0] + max(s[0], r[0])
+    cap = max(least, int(part * (160 * d[1] + 480 * s[1])))
+    fake.lib.fake_reset()
+    with fake.pkg.Batch(reqs, fake.sched(scratch_cap_bytes=cap)) as batch:
+        rc, st = batch.run()
+    ran = fake.launches()
+    assert rc == 0 and st["scratch_bytes"] == sum(x.scratch for x in ran) <= cap
+    if kernel == "1":  # both deep parts on the depth kernel whenever both fit it
+        assert [x.kind for x in ran] == [DEPTH, DEPTH, MULTI]
