@@ -343,7 +343,10 @@ static int admit_deep(pose_b200_server_t *s)
         return 1;
     }
     /* units per CTA: by the load, all deep units waiting or running spread
-     * over the SMs the depth kernel may hold */
+     * over the SMs the depth kernel may hold; more where the free SMs then
+     * take the group in fewer rounds of CTAs, one after the other (a second
+     * round is a second chain: 129 SMs, 29 of them free, 100 units in flight
+     * and 100 in the group are 50 CTAs by the load, 25 at four units) */
     uint32_t G = s->deep_units;
     if (!G) {
         uint64_t all = s->deep_inflight;
@@ -355,13 +358,23 @@ static int admit_deep(pose_b200_server_t *s)
         const uint64_t want = (all + s->sms - 1) / s->sms;
         G = want < 1 ? 1 : want < gmax ? (uint32_t)want : gmax;
     }
-    const uint64_t nbatches = (units + G - 1) / G;
-    uint32_t grid = (uint32_t)(nbatches < free_sms ? nbatches : free_sms);
-    const uint64_t per = (uint64_t)v2.gpool * 32 * G;
-    const uint64_t fit = arena_largest(s) / per;
-    if (fit < grid) grid = (uint32_t)fit;
+    const uint64_t copy = (uint64_t)(v2.gpool ? v2.gpool : 1) * 32, arena = arena_largest(s);
+    while (G > 1 && G * copy > s->arena_bytes) G--; /* a CTA that the arena can hold */
+    uint64_t rounds = 0;
+    uint32_t grid = 0;
+    for (uint32_t g = G, most = s->deep_units ? G : gmax; g <= most; g++) {
+        const uint64_t nb = (units + g - 1) / g;
+        uint64_t ctas = arena / (g * copy);
+        if (ctas > free_sms) ctas = free_sms;
+        if (ctas > nb) ctas = nb;
+        if (ctas == 0 || (grid && (nb + ctas - 1) / ctas >= rounds)) continue;
+        rounds = (nb + ctas - 1) / ctas;
+        grid = (uint32_t)ctas;
+        G = g;
+    }
     if (grid == 0) return 0; /* wait for scratch */
-    const uint64_t scratch = (uint64_t)grid * per;
+    const uint64_t nbatches = (units + G - 1) / G;
+    const uint64_t scratch = (uint64_t)grid * G * copy;
     uint64_t off = 0;
     if (arena_take(s, scratch, &off) != 0) return 0;
     /* tables: units | jobs | seeds | queue, 256-byte aligned */

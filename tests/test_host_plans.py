@@ -193,3 +193,39 @@ def test_deep_parts_keep_the_cap(fake, monkeypatch, part, kernel):
     assert rc == 0 and st["scratch_bytes"] == sum(x.scratch for x in ran) <= cap
     if kernel == "1":  # both deep parts on the depth kernel whenever both fit it
         assert [x.kind for x in ran] == [DEPTH, DEPTH, MULTI]
+
+
+# a deep request that fits the free SMs at the most copies a CTA takes runs in
+# one round of CTAs, whatever the load asks for; chunks of two copies each
+@pytest.mark.parametrize("sizes", [(50, 50), (60, 20), (30, 10, 50), (64, 1)])
+def test_served_depth_group_runs_in_one_round(fake, monkeypatch, sizes):
+    monkeypatch.setenv("POSE_B200_SERVER_DEEP_LEVELS", "1")
+    topo = fake.topo(512)
+    fake.lib.fake_reset()
+    fake.lib.fake_hold_events()
+    server = fake.pkg.Server(scratch_bytes=1 << 28)
+    sid, free, tickets = server.session(b"k" * 32), 148 - 148 // 8, []
+    for chunks in sizes:
+        assert 2 * chunks <= 4 * free
+        tickets.append(server.submit(topo, sid, 1 << 40, chunks * topo.super_bytes, 0))
+        end = time.time() + 20
+        while len(fake.launches()) < len(tickets) and time.time() < end:
+            time.sleep(0.01)
+        ran = fake.launches()[-1]
+        free -= ran.grid
+        assert ran.kind == DEPTH and ran.nunits == 2 * chunks and free >= 0
+        if ran.nbatches > ran.grid:
+            fake.lib.fake_finish_events()
+        assert ran.nbatches <= ran.grid, (ran.grid, ran.units_per, ran.nbatches)
+    fake.lib.fake_finish_events()
+    assert not wait_all(fake, server, tickets)
+    server.close()
+
+
+def test_served_depth_group_fits_the_arena(fake, monkeypatch):
+    monkeypatch.setenv("POSE_B200_SERVER_DEEP_LEVELS", "1")
+    topo = fake.topo(512)
+    server = fake.pkg.Server(scratch_bytes=fake.copy_bytes(topo)[0])  # one copy on the lockstep kernel
+    sid = server.session(b"k" * 32)
+    assert not wait_all(fake, server, [server.submit(topo, sid, 1 << 40, 200 * topo.super_bytes, 0)])
+    server.close()
