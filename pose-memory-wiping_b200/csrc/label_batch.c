@@ -854,13 +854,8 @@ no_split:
     if (!b) goto fail_host;
     b->device = dev;
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) goto fail;
-    {
-        int lo = 0, hi = 0; /* numerically lower is higher */
-        if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess) lo = hi = 0;
-        const int mid = hi < lo ? hi + 1 : hi;
-        if (nd && cudaStreamCreateWithPriority(&b->stream2, cudaStreamNonBlocking, hi) != cudaSuccess) goto fail;
-        if (nd2 && cudaStreamCreateWithPriority(&b->stream3, cudaStreamNonBlocking, mid) != cudaSuccess) goto fail;
-    }
+    if (nd && cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking) != cudaSuccess) goto fail;
+    if (nd2 && cudaStreamCreateWithFlags(&b->stream3, cudaStreamNonBlocking) != cudaSuccess) goto fail;
     for (int i = 0; i < 8; i++) if (cudaEventCreate(&b->ev[i]) != cudaSuccess) goto fail;
     b->blob_len = blob_len;
     if (pb_dev_malloc(&b->d_blob, blob_len ? blob_len : 1) != cudaSuccess) {
@@ -1024,9 +1019,11 @@ no_split:
         b->cv0 = (pl[0].nunits == 0 || b->part[0].cv0) && (!nd || b->part[1].cv0) && (!nd2 || b->part[2].cv0);
 
         /* capture: every launch's seeds on the batch's stream, then the deep
-         * parts forked onto streams of higher priority and the rest behind a
-         * second reset of its queue, so that the deep parts' CTAs, which need
-         * whole SMs and run longest, are placed first */
+         * parts forked off and the rest behind a second reset of its queue.
+         * The deep parts' CTAs need whole SMs and run longest, so they should
+         * be placed first.  Nothing orders the three launches, whose nodes all
+         * run at one priority: the deep ones are merely ready sooner, by the
+         * time that the reset takes. */
         if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) goto fail;
         int crc = 0;
         for (int i = b->nparts - 1; i >= 0 && crc == 0; i--)

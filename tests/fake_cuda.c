@@ -27,7 +27,7 @@ static fake_launch_t launches[4096];
 static int nlaunches;
 static uint64_t free_bytes = (uint64_t)170 << 30, live_bytes;
 static uint64_t event_seq, events_done = UINT64_MAX; /* events up to this one are complete */
-static int fail_multi_occupancy, occupancy_queries, node_priorities;
+static int fail_multi_occupancy, occupancy_queries, node_priorities, priority_streams;
 
 int fake_launches(fake_launch_t *out, int max)
 {
@@ -41,7 +41,7 @@ void fake_reset(void)
 {
     pthread_mutex_lock(&mu);
     nlaunches = 0;
-    occupancy_queries = 0;
+    occupancy_queries = priority_streams = 0;
     pthread_mutex_unlock(&mu);
 }
 void fake_set_free(uint64_t bytes) { free_bytes = bytes; }
@@ -50,6 +50,8 @@ void fake_hold_events(void) { pthread_mutex_lock(&mu); events_done = event_seq; 
 void fake_finish_events(void) { pthread_mutex_lock(&mu); events_done = UINT64_MAX; pthread_mutex_unlock(&mu); }
 void fake_fail_multi_occupancy(int on) { fail_multi_occupancy = on; }
 int fake_occupancy_queries(void) { return occupancy_queries; }
+int fake_priority_streams(void) { return priority_streams; }
+int fake_node_priorities(void) { return node_priorities; } /* of the last graph */
 
 static int record(uint32_t kind, uint32_t grid, uint32_t warps, uint32_t per, uint32_t nunits, uint32_t nbatches,
                   uint32_t smem, uint64_t scratch)
@@ -122,7 +124,12 @@ cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t e) { (void)e; return "fake"; }
 cudaError_t cudaStreamCreate(cudaStream_t *s) { *s = (cudaStream_t)calloc(1, 8); return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned f) { (void)f; return cudaStreamCreate(s); }
-cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned f, int p) { (void)f; (void)p; return cudaStreamCreate(s); }
+cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned f, int p)
+{
+    (void)f; (void)p;
+    priority_streams++;
+    return cudaStreamCreate(s);
+}
 cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned f) { (void)s; (void)e; (void)f; return cudaSuccess; }

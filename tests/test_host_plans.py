@@ -229,3 +229,13 @@ def test_served_depth_group_fits_the_arena(fake, monkeypatch):
     sid = server.session(b"k" * 32)
     assert not wait_all(fake, server, [server.submit(topo, sid, 1 << 40, 200 * topo.super_bytes, 0)])
     server.close()
+
+
+# a graph's nodes keep the priority of the stream they were captured from only
+# when it is instantiated so
+def test_no_priority_that_the_graph_ignores(fake):
+    fake.lib.fake_reset()
+    with fake.pkg.Batch(requests(fake.topo(4096), 8) + requests(fake.topo(2048), 8) + requests(fake.topo(256), 8)):
+        pass
+    assert len(fake.launches()) == 3
+    assert fake.lib.fake_priority_streams() == 0 or fake.lib.fake_node_priorities()
