@@ -203,8 +203,9 @@ static int build_pipelined(uint32_t S, uint32_t L, const uint8_t *np, const uint
     uint32_t *gstack = (uint32_t *)malloc((size_t)S * 4);
     uint32_t *sstack = (uint32_t *)malloc(((size_t)csm + 1) * 4);
     uint32_t *recs = (uint32_t *)malloc((size_t)S * 32);
+    const uint32_t none = csm > PB_CSM ? csm : PB_CSM; /* the entry after the pool */
     int rc = -1;
-    if (!d1 || !ss || !gs || !gstack || !sstack || !recs) goto out;
+    if (!d1 || !ss || !gs || !gstack || !sstack || !recs || none > PB_PLACE_SLOT_MASK) goto out;
     for (uint32_t id = 0; id < S; id++) {
         if (np[id] >= 1 && lvl[p0[id]] + 1 == lvl[id]) d1[p0[id]] = 1;
         if (np[id] >= 2 && lvl[p1[id]] + 1 == lvl[id]) d1[p1[id]] = 1;
@@ -234,7 +235,7 @@ static int build_pipelined(uint32_t S, uint32_t L, const uint8_t *np, const uint
     }
     for (uint32_t p = 0; p < S; p++) {
         uint32_t id = order[p], k = np[id], *r = recs + (size_t)8 * p;
-        uint32_t ref[2] = {0, 0}, place[2] = {PB_CSM, PB_CSM};
+        uint32_t ref[2] = {0, 0}, place[2] = {none, none};
         for (uint32_t e = 0; e < k; e++) {
             uint32_t q = e == 0 ? p0[id] : p1[id];
             if (lvl[q] + 1 != lvl[id]) {
@@ -245,7 +246,7 @@ static int build_pipelined(uint32_t S, uint32_t L, const uint8_t *np, const uint
                 place[e] = ss[q];
             } else {
                 ref[e] = PB_REF_PREV | gs[q];
-                place[e] = PB_PLACE_GLOBAL | PB_CSM;
+                place[e] = PB_PLACE_GLOBAL | none;
             }
         }
         r[0] = id | (k << PB_REC_NP_SHIFT) | (rank_of[id] != PB_NO_RANK ? PB_REC_OUT_BIT : 0);

@@ -46,7 +46,8 @@ extern "C" {
  *       begins: PB_PLACE_STAGED = staged for the node; else a slot of the
  *       shared-memory pool, PB_CSM (the entry after the pool, all zero) for an
  *       absent predecessor and, with PB_PLACE_GLOBAL, for one that is read
- *       from the global pool instead
+ *       from the global pool instead (records built for a pool of more than
+ *       PB_CSM slots, which the kernels refuse, have the entry after theirs)
  * A node's shared-memory copy lives for its own level and the next; nodes
  * whose level has more next-level-read labels than the pool holds fall back
  * to the global pool. */
