@@ -94,7 +94,9 @@ typedef struct {
 
 int pb_dev_label_multi(const pb_multi_params_t *params, uint32_t grid, uint32_t cta_threads, uint32_t smem_bytes,
                        cudaStream_t stream);
-/* Once per device before any launch or stream capture of k_label_multi. */
+/* Raises k_label_multi's shared memory limit too: once per device, and with
+ * success, before any launch or stream capture of it with more than 8 warps or
+ * with smem_bytes. */
 int pb_dev_label_multi_occupancy(uint32_t cta_threads, int *blocks_per_sm, uint32_t *alone_smem);
 int pb_dev_seed_jobs(const void *jobs, uint32_t njobs, const uint8_t *blob, uint32_t *seeds, cudaStream_t stream);
 

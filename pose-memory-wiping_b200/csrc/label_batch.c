@@ -868,9 +868,13 @@ no_split:
     {
         int occ = 0; /* 8-warp CTAs per SM */
         uint32_t alone_smem = 0;
-        if (pb_dev_label_multi_occupancy(256, &occ, &alone_smem) != 0 || occ <= 0) {
+        /* where the query fails, the default shared memory limit stands: teams
+         * of at most 8 warps, no padding */
+        const int wide = pb_dev_label_multi_occupancy(256, &occ, &alone_smem) == 0 && occ > 0;
+        if (!wide) {
+            cudaGetLastError();
             occ = 1;
-            alone_smem = 64 * 1024;
+            alone_smem = 0;
         }
         uint64_t budget = pb_topo_scratch_budget(reqs[0].topo, sched ? sched->scratch_cap_bytes : 0);
         uint64_t deep_ctas = 0;
@@ -939,12 +943,13 @@ no_split:
             budget = budget > used ? budget - used : 0;
         }
         const uint32_t gcap = sched && sched->units_per_team ? sched->units_per_team : 32;
-        uint32_t T = 16;
+        uint32_t T = wide ? 16 : 8;
         double eff = 0.0;
         const pose_hbm_topo_t *only = NULL;
         uint32_t ukern = 0, uT = 0, uG = 0, uteams = 0;
         if (open_sched && !nd && (only = one_topology(ps, ns)) != NULL &&
-            pb_topo_auto_plan(only, request_units(ps, ns), budget, &ukern, &uT, &uG, &uteams) != 0)
+            (pb_topo_auto_plan(only, request_units(ps, ns), budget, &ukern, &uT, &uG, &uteams) != 0 ||
+             (ukern == 1 && uT > T)))
             ukern = 0;
         pb_topo_view2_t uv2;
         uint32_t umax = 0;
@@ -987,7 +992,7 @@ no_split:
                  * end when the second one could have ended elsewhere (256
                  * sessions, 5 and 8 copies a CTA: 1284 against 1181 ms) */
                 const uint32_t per_sm = 16 / T;
-                b->part[0].smem = per_sm == 1 ? alone_smem : alone_smem / per_sm - 2048;
+                b->part[0].smem = per_sm == 1 || !wide ? alone_smem : alone_smem / per_sm - 2048;
                 cap = (uint64_t)pl[0].sms * per_sm;
             } else if (open_sched) {
                 int o = 1;

@@ -147,7 +147,8 @@ struct pose_b200_server {
     uint32_t all_sms;
     uint32_t conns;            /* host-to-device work queues (CUDA_DEVICE_MAX_CONNECTIONS, default 8) */
     uint32_t wsg_smem_max;     /* the depth kernel's shared-memory limit (0: no depth kernel) */
-    int occ;
+    int occ;                   /* teams of a wave per SM */
+    uint32_t wave_warps;       /* and warps per team */
     uint64_t waves_launched;
     double busy_ms;
 };
@@ -499,7 +500,7 @@ static int admit_wave(pose_b200_server_t *s)
         pr[i].seed_len = s->sess_len[r->session];
     }
     pb_plan_tables_t pl;
-    const uint32_t Tw = 16;
+    const uint32_t Tw = s->wave_warps;
     if (pb_plan_fill(pr, n, s->all_sms - s->deep_ctas, Tw, s->arena_bytes, &pl) != 0) {
         free(pr);
         for (size_t i = 0; i < n; i++) { s->reqs[wv->reqs[i]].state = 3; s->reqs[wv->reqs[i]].t_done = now_ms(); }
@@ -794,7 +795,13 @@ pose_b200_server_t *pose_b200_server_create(uint64_t scratch_bytes, uint32_t max
         const char *e5 = getenv("POSE_B200_SERVER_DEEP_EXCL");
         if (e5 && e5[0]) s->deep_excl = atoi(e5) != 0;
     }
-    if (pb_dev_label_multi_occupancy(512, &s->occ, NULL) != 0) s->occ = 1;
+    s->wave_warps = 16;
+    if (pb_dev_label_multi_occupancy(512, &s->occ, NULL) != 0) {
+        /* the default shared memory limit stands, which 8-warp teams keep */
+        cudaGetLastError();
+        s->wave_warps = 8;
+        s->occ = 1;
+    }
     /* Launch tables and completion counters of every slot, allocated up
      * front: the dispatcher then makes no allocation while kernels run (a
      * cudaFree there waits for the whole device, and the submitters and

@@ -239,3 +239,24 @@ def test_no_priority_that_the_graph_ignores(fake):
         pass
     assert len(fake.launches()) == 3
     assert fake.lib.fake_priority_streams() == 0 or fake.lib.fake_node_priorities()
+
+
+# k_label_multi's occupancy query also raises its shared memory limit: where it
+# fails, launches keep to the default one (48 KB a CTA, 96 bytes a thread)
+@pytest.mark.parametrize("mix", [(300, 256), (4096, 2048, 256), (512,)])
+def test_default_shared_memory_limit(fake, mix):
+    topos = [fake.topo(cb) for cb in mix]
+    reqs = [r for t in topos for r in requests(t, 400)]
+    fake.lib.fake_fail_multi_occupancy(1)
+    try:
+        fake.lib.fake_reset()
+        with fake.pkg.Batch(reqs) as b:
+            assert b.run()[0] == 0
+        server = fake.pkg.Server(scratch_bytes=1 << 30)
+        sid = server.session(b"k" * 32)
+        assert not wait_all(fake, server, [server.submit(t, sid, 1 << 40, t.super_bytes, 0) for t in topos])
+        server.close()
+        ran = [x for x in fake.launches() if x.kind == MULTI]
+        assert ran and all(x.warps <= 8 and x.smem <= 48 * 1024 - 1024 for x in ran)
+    finally:
+        fake.lib.fake_fail_multi_occupancy(0)
