@@ -833,10 +833,6 @@ static int topo_label_core_impl(const pose_hbm_topo_t *ct, const uint8_t *sessio
         set_err("pose_b200_topo_label: cluster_ctas must be 0, 1, 2, 4, 8 or 16, with the depth kernel");
         return -1;
     }
-    if (sched && sched->kernel > 3) {
-        set_err("pose_b200_topo_label: kernel must be 0 (automatic), 1, 2 or 3");
-        return -1;
-    }
     int prev = -1, rc = -1;
     uint32_t *h_seeds = NULL;
     cudaGetDevice(&prev);

@@ -10,8 +10,8 @@
  *     records, so a team runs G units of the same topology in lockstep and a
  *     level of width w becomes G*w independent node hashes.  That packs the
  *     many narrow levels of the depth-robust DAG into full warps.
- *   - A team is T warps (T = 1: __syncwarp between levels; T > 1: a named
- *     barrier per team).  Teams pull batches of G units from a device work
+ *   - A team is a CTA of T warps (T = 1: __syncwarp between levels; T > 1: the
+ *     CTA barrier).  Teams pull batches of G units from a device work
  *     counter until the launch's units are exhausted (no waiting on other
  *     teams, so no spin-waits exist anywhere).
  *   - Scratch is the recycled slot pool of the topology, one per unit,
@@ -38,20 +38,13 @@ __constant__ uint32_t c_key_src[8];
 __constant__ uint32_t c_key_int[8];
 __constant__ uint32_t c_key_chunk_seed[8];
 
-/* Team barrier.  CTA_TEAM: the team is the whole CTA, so barrier 0 serves
- * (a kernel that names only barrier 0 reserves one barrier per CTA, not all
- * sixteen, and its CTAs are not held back by the SM's barrier count);
- * otherwise the named barrier bar_id over the team's nthreads threads. */
-template <bool CTA_TEAM>
-__device__ __forceinline__ void team_sync(uint32_t team_warps, uint32_t bar_id, uint32_t nthreads)
+/* Team barrier.  A team is a whole CTA, so barrier 0 serves: a kernel that
+ * names only barrier 0 reserves one barrier per CTA, not all sixteen, and its
+ * CTAs are not held back by the SM's barrier count. */
+__device__ __forceinline__ void team_sync(uint32_t team_warps)
 {
-    if (team_warps == 1) {
-        __syncwarp();
-    } else if (CTA_TEAM) {
-        __syncthreads();
-    } else {
-        asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(nthreads) : "memory");
-    }
+    if (team_warps == 1) __syncwarp();
+    else __syncthreads();
 }
 
 __device__ __forceinline__ void key_words(uint32_t (&cv)[8], bool source)
@@ -218,9 +211,8 @@ __device__ __forceinline__ void seed_words(uint32_t (&m)[16], const pb_topo_view
  * reads back only its own staging slots, after waiting for its own copies.
  * TABLE: every topology of the launch has its block-0 table (a kernel without
  * the other path runs 1 % faster than one that has it and does not use it). */
-template <bool TABLE, bool CTA_TEAM>
-__device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const UnitCtx &c, uint32_t T,
-                                             uint32_t bar_id, uint32_t TT)
+template <bool TABLE>
+__device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const UnitCtx &c, uint32_t T)
 {
     const uint32_t L = tp.L;
     uint32_t s0 = __ldg(tp.lstart);
@@ -289,7 +281,7 @@ __device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const Uni
                 }
             }
         }
-        team_sync<CTA_TEAM>(T, bar_id, TT);
+        team_sync(T);
         s0 = s1;
         s1 = s2;
         s2 = s3;
@@ -297,19 +289,17 @@ __device__ __forceinline__ void label_levels(const pb_topo_view_t &tp, const Uni
 }
 
 /* Team-wide batch index from the work counter. */
-template <bool CTA_TEAM>
-__device__ __forceinline__ uint32_t grab_batch(unsigned int *queue, uint32_t T, uint32_t team, uint32_t tt,
-                                               uint32_t bar_id, uint32_t TT, uint32_t *s_batch)
+__device__ __forceinline__ uint32_t grab_batch(unsigned int *queue, uint32_t T, uint32_t tt, uint32_t *s_batch)
 {
     if (T == 1) {
         uint32_t b = 0;
         if ((threadIdx.x & 31) == 0) b = atomicAdd(queue, 1u);
         return __shfl_sync(0xFFFFFFFFu, b, 0);
     }
-    if (tt == 0) s_batch[team] = atomicAdd(queue, 1u);
-    team_sync<CTA_TEAM>(T, bar_id, TT);
-    const uint32_t b = s_batch[team];
-    team_sync<CTA_TEAM>(T, bar_id, TT);
+    if (tt == 0) *s_batch = atomicAdd(queue, 1u);
+    team_sync(T);
+    const uint32_t b = *s_batch;
+    team_sync(T);
     return b;
 }
 
@@ -320,12 +310,10 @@ __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant_
 {
     const uint32_t T = p.team_warps;
     const uint32_t TT = T * 32;
-    const uint32_t team = 0;
     const uint32_t tt = threadIdx.x;
     const uint64_t gteam = blockIdx.x;
-    const uint32_t bar_id = 0;
     const pb_topo_view_t &tp = p.topo;
-    __shared__ uint32_t s_batch[1];
+    __shared__ uint32_t s_batch;
     UnitCtx c;
     c.G = p.units_per_team;
     c.q = tt / c.G;
@@ -334,7 +322,7 @@ __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant_
     c.tscr = reinterpret_cast<uint4 *>(p.scratch + gteam * p.team_scratch_bytes);
 
     for (;;) {
-        const uint32_t batch = grab_batch<true>(p.queue, T, team, tt, bar_id, TT, s_batch);
+        const uint32_t batch = grab_batch(p.queue, T, tt, &s_batch);
         if (batch >= p.nbatches) break;
         const uint32_t unit = batch * c.G + c.u;
         c.valid = c.q < c.stride && unit < p.nunits; /* TT - stride * G threads have no unit */
@@ -347,7 +335,7 @@ __global__ void __launch_bounds__(PB_CTA_THREADS) k_label(const __grid_constant_
         c.cv0 = tp.cv0 ? tp.cv0 + (uint64_t)copy * tp.S * 2 : nullptr;
 #pragma unroll
         for (int i = 0; i < 8; i++) c.seed[i] = c.valid ? p.seeds[8 * (size_t)chunk + i] : 0u;
-        label_levels<TABLE, true>(tp, c, T, bar_id, TT);
+        label_levels<TABLE>(tp, c, T);
     }
 }
 
@@ -360,24 +348,22 @@ __global__ void __launch_bounds__(PB_MULTI_CTA_THREADS, 2) k_label_multi(const _
 {
     const uint32_t T = p.team_warps;
     const uint32_t TT = T * 32;
-    const uint32_t team = 0;
     const uint32_t tt = threadIdx.x;
     const uint64_t gteam = blockIdx.x;
-    const uint32_t bar_id = 0;
-    __shared__ uint32_t s_batch[1];
-    __shared__ pb_topo_view_t s_topo[1];
+    __shared__ uint32_t s_batch;
+    __shared__ pb_topo_view_t s_topo;
     UnitCtx c;
     c.tscr = reinterpret_cast<uint4 *>(p.scratch + gteam * p.team_scratch_bytes);
 
     for (;;) {
-        const uint32_t batch = grab_batch<true>(p.queue, T, team, tt, bar_id, TT, s_batch);
+        const uint32_t batch = grab_batch(p.queue, T, tt, &s_batch);
         if (batch >= p.nbatches) break;
         const pb_mbatch_t bd = p.batches[batch];
         if (tt < sizeof(pb_topo_view_t) / 4)
-            reinterpret_cast<uint32_t *>(&s_topo[team])[tt] =
+            reinterpret_cast<uint32_t *>(&s_topo)[tt] =
                 reinterpret_cast<const uint32_t *>(p.topos + bd.topo)[tt];
-        team_sync<true>(T, bar_id, TT);
-        const pb_topo_view_t &tp = s_topo[team];
+        team_sync(T);
+        const pb_topo_view_t &tp = s_topo;
         c.G = bd.G;
         c.q = tt / c.G;
         c.u = tt - c.q * c.G;
@@ -392,14 +378,14 @@ __global__ void __launch_bounds__(PB_MULTI_CTA_THREADS, 2) k_label_multi(const _
         c.cv0 = tp.cv0 ? tp.cv0 + (uint64_t)copy * tp.S * 2 : nullptr;
 #pragma unroll
         for (int i = 0; i < 8; i++) c.seed[i] = c.valid ? p.seeds[8 * (size_t)un.seed + i] : 0u;
-        label_levels<TABLE, true>(tp, c, T, bar_id, TT);
+        label_levels<TABLE>(tp, c, T);
         /* label_levels ended with a team barrier, so every persisted label of
          * the batch is ordered before this fence */
         if (p.req_done != nullptr && tt < bd.count) {
             __threadfence_system();
             atomicAdd_system(p.req_done + p.unit_req[bd.first_unit + tt], 1u);
         }
-        team_sync<true>(T, bar_id, TT); /* s_topo[team] is rewritten by the next batch */
+        team_sync(T); /* s_topo is rewritten by the next batch */
     }
 }
 

@@ -164,7 +164,7 @@ static int pose_b200_label_stream_impl(const pose_hbm_topo_t *topo, const uint8_
     cudaGetDevice(&s.device);
     int rc = -1, started = 0;
     pthread_t th;
-    double t0 = now_ms(), kernel_ms = 0, label_ms = 0;
+    double t0 = now_ms(), kernel_ms = 0;
     uint64_t nodes = 0;
     uint32_t launches = 0;
     pose_b200_stats_t last;
@@ -198,12 +198,10 @@ static int pose_b200_label_stream_impl(const pose_hbm_topo_t *topo, const uint8_
         int err = s.error;
         pthread_mutex_unlock(&s.mu);
         if (err) goto out;
-        double l0 = now_ms();
         pose_b200_stats_t st;
         if (pose_b200_topo_label(topo, session_seed, seed_len, s.dev[i], n * sb,
                                  region_block_offset + first * (uint64_t)cb, sched, &st) != 0)
             goto out;
-        label_ms += now_ms() - l0;
         kernel_ms += st.kernel_ms;
         nodes += st.nodes;
         launches += st.kernel_launches;
@@ -249,7 +247,6 @@ out:
     if (s.stream) cudaStreamDestroy(s.stream);
     pthread_mutex_destroy(&s.mu);
     pthread_cond_destroy(&s.cv);
-    (void)label_ms;
     return rc;
 }
 
