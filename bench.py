@@ -141,12 +141,13 @@ class ClockSampler:
 KERNEL_NAMES = {1: "k_label", 3: "k_label_ws", 4: "k_label_multi"}
 
 
-def profiled_traffic(workload_name: str, kernel: int) -> float | None:
-    """DRAM bytes (read + write) per launch of the kernel the plan ran, from
-    the `bench-traffic: <workload> <kernel> <bytes>` lines of the ncu
-    summaries in profiles/ (one ncu capture of the same command); None when
-    no capture covers this workload and kernel."""
-    name = KERNEL_NAMES.get(kernel)
+def profiled_traffic(workload_name: str, kernel: int, cluster_ctas: int = 0) -> float | None:
+    """DRAM bytes (read + write) per launch of the kernel the plan ran (the
+    depth kernel with a cluster per copy is k_label_wsc), from the
+    `bench-traffic: <workload> <kernel> <bytes>` lines of the ncu summaries in
+    profiles/ (one ncu capture of the same command); None when no capture
+    covers this workload and kernel."""
+    name = "k_label_wsc" if kernel == 3 and cluster_ctas > 1 else KERNEL_NAMES.get(kernel)
     pdir = os.path.join(ROOT, "profiles")
     if not name or not os.path.isdir(pdir):
         return None
@@ -565,7 +566,7 @@ def run_b200(args) -> None:
     peak_ops = rate * ops_per_compress
     info = topo.info()
     levels = info["levels"]
-    traffic = profiled_traffic(w["name"], st0["kernel"]) if not args.chunks else None
+    traffic = profiled_traffic(w["name"], st0["kernel"], st0["cluster_ctas"]) if not args.chunks else None
     hbm_gbs = measured_hbm_gbs()
     clocks = clk.summary()
     # depth bound: one label per level on the critical path, each ~comps
