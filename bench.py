@@ -161,6 +161,19 @@ def profiled_traffic(workload_name: str, kernel: int, cluster_ctas: int = 0) -> 
     return None
 
 
+# Clocks of one compression by four lanes, the shortest chain that the depth
+# kernel has on a narrow level (measured with 1 to 4 warps an SM;
+# csrc/b3_device.cuh, quad_compress).
+FOUR_LANE_CYCLES = 755.0
+
+
+def chain_cycles(comps: int, lat_cycles: float) -> float:
+    """Clocks of one compression on a level's dependent chain: by one lane as
+    measured in this run, or, with the block-0 table (two compressions a
+    node), which the depth kernel needs, by four."""
+    return min(lat_cycles, FOUR_LANE_CYCLES) if comps == 2 else lat_cycles
+
+
 def measured_hbm_gbs() -> float | None:
     """The pool's measured HBM copy bandwidth (MEASURED_PEAKS.json, written
     per GPU pod), or None when the file is absent."""
@@ -349,7 +362,7 @@ def run_plain_leg(pkg, torch, name: str, rate: float, lat_cycles: float, warm: i
     comps = 2 if best["used_cv0_table"] else 3
     clocks = clk.summary()
     sm_hz = (clocks.get("sm_mhz") or 1965.0) * 1e6
-    t_depth = levels * comps * lat_cycles / sm_hz
+    t_depth = levels * comps * chain_cycles(comps, lat_cycles) / sm_hz
     achieved = best["nodes"] * comps * 680.0 / (best["kernel_ms"] * 1e-3)
     out = {"workload": f"{name}: {nsup} super-chunks of chunk_blocks {cb}, key splitmix64",
            "value": nbytes / MIB / (best["total_ms"] * 1e-3), "unit": "MiB/s", "ms": best["total_ms"],
@@ -569,10 +582,10 @@ def run_b200(args) -> None:
     traffic = profiled_traffic(w["name"], st0["kernel"], st0["cluster_ctas"]) if not args.chunks else None
     hbm_gbs = measured_hbm_gbs()
     clocks = clk.summary()
-    # depth bound: one label per level on the critical path, each ~comps
-    # dependent compressions at the measured compression latency
+    # depth bound: one label per level on the critical path, each comps
+    # dependent compressions
     sm_hz = (clocks.get("sm_mhz") or 1965.0) * 1e6
-    t_depth = levels * comps * lat_cycles / sm_hz
+    t_depth = levels * comps * chain_cycles(comps, lat_cycles) / sm_hz
     line = {
         "metric": "label MiB/s (persisted output-set bytes / time)",
         "value": value, "unit": "MiB/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
@@ -598,7 +611,8 @@ def run_b200(args) -> None:
                      "spec_ops_per_node": 3 * ops_per_compress,
                      "depth_bound_mib_s": nsup * sb / MIB / t_depth if t_depth > 0 else None,
                      "depth_frac": (t_depth * 1e3) / kernel_ms if kernel_ms > 0 else None,
-                     "compress_latency_cycles": lat_cycles},
+                     "compress_latency_cycles": lat_cycles,
+                     "chain_latency_cycles": chain_cycles(comps, lat_cycles)},
         "e2e": {"value": e2e_value, "unit": "MiB/s", "h2d_bytes_per_step": len(w["key"]),
                 "d2h_bytes_per_step": nbytes},
         "parity": "mismatch" if "mismatch" in (par_dev["parity"], par_host["parity"]) else par_dev["parity"],

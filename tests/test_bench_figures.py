@@ -28,3 +28,10 @@ def test_traffic_of_the_kernel_that_ran(bench):
     assert any(w == "plain_2e17" for w, _ in lines)
     for kernel, cluster, name in ((1, 0, "k_label"), (3, 1, "k_label_ws"), (3, 2, "k_label_wsc")):
         assert bench.profiled_traffic("plain_2e17", kernel, cluster) == lines.get(("plain_2e17", name))
+
+
+def test_depth_bound_is_the_shortest_chain(bench):
+    # narrow levels are hashed by four lanes a node where there is a block-0 table
+    assert bench.chain_cycles(2, 995.5) == bench.FOUR_LANE_CYCLES < 964
+    assert bench.chain_cycles(2, 700.0) == 700.0
+    assert bench.chain_cycles(3, 995.5) == 995.5
