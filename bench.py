@@ -243,7 +243,13 @@ def run_reference_arm(args) -> None:
     # 2 s), so the requested K and W are run as given
     steps = max(1, args.steps)
     warm = max(0, args.warmup)
-    cb = cpu_reference(w, steps, warm)
+    try:
+        cb = cpu_reference(w, steps, warm)
+    except FileNotFoundError as e:
+        # the reference CPU build is made from the reference's sources, where those are
+        print(json.dumps({"impl": "reference", "unavailable": f"no reference CPU build: {os.path.basename(str(e))}"}),
+              flush=True)
+        return
     line = {"metric": "label MiB/s (persisted output-set bytes / time)", "value": cb["value"],
             "unit": "MiB/s", "n_gpus": args.gpus, "steps": steps, "warmup": warm,
             "ms_per_step": cb["seconds_per_step"] * 1e3, "higher_is_better": True, "scaling": "weak",

@@ -35,3 +35,16 @@ def test_depth_bound_is_the_shortest_chain(bench):
     assert bench.chain_cycles(2, 995.5) == bench.FOUR_LANE_CYCLES < 964
     assert bench.chain_cycles(2, 700.0) == 700.0
     assert bench.chain_cycles(3, 995.5) == 995.5
+
+
+def test_reference_arm_without_its_build(bench, monkeypatch, capsys):
+    import types
+
+    def missing(*_):
+        raise FileNotFoundError("/somewhere/libposeref.so")
+    monkeypatch.setattr(bench, "cpu_reference", missing)
+    monkeypatch.setattr(bench, "load_pkg", lambda: None)
+    monkeypatch.delenv("RANK", raising=False)
+    bench.run_reference_arm(types.SimpleNamespace(workload="plain_small", steps=1, warmup=0, gpus=1, no_aux=True))
+    line = bench.json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "libposeref.so" in line["unavailable"]
