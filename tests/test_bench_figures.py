@@ -43,7 +43,6 @@ def test_reference_arm_without_its_build(bench, monkeypatch, capsys):
     def missing(*_):
         raise FileNotFoundError("/somewhere/libposeref.so")
     monkeypatch.setattr(bench, "cpu_reference", missing)
-    monkeypatch.setattr(bench, "load_pkg", lambda: None)
     monkeypatch.delenv("RANK", raising=False)
     bench.run_reference_arm(types.SimpleNamespace(workload="plain_small", steps=1, warmup=0, gpus=1, no_aux=True))
     line = bench.json.loads(capsys.readouterr().out)
