@@ -178,8 +178,14 @@ typedef int (*pose_b200_sink_fn)(void *ctx, const uint8_t *buf, size_t len, uint
  * k+1 is labelled on the GPU while window k is copied to pinned host memory
  * and sunk, which the reference's disk worker does one after the other
  * (tools/disk-wipe-bench/disk_wipe_bench.cu:646-697).  `off` of window k is
- * byte_offset + k*window.  Synchronous; 0 on success, -1 on error (including
- * a failing sink). */
+ * byte_offset + k*window.  Without a schedule, windows of few chunk copies
+ * are labelled several at a time (up to eight copies per SM, half the region
+ * and a quarter of the free device memory) and still sunk one by one: the call
+ * then holds two device buffers of that many windows, and the topology's
+ * workspace grows as for one labeling call of that size; with a schedule each
+ * window is labelled by itself.  Synchronous; 0 on success, -1 on error
+ * (including a failing sink, after which the sink is not called again and the
+ * call returns once the labeling in progress has ended). */
 int pose_b200_label_stream(const pose_hbm_topo_t *topo, const uint8_t *session_seed, size_t seed_len,
                            uint64_t region_bytes, uint64_t region_block_offset, uint64_t byte_offset,
                            size_t window_bytes, pose_b200_sink_fn sink, void *sink_ctx,

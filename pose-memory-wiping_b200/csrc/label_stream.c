@@ -11,13 +11,14 @@
  * already labels the next ones.  A window of few chunk copies leaves most of
  * the GPU idle for the length of their chain, so consecutive windows are
  * labelled in one call until it has some eight copies per SM
- * (PB_STREAM_UNITS); the sink still gets them one by one, in order.  The sink
+ * (PB_STREAM_UNITS_PER_SM); the sink still gets them one by one, in order.  The sink
  * has the shape of the reference's pose_label_sink_fn
  * (common/include/graph.h:244-245) and, as there, may be called from a worker
  * thread.
  */
 #include "pose_b200.h"
 #include "dev_alloc.h"
+#include "topo_internal.h"
 
 #include <nvtx3/nvToolsExt.h>
 #include <cuda_runtime_api.h>
@@ -27,10 +28,10 @@
 #include <string.h>
 #include <time.h>
 
-/* Chunk copies of one labelling call.  2048 chunks of 4096 blocks in windows
- * of 256 chunks, 512 copies: 19.9 ms a call; 1024 copies 28.5, 1536 copies
- * about 36, 4096 copies 78. */
-#define PB_STREAM_UNITS 1184u
+/* Chunk copies per SM of one labelling call.  On 148 SMs, 2048 chunks of 4096
+ * blocks in windows of 256 chunks, 512 copies: 19.9 ms a call; 1024 copies
+ * 28.5, 1536 copies about 36, 4096 copies 78. */
+#define PB_STREAM_UNITS_PER_SM 8u
 
 typedef struct {
     pthread_mutex_t mu;
@@ -127,27 +128,29 @@ static int pose_b200_label_stream_impl(const pose_hbm_topo_t *topo, const uint8_
         fprintf(stderr, "pose_b200_label_stream: NULL topology or sink\n");
         return -1;
     }
-    uint32_t cb = 0;
-    pose_b200_topo_info(topo, &cb, NULL, NULL, NULL, NULL);
-    const uint64_t sb = (uint64_t)cb * 32;
+    pb_topo_internal_t ti;
+    if (pb_topo_internal(topo, &ti) != 0) return -1;
+    const uint32_t cb = ti.cb;
+    const uint64_t sb = ti.super_bytes;
     const uint64_t nsuper = region_bytes / sb;
     if (nsuper == 0) return 0;
     uint64_t W = window_bytes / sb;
     if (W == 0) W = 1;
     if (W > nsuper) W = nsuper;
-    /* windows per labelling call: up to PB_STREAM_UNITS chunk copies, half
-     * the region (the first half is sunk while the second is labelled) and a
-     * quarter of the free device memory; a caller's schedule is for its own
-     * window */
+    /* windows per labelling call: up to PB_STREAM_UNITS_PER_SM chunk copies
+     * an SM, half the region (the first half is sunk while the second is
+     * labelled) and a quarter of the free device memory; a caller's schedule
+     * is for its own window */
     uint64_t per = 1;
     if (!sched) {
-        const uint64_t copies = W * 2, half = (nsuper + W - 1) / W / 2;
+        const uint64_t units = (uint64_t)PB_STREAM_UNITS_PER_SM * (uint64_t)(ti.sms > 0 ? ti.sms : 1);
+        const uint64_t copies = W * ti.copies, half = (nsuper + W - 1) / W / 2;
         size_t fr = 0, tot = 0;
         if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
             cudaGetLastError();
             fr = 0;
         }
-        per = (PB_STREAM_UNITS + copies - 1) / copies;
+        per = (units + copies - 1) / copies;
         if (per > half) per = half;
         while (per > 1 && 2 * per * W * sb > fr / 4) per--;
         if (per == 0) per = 1;

@@ -260,3 +260,22 @@ def test_default_shared_memory_limit(fake, mix):
         assert ran and all(x.warps <= 8 and x.smem <= 48 * 1024 - 1024 for x in ran)
     finally:
         fake.lib.fake_fail_multi_occupancy(0)
+
+
+# windows labelled together: eight chunk copies an SM, of one or two copies a chunk
+@pytest.mark.parametrize("cb,copies", [(1, 1), (64, 2)])
+def test_stream_groups(fake, cb, copies):
+    topo, window, n = fake.topo(cb), 16, 4096
+    got = []
+    fake.lib.fake_reset()
+    rc, st = topo.label_stream(b"k" * 32, n * topo.super_bytes, lambda v, off: got.append((len(v), off)),
+                               window_bytes=window * topo.super_bytes)
+    wb = window * topo.super_bytes
+    assert rc == 0 and got == [(wb, i * wb) for i in range(n // window)]
+    per = -(-8 * 148 // (window * copies))  # windows a call
+    assert [x.nunits for x in fake.launches()][0] == per * window * copies
+    # a caller's schedule is for its own window
+    fake.lib.fake_reset()
+    rc, _ = topo.label_stream(b"k" * 32, 64 * topo.super_bytes, lambda v, off: 0, window_bytes=wb,
+                              sched=fake.sched(kernel=1))
+    assert rc == 0 and [x.nunits for x in fake.launches()] == [window * copies] * 4
