@@ -138,11 +138,12 @@ typedef struct pose_b200_batch pose_b200_batch_t;
  * team slots.  The environment variable POSE_B200_DEEP_KERNEL=0 selects the
  * lockstep kernel in every case.  With the depth kernel, the requests of the
  * deepest remaining topology, when its chain is at least a third of the
- * deepest, run as a third launch of it.  The copies per CTA of both launches
- * are those with the shortest estimated makespan, the rest filled in behind
- * them.  Requests that all share one topology run as pose_b200_topo_label
- * would run that many chunk copies, unless sched fixes something;
- * POSE_B200_DEEP2=0 keeps them with the rest. */
+ * deepest, run as a third launch of it (POSE_B200_DEEP2=0 keeps them with the
+ * rest).  The copies per CTA of both launches are those with the shortest
+ * estimated makespan, the rest filled in behind them; where scratch_cap_bytes
+ * or the free memory allows fewer CTAs, those run several batches each.
+ * Requests that all share one topology run as pose_b200_topo_label would run
+ * that many chunk copies, unless sched fixes more than the cap. */
 pose_b200_batch_t *pose_b200_batch_create(const pose_b200_request_t *reqs, size_t n,
                                           const pose_b200_sched_t *sched);
 /* The empirical autotuner: rank the schedules sched leaves open (team size
@@ -202,7 +203,7 @@ int pose_b200_label_stream(const pose_hbm_topo_t *topo, const uint8_t *session_s
  * the device:
  *   - requests of deep topologies (chunk_blocks 2^15 and up) run on the depth
  *     kernel, the pending ones of one topology together, one to four chunk
- *     copies per CTA by the load, each CTA holding its SM alone, on
+ *     copies per CTA by the load and the free SMs, each CTA holding its SM alone, on
  *     high-priority streams and at most 7/8 of the SMs; one that does not fit
  *     the free SMs waits;
  *   - the others run in waves: one persistent multi-topology launch per
@@ -215,7 +216,7 @@ int pose_b200_label_stream(const pose_hbm_topo_t *topo, const uint8_t *session_s
  * CUDA_DEVICE_MAX_CONNECTIONS (8 by default; 32 gives every slot its own)
  * bounds how many run at once.  Tuning variables, read at creation:
  * POSE_B200_SERVER_DEEP_LEVELS (levels from which a topology is deep),
- * POSE_B200_SERVER_DEEP_UNITS (copies per depth CTA; 0 = by the load),
+ * POSE_B200_SERVER_DEEP_UNITS (copies per depth CTA; 0 = by load and free SMs),
  * POSE_B200_SERVER_DEEP_GMAX (the most then), POSE_B200_SERVER_DEEP_EXCL and POSE_B200_SERVER_DEEP_WAIT
  * (0: share SMs; 0: join a wave instead of waiting), POSE_B200_SERVER_DEEP=0
  * (every request in waves), POSE_B200_SERVER_DEEP_SMS (SMs the depth kernel
@@ -230,9 +231,8 @@ typedef struct pose_b200_server pose_b200_server_t;
 pose_b200_server_t *pose_b200_server_create(uint64_t scratch_bytes, uint32_t max_waves);
 /* Register a session seed (<= 1016 bytes); returns its id, or -1. */
 int pose_b200_server_session(pose_b200_server_t *server, const uint8_t *seed, size_t seed_len);
-/* Make ready, ahead of the first request, what requests of this topology
- * need beyond the topology itself (at present nothing).  Optional.  0 on
- * success, -1 on a bad argument. */
+/* Does nothing: a topology has all that its requests need.  0, or -1 on a
+ * NULL argument. */
 int pose_b200_server_prepare(pose_b200_server_t *server, const pose_hbm_topo_t *topo);
 /* Queue one request; returns its ticket, or -1. */
 int64_t pose_b200_server_submit(pose_b200_server_t *server, const pose_hbm_topo_t *topo, int session,

@@ -418,8 +418,8 @@ class Server:
         return sid
 
     def prepare(self, topo: "Topology") -> None:
-        """Build what requests of this topology need before the first one
-        arrives (the depth kernel's records of a deep topology)."""
+        """pose_b200_server_prepare, which does nothing: a topology has all
+        that its requests need."""
         if load().pose_b200_server_prepare(self.handle, topo.handle) != 0:
             raise RuntimeError("server prepare failed")
 
