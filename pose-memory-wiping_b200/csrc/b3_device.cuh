@@ -65,13 +65,13 @@ __device__ __forceinline__ uint32_t madd(uint32_t a, uint32_t one, uint32_t b)
  * ALU pipe, which then bounds both one warp and a full SM, so its additions
  * are kept off that pipe: a + b + m is a plain a + m, off the dependent chain
  * since a and m are known before b, then an integer multiply-add b * 1 + that
- * (`one`, opaque to the compiler, keeps it a multiply-add, which the FMA pipe
- * executes); c + d is left to the compiler, which spreads it over both pipes.
+ * (`one`, opaque to the compiler, keeps it a multiply-add, which goes to the
+ * FMA pipe); c + d is left to the compiler.
  * The best of 145 mixes of the four additions (plain, multiply-add, either
  * order, alternating between columns) in latency and in throughput: 964
  * clocks a compression for one warp and 40.0 G compressions/s with every SM
- * full, against 1162 clocks and 32.7 G/s with all additions plain, and at
- * most 36.9 G/s with all of them multiply-adds. */
+ * full (39.7 in k_compress_bench), against 1162 clocks and 32.7 G/s with all
+ * additions plain, and at most 36.9 G/s with all of them multiply-adds. */
 __device__ __forceinline__ void g_mix(uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d,
                                       uint32_t x, uint32_t y, uint32_t one)
 {
@@ -125,8 +125,8 @@ __device__ __forceinline__ void compress(uint32_t (&cv)[8], const uint32_t (&m)[
  * finishes last, stays in place; rows a, c and d, finished earlier, move
  * (a by one lane down, c one up, d two across), so most of their shuffle
  * latency (26 clocks) passes behind the rest of G.  A rotated word is added
- * to the next row straight from the unrotated one (rotate and add are one
- * instruction), which takes four operations off G's chain of twelve.
+ * to the next row straight from the unrotated one (rotl_add), beside the
+ * rotation that keeps the row, so that the chain need not pass through it.
  * Measured: 755 clocks a compression for 1 to 4 warps of an SM (8 nodes each)
  * and 824 for 8 warps, against 964 for one lane a node; a full SM does only
  * 24 G compressions/s this way against 40.0, so it is for narrow levels. */
@@ -136,8 +136,8 @@ struct QuadLane {
     bool b0, b1;      /* bits of i */
     __device__ __forceinline__ explicit QuadLane(uint32_t lane)
     {
-        /* opaque to the compiler, which otherwise computes them anew before
-         * most of a level's 84 shuffles and 84 selections */
+        /* opaque to the compiler, so that it keeps them for a level's 84
+         * shuffles and selections in place of computing them anew */
         asm volatile("and.b32 %0, %1, 3;" : "=r"(i) : "r"(lane));
         asm volatile("add.s32 %0, %1, 3;" : "=r"(below) : "r"(i));
         asm volatile("add.s32 %0, %1, 1;" : "=r"(above) : "r"(i));
@@ -150,8 +150,8 @@ struct QuadLane {
     }
 };
 
-/* shf.l written out, so that the compiler keeps it apart from the rotation
- * that produces the row itself and can fold it into the addition. */
+/* shf.l written out, apart from the rotation that produces the row itself,
+ * so that the compiler may fold it into the addition. */
 template <int N>
 __device__ __forceinline__ uint32_t rotl_add(uint32_t x, uint32_t y)
 {
@@ -160,7 +160,7 @@ __device__ __forceinline__ uint32_t rotl_add(uint32_t x, uint32_t y)
     return y + r;
 }
 
-/* Half a round: G with message words x and y, then the rows' move.  `down`:
+/* Half a round: G with message words x and y, then the rows' move.  COLUMN:
  * the step just done was the column step (a goes to the lane above's place,
  * that is, each lane reads a from the lane below). */
 template <bool COLUMN>
