@@ -1024,11 +1024,11 @@ no_split:
         b->cv0 = (pl[0].nunits == 0 || b->part[0].cv0) && (!nd || b->part[1].cv0) && (!nd2 || b->part[2].cv0);
 
         /* capture: every launch's seeds on the batch's stream, then the deep
-         * parts forked off and the rest behind a second reset of its queue.
-         * The deep parts' CTAs need whole SMs and run longest, so they should
-         * be placed first.  Nothing orders the three launches, whose nodes all
-         * run at one priority: the deep ones are merely ready sooner, by the
-         * time that the reset takes. */
+         * parts forked off and the rest.  Nothing orders the three launches,
+         * whose nodes all run at one priority.  (A node that delays the rest,
+         * for the deep parts' CTAs to be placed first, changes nothing: 256
+         * sessions 1189.8-1190.8 ms without one, 1190.9-1191.2 with; three
+         * other mixes 140.7, 313.2 and 393.0 ms either way.) */
         if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) goto fail;
         int crc = 0;
         for (int i = b->nparts - 1; i >= 0 && crc == 0; i--)
@@ -1046,8 +1046,7 @@ no_split:
             if (crc == 0) crc = cudaEventRecord(b->ev[7], b->stream3) == cudaSuccess ? 0 : -1;
         }
         if (crc == 0 && pl[0].nunits) {
-            if (nd) crc = cudaMemsetAsync(b->part[0].d_queue, 0, 64, b->stream) == cudaSuccess ? 0 : -1;
-            if (crc == 0) crc = part_capture(&b->part[0], b->stream, b->ev[1], b->ev[2]);
+            crc = part_capture(&b->part[0], b->stream, b->ev[1], b->ev[2]);
         }
         if (crc == 0 && nd) crc = cudaStreamWaitEvent(b->stream, b->ev[5], 0) == cudaSuccess ? 0 : -1;
         if (crc == 0 && nd2) crc = cudaStreamWaitEvent(b->stream, b->ev[7], 0) == cudaSuccess ? 0 : -1;
