@@ -72,7 +72,7 @@ def fake(tmp_path_factory):
     src = [os.path.join(CSRC, f) for f in ("label_api.c", "label_batch.c", "label_server.c", "label_stream.c",
                                            "label_verify.c", "topology.c", "b3_host.c")]
     src.append(os.path.join(ROOT, "tests", "fake_cuda.c"))
-    subprocess.run(["gcc", "-O2", "-std=c11", "-fPIC", "-shared", "-D_GNU_SOURCE", "-I" + CUDA_INC,
+    subprocess.run(["gcc", "-O2", "-std=c11", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-D_GNU_SOURCE", "-I" + CUDA_INC,
                     "-I" + os.path.join(ROOT, "include"), "-I" + CSRC, "-o", so, *src, "-lpthread", "-lm", "-ldl"],
                    check=True)
     return Fake(so)
