@@ -425,6 +425,7 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
         __syncthreads();
         uint32_t w = uniform(smem[Layout::hdr].y);
         if (CLUSTER && w > sw) cg::this_cluster().sync(); /* boundary 0 */
+        __syncthreads(); /* every warp has read level 0 */
         for (uint32_t l = 0; l < L; l++) {
             const uint32_t wn = uniform(smem[Layout::hdr + (l + 1) % 3].y);
             stage_data(p, smem, o, cnt, l + 1, lane, ginv);
@@ -462,8 +463,8 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
     };
     /* The level's start and width, this warp's part in it, and the ring stage
      * of the next level. */
-    uint32_t ls = 0, w = 0, st1 = 0, global = 0;
-    bool busy = false; /* this warp has a quad with an item */
+    uint32_t ls, w, st1, global;
+    bool busy; /* this warp has a quad with an item */
     Desc d;
     const auto enter = [&](uint32_t lv) {
         const uint32_t st = lv % 3;
@@ -475,14 +476,15 @@ __device__ __forceinline__ void depth_levels(const pb_depth_params_t &p, uint4 *
         global = __any_sync(0xFFFFFFFFu, d.global != 0);
     };
     const bool skips = warp >= PB_NARROW_WARPS;
+    if (CLUSTER && uniform(smem[Layout::hdr].y) > sw) cg::this_cluster().sync(); /* boundary 0 */
+    enter(0);
     /* A warp reads the ring only at levels whose next boundary it passes: past
      * one that it skips the producer may already have refilled the stage
-     * (level 0's in level 1).  A warp that skips level 0 knows its width from
-     * the level offsets, as it does further on. */
-    const uint32_t w0 = uniform(__ldg(tp.lstart + 1) - __ldg(tp.lstart));
-    if (CLUSTER && w0 > sw) cg::this_cluster().sync(); /* boundary 0 */
-    if (skips && !all_hands(w0)) w = w0;
-    else enter(0);
+     * (level 0's in level 1).  Level 0 is read by all: the producer waits for
+     * them.  (Its width read elsewhere by the warps that skip it, in place of
+     * this barrier: 471.7 ms for 32 chunks of 2^17, 904 for 4 of 2^18, 709 for
+     * 512 of 2^16; with it 470.4, 897 and 708.) */
+    __syncthreads();
 #pragma unroll 1
     for (uint32_t l = 0; l < L;) {
         if (skips && !all_hands(w)) {

@@ -1,5 +1,7 @@
 """Which levels' ring stages (records and header, three of them) a hashing warp
-of the depth kernels reads between two of its barriers (label_ws.cu).
+of the depth kernels reads between two of its barriers (label_ws.cu).  Every
+warp reads level 0 before a barrier that the producer passes before its first
+level.
 
 The producer fills the stage of level m while level m - 2 runs, and passes
 every boundary; a warp that skips narrow levels passes only the boundaries at
@@ -15,14 +17,13 @@ from test_depth_levels import NARROW_ITEMS, level_widths
 from test_topology import host  # noqa: F401  (the fixture)
 
 
-def skipping_warp(w, hands, reads_level_0):
+def skipping_warp(w, hands, barrier_0):
     """(level read, last boundary passed, next boundary) of a warp that skips
-    levels that are not of all hands; reads_level_0: also level 0 when it
-    skips it."""
+    levels that are not of all hands; barrier_0: a barrier follows the read of
+    level 0."""
     L = len(w)
-    walk, passed = [], [0]  # (level read, last boundary passed)
-    if hands[0] or reads_level_0:
-        walk.append((0, 0))
+    first = -1 if barrier_0 else 0
+    walk, passed = [(0, first)], sorted({first, 0})  # (level read, last boundary passed)
     for l in np.nonzero(hands)[0].tolist():
         if passed[-1] != l:  # after levels that it skipped
             passed.append(l)
@@ -34,7 +35,8 @@ def skipping_warp(w, hands, reads_level_0):
 
 
 def unsafe(reads):
-    return [(r, b1, b2) for r, b1, b2 in reads if not b2 - 1 <= r <= b1 + 1]
+    # the prologue (boundary -1) fills the stages of levels 0 and 1
+    return [(r, b1, b2) for r, b1, b2 in reads if not b2 - 1 <= r <= max(b1, 0) + 1]
 
 
 @pytest.mark.parametrize("cb", [2, 64, 300, 1024, 3000, 1 << 14])
@@ -44,9 +46,9 @@ def test_ring_reads(host, cb):  # noqa: F811
     for G in range(1, 9):
         for sw in ((1 << 30,) if G > 1 else (1 << 30, 0, 10, 480)):
             hands = (w * G > NARROW_ITEMS) | (w > sw)
-            assert not unsafe(skipping_warp(w, hands, reads_level_0=False)), (cb, G, sw)
-            # level 0 is the graph's one source node: a warp that reads its
-            # stage and skips it may find a later level there
-            seen += bool(unsafe(skipping_warp(w, hands, reads_level_0=True)))
+            assert not unsafe(skipping_warp(w, hands, barrier_0=True)), (cb, G, sw)
+            # level 0 is the graph's one source node: without the barrier a warp
+            # that reads its stage and skips it may find a later level there
+            seen += bool(unsafe(skipping_warp(w, hands, barrier_0=False)))
     if (w * 8 > NARROW_ITEMS).any():
         assert seen
