@@ -469,7 +469,7 @@ def run_served(pkg, torch, requests: int = 300, alone: bool = False, rate: float
            "value": sum(sizes) / MIB / wall, "unit": "MiB/s", "p50_ms": lat_sorted[len(lat) // 2],
            "p99_ms": lat_sorted[min(len(lat) - 1, int(0.99 * len(lat)))], "waves": st["waves"],
            "offered_mib_s": sum(sizes) / MIB / trace[-1]["arrival_s"], "wall_s": wall,
-           "policy": "chunk_blocks 2^15 and up on the depth kernel (1 to 4 copies per CTA by the load, SM held alone), "
+           "policy": "chunk_blocks 2^15 and up on the depth kernel (1 to 4 copies per CTA by load and free SMs, SM held alone), "
                      "the rest in up to 5 concurrent lockstep waves (3 with fewer than 16 work queues)",
            "work_queues": int(os.environ.get("CUDA_DEVICE_MAX_CONNECTIONS", "8"))}
     if alone:
